@@ -111,7 +111,7 @@ __global__ void k_set_int(int* p, int v) { *p = v; }
 // of the step and before the step counter advances.
 __global__ void k_angle(Geom g, KArgs a, float* __restrict__ ang, int hw)
 {
-    const int it = *a.it_ptr;
+    const int it = *a.it_ptr + a.it_add;
     const float* tp = a.f[F_TP];
     const float* vxp = a.f[F_VXP];
     const float* vzp = a.f[F_VZP];

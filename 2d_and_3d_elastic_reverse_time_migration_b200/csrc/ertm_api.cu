@@ -290,16 +290,16 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder()
 }
 
 // One tensor map over a whole padded volume (allocation base, [pz][py][px]) with a
-// bx x by x 1 box.  TMA requires 16-byte aligned bases and strides: cudaMalloc bases
+// bx x by x bz box.  TMA requires 16-byte aligned bases and strides: cudaMalloc bases
 // are 256-byte aligned and the row pitch is a multiple of 128 bytes.
-int encode_map(ertm_ctx* c, CUtensorMap* m, const void* base, bool is_int, int bx, int by)
+int encode_map(ertm_ctx* c, CUtensorMap* m, const void* base, bool is_int, int bx, int by, int bz = 1)
 {
     auto enc = tensor_map_encoder();
     if (!enc) return fail(c, ERTM_ECUDA, "cuTensorMapEncodeTiled unavailable");
     const Geom& g = c->g;
     cuuint64_t dims[3] = {(cuuint64_t)g.px, (cuuint64_t)g.py, (cuuint64_t)g.pz};
     cuuint64_t strides[2] = {(cuuint64_t)g.px * 4, (cuuint64_t)(g.px * g.py) * 4};
-    cuuint32_t box[3] = {(cuuint32_t)bx, (cuuint32_t)by, 1};
+    cuuint32_t box[3] = {(cuuint32_t)bx, (cuuint32_t)by, (cuuint32_t)bz};
     cuuint32_t es[3] = {1, 1, 1};
     CUresult r = enc(m, is_int ? CU_TENSOR_MAP_DATA_TYPE_INT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3,
                      const_cast<void*>(base), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
@@ -309,29 +309,27 @@ int encode_map(ertm_ctx* c, CUtensorMap* m, const void* base, bool is_int, int b
     return ERTM_OK;
 }
 
-struct BoxDims {
-    int c_x, c_y, x_x, y_y;
-};
-BoxDims box_dims(const ertm_ctx* c)
-{
-    const int tyb = c->g.tyb;
-    const int xw = TX + 2 * xb_of(c->R);
-    const int yh = tyb + (c->g.two_d ? 0 : 2 * c->R);
-    return {TX, tyb, xw, yh};
-}
-
 // tensor maps of every field: centre boxes for all, halo boxes where a kernel
-// differentiates along x / y: vx vy vz tp txy (XY), txx txz (X), tyy tyz (Y)
+// differentiates along x / y: vx vy vz tp txy (XY), txx txz (X), tyy tyz (Y).  2D:
+// tile boxes of the x-z plane, vx vz txz tp with both halos (XY), txx (X), tzz (Y)
 int build_field_maps(ertm_ctx* c)
 {
-    BoxDims b = box_dims(c);
     int rc;
+    if (c->g.two_d) {
+        const int xw = TX2 + 2 * xb_of(c->R), tz = 4 * c->g.nr2, zh = tz + 2 * c->R;
+        const int xz[4] = {F_VX, F_VZ, F_TXZ, F_TP};
+        for (int q : xz)
+            if ((rc = encode_map(c, &c->mXY[q], c->f_base[q], false, xw, 1, zh))) return rc;
+        if ((rc = encode_map(c, &c->mX[F_TXX], c->f_base[F_TXX], false, xw, 1, tz))) return rc;
+        return encode_map(c, &c->mY[F_TZZ], c->f_base[F_TZZ], false, TX2, 1, zh);
+    }
+    const int xw = TX + 2 * xb_of(c->R), yh = TY3 + 2 * c->R;
     for (int q = 0; q < NFIELD; q++) {
         if (!c->f_base[q]) continue;
-        if ((rc = encode_map(c, &c->mC[q], c->f_base[q], false, b.c_x, b.c_y))) return rc;
-        if ((rc = encode_map(c, &c->mX[q], c->f_base[q], false, b.x_x, b.c_y))) return rc;
-        if ((rc = encode_map(c, &c->mXY[q], c->f_base[q], false, b.x_x, b.y_y))) return rc;
-        if ((rc = encode_map(c, &c->mY[q], c->f_base[q], false, b.c_x, b.y_y))) return rc;
+        if ((rc = encode_map(c, &c->mC[q], c->f_base[q], false, TX, TY3))) return rc;
+        if ((rc = encode_map(c, &c->mX[q], c->f_base[q], false, xw, TY3))) return rc;
+        if ((rc = encode_map(c, &c->mXY[q], c->f_base[q], false, xw, yh))) return rc;
+        if ((rc = encode_map(c, &c->mY[q], c->f_base[q], false, TX, yh))) return rc;
     }
     return ERTM_OK;
 }
@@ -340,6 +338,11 @@ StressMaps stress_maps(const ertm_ctx* c, int which)
 {
     StressMaps m;
     std::memset(&m, 0, sizeof m);
+    if (c->g.two_d) {
+        m.v[0] = c->mXY[F_VX];
+        m.v[1] = c->mXY[F_VZ];
+        return m;
+    }
     const int v[3] = {F_VX, F_VZ, F_VY};
     for (int q = 0; q < 3; q++) {
         m.v[q] = c->mXY[v[q]];
@@ -357,7 +360,14 @@ VelMaps vel_maps(const ertm_ctx* c, int which, int epi)
 {
     VelMaps m;
     std::memset(&m, 0, sizeof m);
-    const bool Y = !c->g.two_d, ps = (epi != EPI_NONE);
+    if (c->g.two_d) {
+        m.txx = c->mX[F_TXX];
+        m.txz = c->mXY[F_TXZ];
+        m.tp = c->mXY[F_TP];
+        m.tyy = c->mY[F_TZZ];
+        return m;
+    }
+    const bool ps = (epi != EPI_NONE);
     m.txx = c->mX[F_TXX];
     m.txz = c->mX[F_TXZ];
     m.txy = c->mXY[F_TXY];
@@ -367,11 +377,11 @@ VelMaps vel_maps(const ertm_ctx* c, int which, int epi)
     int n = 0;
     m.c[n++] = c->mC[F_VX];
     m.c[n++] = c->mC[F_VZ];
-    if (Y) m.c[n++] = c->mC[F_VY];
+    m.c[n++] = c->mC[F_VY];
     if (ps) {
         m.c[n++] = c->mC[F_VXP];
         m.c[n++] = c->mC[F_VZP];
-        if (Y) m.c[n++] = c->mC[F_VYP];
+        m.c[n++] = c->mC[F_VYP];
     }
     m.c[n++] = c->mModel[which][2];
     if (epi == EPI_EXCITE) m.c[n++] = c->mExAmp;
@@ -379,7 +389,7 @@ VelMaps vel_maps(const ertm_ctx* c, int which, int epi)
     n = 0;
     m.fr[n++] = c->mC[F_TXZ];
     m.fr[n++] = c->mC[F_TZZ];
-    if (Y) m.fr[n++] = c->mC[F_TYZ];
+    m.fr[n++] = c->mC[F_TYZ];
     if (ps) m.fr[n++] = c->mC[F_TP];
     return m;
 }
@@ -407,9 +417,9 @@ int ensure_excitation(ertm_ctx* c)
         if ((rc = alloc_volume(c, &c->ex_v_base[q], &dummy))) return rc;
     }
     if ((rc = alloc_volume(c, &c->ex_tp_base, &dummy))) return rc;
-    const int tyb = c->g.tyb;
-    if ((rc = encode_map(c, &c->mExAmp, c->ex_amp2_base, false, TX, tyb))) return rc;
-    if ((rc = encode_map(c, &c->mExTime, c->ex_time_base, true, TX, tyb))) return rc;
+    if (c->g.two_d) return ERTM_OK;
+    if ((rc = encode_map(c, &c->mExAmp, c->ex_amp2_base, false, TX, TY3))) return rc;
+    if ((rc = encode_map(c, &c->mExTime, c->ex_time_base, true, TX, TY3))) return rc;
     return ERTM_OK;
 }
 
@@ -529,6 +539,7 @@ std::map<TuneKey, int> g_tuned;
 int autotune_kchunk(ertm_ctx* c, int which, int* out)
 {
     const Geom& g = c->g;
+    if (g.two_d) return ERTM_OK;   // the 2D kernels' tiles have no z chunk
     const bool cpml = c->cfg.boundary == ERTM_BOUNDARY_CPML;
     const TuneKey key{c->device, g.nx, g.ny, g.nz, c->R, cpml ? 1 : 0};
     {
@@ -619,37 +630,48 @@ struct Range {
 
 // One pass of `nsteps` steps.  MODE_MODEL records into `traces` ([3][nt][nrec],
 // device), MODE_RECEIVER injects from it.
-// The time loop of a pass: `one_step` (which launches one step's kernels on
-// c->stream) runs nsteps times, as a CUDA graph of kGraphSteps steps replayed
-// back to back (the kernels read the step index from device memory, so one graph
-// serves every chunk); the first step and the remainder are launched directly.
+// The time loop of a pass: `one_step(add)` launches one step's kernels on c->stream
+// for the step index *c->it_d + add.  nsteps steps run in direction `dir`, as a CUDA
+// graph of kGraphSteps steps replayed back to back (the base index lives in device
+// memory and moves once per replay, so one graph serves every chunk and no step
+// carries a counter launch); the first step and the remainder are launched directly.
+// A short graph: building one costs about 6 us per launch in it (measured 400 us for 32
+// steps of a 2D pass, against 0.6 us that a replayed step saves over a direct launch),
+// while a replay of 8 steps already hides its own launch.  Long passes amortise 32.
 template <typename F>
-int time_loop(ertm_ctx* c, int nsteps, F&& one_step)
+int time_loop(ertm_ctx* c, int nsteps, int dir, F&& one_step)
 {
-    constexpr int kGraphSteps = 32;
+    const int kGraphSteps = nsteps >= 1500 ? 32 : 8;
     int done = 0;
     if (nsteps > 0) {
-        CK(c, one_step());
+        CK(c, one_step(0));
         done = 1;
     }
+    int base = 0;                    // steps that the device's index has moved
     if (nsteps - done >= 2 * kGraphSteps) {
+        CK(c, launch_advance(c->it_d, dir * done, c->stream));
+        base = done;
+        c->launches++;
         cudaGraph_t graph = nullptr;
         cudaGraphExec_t exec = nullptr;
         CK(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
         cudaError_t e = cudaSuccess;
-        for (int q = 0; q < kGraphSteps && e == cudaSuccess; q++) e = one_step();
+        for (int q = 0; q < kGraphSteps && e == cudaSuccess; q++) e = one_step(dir * q);
+        if (e == cudaSuccess) e = launch_advance(c->it_d, dir * kGraphSteps, c->stream);
         cudaError_t e2 = cudaStreamEndCapture(c->stream, &graph);
         if (e == cudaSuccess) e = e2;
         if (e == cudaSuccess) e = cudaGraphInstantiate(&exec, graph, 0);
         while (e == cudaSuccess && nsteps - done >= kGraphSteps) {
             e = cudaGraphLaunch(exec, c->stream);
             done += kGraphSteps;
+            c->launches++;
         }
         if (exec) cudaGraphExecDestroy(exec);
         if (graph) cudaGraphDestroy(graph);
         if (e != cudaSuccess) return fail(c, ERTM_ECUDA, "graph time loop: %s", cudaGetErrorString(e));
     }
-    for (; done < nsteps; done++) CK(c, one_step());
+    if (base) base = done;           // the replays moved the index along
+    for (; done < nsteps; done++) CK(c, one_step(dir * (done - base)));
     return ERTM_OK;
 }
 
@@ -662,7 +684,7 @@ int run_pass(ertm_ctx* c, int which, const ertm_shot* s, int mode, int nsteps, f
     int rc;
     float vmax = c->cfg.pml_vmax > 0 ? c->cfg.pml_vmax : c->vpmax[which];
     if ((rc = upload_profiles(c, vmax))) return rc;
-    int kchunk = choose_kchunk(c->g, c->R, c->device);
+    int kchunk = choose_kchunk(c->g);
     if (c->cfg.autotune == 1 && (rc = autotune_kchunk(c, which, &kchunk))) return rc;
     if ((rc = reset_state(c))) return rc;
     if (mode != MODE_RECEIVER && (rc = upload_wavelet(c, s))) return rc;
@@ -691,16 +713,16 @@ int run_pass(ertm_ctx* c, int which, const ertm_shot* s, int mode, int nsteps, f
     float* ang = nullptr;
     if (c->angles && mode == MODE_SOURCE) ang = c->ang_base[0] + c->g.off0;
     if (c->angles && mode == MODE_RECEIVER) ang = c->ang_base[1] + c->g.off0;
-    auto one_step = [&]() -> cudaError_t {
+    auto one_step = [&](int add) -> cudaError_t {
+        a.it_add = add;
         cudaError_t e = launch_stress(R, c->g, a, sm, cpml, psplit, c->stream);
         if (e == cudaSuccess) e = launch_velocity(R, c->g, a, vm, cpml, epi, record, c->stream);
         if (e == cudaSuccess && ang)
             e = launch_angle(c->g, a, ang, mode == MODE_SOURCE ? 2 : 4, c->stream);
-        if (e == cudaSuccess) e = launch_advance(c->it_d, dir, c->stream);
         return e;
     };
-    if ((rc = time_loop(c, nsteps, one_step))) return rc;
-    c->launches += (ang ? 4LL : 3LL) * nsteps;
+    if ((rc = time_loop(c, nsteps, dir, one_step))) return rc;
+    c->launches += (ang ? 3LL : 2LL) * nsteps;
     return check_device_error(c);
 }
 
@@ -975,8 +997,8 @@ int ertm_set_model(ertm_ctx* c, int which, const float* vp, const float* vs, con
     for (int q = 0; q < 5; q++) {
         if (c->m_base[which][q]) continue;
         if ((rc = alloc_volume(c, &c->m_base[which][q], &c->m[which][q]))) return rc;
-        if (q < 3 && (rc = encode_map(c, &c->mModel[which][q], c->m_base[which][q], false, TX,
-                                      c->g.tyb)))
+        if (q < 3 && !c->g.two_d &&
+            (rc = encode_map(c, &c->mModel[which][q], c->m_base[which][q], false, TX, TY3)))
             return rc;
     }
     if ((rc = ensure_stage(c))) return rc;
@@ -1182,7 +1204,7 @@ int ertm_rtm_multi(ertm_ctx* const* ctx, int n, const ertm_shot* shots, const fl
         ertm_ctx* c = ctx[q];
         if ((rc = upload_profiles(c, c->cfg.pml_vmax > 0 ? c->cfg.pml_vmax : c->vpmax[1]))) return rc;
     }
-    int kchunk = choose_kchunk(c0->g, c0->R, c0->device);
+    int kchunk = choose_kchunk(c0->g);
     if (c0->cfg.autotune == 1 && (rc = autotune_kchunk(c0, 1, &kchunk))) return rc;
     const int chunks = (c0->g.nz + kchunk - 1) / kchunk;
     unsigned gx = 0, gy = 0;
@@ -1212,14 +1234,14 @@ int ertm_rtm_multi(ertm_ctx* const* ctx, int n, const ertm_shot* shots, const fl
         VP->m[q] = vel_maps(c, 1, epi);
     };
     auto loop = [&](int epi, int nsteps, int dir) -> int {
-        auto one_step = [&]() -> cudaError_t {
+        auto one_step = [&](int add) -> cudaError_t {
+            for (int q = 0; q < n; q++) SP->a[q].it_add = VP->a[q].it_add = add;
             cudaError_t e = launch_stress_multi(c0->R, grid, *SP, cpml, st);
             if (e == cudaSuccess) e = launch_velocity_multi(c0->R, grid, *VP, cpml, epi, st);
-            if (e == cudaSuccess) e = launch_advance(c0->it_d, dir, st);
             return e;
         };
-        int r = time_loop(c0, nsteps, one_step);
-        c0->launches += 3LL * nsteps;
+        int r = time_loop(c0, nsteps, dir, one_step);
+        c0->launches += 2LL * nsteps;
         return r;
     };
 
@@ -1407,7 +1429,7 @@ int ertm_time_kernels(ertm_ctx* c, const ertm_shot* s, int nsteps, float* ms)
     if ((rc = upload_wavelet(c, s))) return rc;
     KArgs a;
     fill_args(c, 1, s, a);
-    a.kchunk = choose_kchunk(c->g, c->R, c->device);
+    a.kchunk = choose_kchunk(c->g);
     const bool cpml = c->cfg.boundary == ERTM_BOUNDARY_CPML;
     cudaEvent_t ev[3];
     for (int q = 0; q < 3; q++) CK(c, cudaEventCreate(&ev[q]));

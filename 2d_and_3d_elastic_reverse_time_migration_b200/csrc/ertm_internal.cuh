@@ -21,7 +21,7 @@ namespace ertm {
 constexpr int TX = 32;        // x tile = one warp
 constexpr int TY3 = 8;        // y tile of the 3D kernels
 constexpr int CTAS3 = 2;      // resident CTAs per SM of the 3D step kernels
-constexpr int TY2 = 1;        // y tile of the 2D kernels (a 2D grid has one y row)
+constexpr int TX2 = 64;       // x tile of the 2D kernels
 constexpr int XH = 8;         // allocated x halo, floats (>= R, 32-byte aligned)
 
 enum Field {
@@ -44,7 +44,8 @@ struct Geom {
     long long off0;         // offset of cell (0,0,0)
     long long total;        // floats per volume
     int two_d;
-    int tyb;                // y tile of the kernels for this grid
+    int tyb;                // y tile of the 3D kernels (1 in 2D)
+    int nr2;                // 2D kernels: rows per thread (1, 2 or 4), fixed with the maps' boxes
 };
 
 // Everything a step kernel reads; passed by value (param space).
@@ -74,7 +75,8 @@ struct KArgs {
     int inject_mode;
     float* traces;                   // [3][nt][nrec], recorded or injected
     int nt;
-    const int* it_ptr;               // current step index (device)
+    const int* it_ptr;               // step index (device) of the launch sequence ...
+    int it_add;                      // ... plus this launch's own offset
     // excitation state and images (same geometry as the fields)
     float* ex_amp2;
     int* ex_time;
@@ -90,7 +92,7 @@ struct KArgs {
     unsigned wait_polls;
     // 3D step-kernel variant: 0 = one cell per thread (default), 1 = cell pairs
     int pairs;
-    // several shots per launch only: the shot is idle while *it_ptr >= it_hi
+    // several shots per launch only: the shot is idle while its step index >= it_hi
     int it_hi;
 };
 
@@ -100,9 +102,12 @@ enum DeviceError { DEV_OK = 0, DEV_WAIT_TIMEOUT = 1 };
 // TMA tensor maps of one step kernel, passed as a __grid_constant__ parameter.
 // Every map covers a whole padded volume [pz][py][px]; the box shape is fixed
 // per map: C = TX x TYB (centre), X = (TX+2XB) x TYB, Y = TX x (TYB+2R),
-// XY = (TX+2XB) x (TYB+2R), one plane deep.
+// XY = (TX+2XB) x (TYB+2R), one plane deep.  2D grids use four of them with boxes of
+// one tile of the x-z plane (see step_kernels_2d.cuh; Tile2 boxes, TZ = 4 nr2 rows):
+// v[0], v[1], txz and tp with halos in x and z, txx in x, tyy = the box of tzz with
+// the halo in z.
 struct StressMaps {
-    CUtensorMap v[3];      // vx, vz, vy      (XY boxes; X in 2D)
+    CUtensorMap v[3];      // vx, vz, vy      (XY boxes)
     CUtensorMap vc[3];     // vx, vz, vy      (C boxes: z-queue fronts)
     CUtensorMap sig[6];    // txx tzz txz tyy txy tyz (C)
     CUtensorMap tp;        // (C)
@@ -111,7 +116,7 @@ struct StressMaps {
 
 struct VelMaps {
     CUtensorMap txx, txz;  // X boxes
-    CUtensorMap txy, tp;   // XY boxes (X in 2D)
+    CUtensorMap txy, tp;   // XY boxes
     CUtensorMap tyy, tyz;  // Y boxes
     CUtensorMap c[8];      // C boxes: vx vz vy vxp vzp vyp b excitation(amp2 or time)
     CUtensorMap fr[4];     // C boxes of txz tzz tyz tp: z-queue fronts
@@ -154,6 +159,25 @@ inline cudaError_t smem_opt_in(KPTR K, size_t smem, unsigned long long* done)
     return e;
 }
 
+// A step kernel launched as a programmatic dependent of the launch before it in the
+// stream: its CTAs may become resident while that one drains, and it waits for it
+// (pdl_wait) before touching memory.  The edge survives stream capture.
+template <typename... P>
+inline cudaError_t launch_pdl(void (*K)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, const P&... args)
+{
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cf{};
+    cf.gridDim = grid;
+    cf.blockDim = block;
+    cf.dynamicSmemBytes = smem;
+    cf.stream = st;
+    cf.attrs = &at;
+    cf.numAttrs = 1;
+    return cudaLaunchKernelEx(&cf, K, args...);
+}
+
 // Host set-up shared by the context path and the no-allocation path (setup.cu).
 Geom make_geom(int nx, int ny, int nz, int R);
 // difference coefficients c_0..c_R (c_0 = 0) for ERTM_COEF_* `coef_kind`
@@ -165,8 +189,8 @@ void cpml_profile(int n, int w0, int w1, int stg, double h, double vmax, double 
 // sponge damping (1/s, ERTM_BOUNDARY_SPONGE_COS or _CUBIC ramps) of one axis of n
 // cells, for cells i0 .. i0+m-1 into v[0..m)
 void sponge_profile(int n, int w0, int w1, int kind, float coe, int i0, int m, float* v);
-// z planes per CTA of the step kernels for grid g on `device`
-int choose_kchunk(const Geom& g, int R, int device);
+// z planes per CTA of the 3D step kernels for grid g
+int choose_kchunk(const Geom& g);
 
 // Launchers (one translation unit per stencil radius).
 cudaError_t launch_stress(int R, const Geom& g, const KArgs& a, const StressMaps& m, bool cpml,

@@ -127,7 +127,7 @@ struct Carve {
     }
 };
 
-int encode(CUtensorMap* m, const void* base, const Geom& g, int bx, int by)
+int encode(CUtensorMap* m, const void* base, const Geom& g, int bx, int by, int bz = 1)
 {
     static PFN_cuTensorMapEncodeTiled_v12000 enc = [] {
         void* p = nullptr;
@@ -143,7 +143,7 @@ int encode(CUtensorMap* m, const void* base, const Geom& g, int bx, int by)
     if (!enc) return nfail(ERTM_ECUDA, "cuTensorMapEncodeTiled unavailable");
     cuuint64_t dims[3] = {(cuuint64_t)g.px, (cuuint64_t)g.py, (cuuint64_t)g.pz};
     cuuint64_t strides[2] = {(cuuint64_t)g.px * 4, (cuuint64_t)(g.px * g.py) * 4};
-    cuuint32_t box[3] = {(cuuint32_t)bx, (cuuint32_t)by, 1};
+    cuuint32_t box[3] = {(cuuint32_t)bx, (cuuint32_t)by, (cuuint32_t)bz};
     cuuint32_t es[3] = {1, 1, 1};
     CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<void*>(base), dims, strides,
                      box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
@@ -356,49 +356,55 @@ int run_noalloc(const ertm_config* cfg, const float* vp, const float* vs, const 
     a.it_ptr = counters;
     a.err = counters + 4;
 
-    // z planes per CTA: the context path's rule
-    a.kchunk = choose_kchunk(g, R, c.device);
+    // z planes per CTA (3D): the context path's rule
+    a.kchunk = choose_kchunk(g);
 
     // tensor maps over the scratch volumes
     StressMaps sm;
     VelMaps vm;
     std::memset(&sm, 0, sizeof sm);
     std::memset(&vm, 0, sizeof vm);
-    const int xw = TX + 2 * xb_of(R), yh = g.tyb + (two_d ? 0 : 2 * R);
-    const int vv[3] = {F_VX, F_VZ, F_VY};
-    for (int q = 0; q < (two_d ? 2 : 3); q++) {
-        if ((rc = encode(&sm.v[q], fbase[vv[q]], g, xw, yh))) return rc;
-        if ((rc = encode(&sm.vc[q], fbase[vv[q]], g, TX, g.tyb))) return rc;
-    }
-    const int sg[6] = {F_TXX, F_TZZ, F_TXZ, F_TYY, F_TXY, F_TYZ};
-    for (int q = 0; q < (two_d ? 3 : 6); q++)
-        if ((rc = encode(&sm.sig[q], fbase[sg[q]], g, TX, g.tyb))) return rc;
-    if ((rc = encode(&sm.M, mbase[0], g, TX, g.tyb))) return rc;
-    if ((rc = encode(&sm.MU, mbase[1], g, TX, g.tyb))) return rc;
-    if ((rc = encode(&vm.txx, fbase[F_TXX], g, xw, g.tyb))) return rc;
-    if ((rc = encode(&vm.txz, fbase[F_TXZ], g, xw, g.tyb))) return rc;
-    if (!two_d) {
+    if (two_d) {
+        // one tile of the x-z plane per box (see step_kernels_2d.cuh)
+        const int xw = TX2 + 2 * xb_of(R), tz = 4 * g.nr2, zh = tz + 2 * R;
+        if ((rc = encode(&sm.v[0], fbase[F_VX], g, xw, 1, zh))) return rc;
+        if ((rc = encode(&sm.v[1], fbase[F_VZ], g, xw, 1, zh))) return rc;
+        if ((rc = encode(&vm.txx, fbase[F_TXX], g, xw, 1, tz))) return rc;
+        if ((rc = encode(&vm.txz, fbase[F_TXZ], g, xw, 1, zh))) return rc;
+        if ((rc = encode(&vm.tyy, fbase[F_TZZ], g, TX2, 1, zh))) return rc;
+    } else {
+        const int xw = TX + 2 * xb_of(R), yh = TY3 + 2 * R;
+        const int vv[3] = {F_VX, F_VZ, F_VY};
+        for (int q = 0; q < 3; q++) {
+            if ((rc = encode(&sm.v[q], fbase[vv[q]], g, xw, yh))) return rc;
+            if ((rc = encode(&sm.vc[q], fbase[vv[q]], g, TX, TY3))) return rc;
+        }
+        const int sg[6] = {F_TXX, F_TZZ, F_TXZ, F_TYY, F_TXY, F_TYZ};
+        for (int q = 0; q < 6; q++)
+            if ((rc = encode(&sm.sig[q], fbase[sg[q]], g, TX, TY3))) return rc;
+        if ((rc = encode(&sm.M, mbase[0], g, TX, TY3))) return rc;
+        if ((rc = encode(&sm.MU, mbase[1], g, TX, TY3))) return rc;
+        if ((rc = encode(&vm.txx, fbase[F_TXX], g, xw, TY3))) return rc;
+        if ((rc = encode(&vm.txz, fbase[F_TXZ], g, xw, TY3))) return rc;
         if ((rc = encode(&vm.txy, fbase[F_TXY], g, xw, yh))) return rc;
         if ((rc = encode(&vm.tyy, fbase[F_TYY], g, TX, yh))) return rc;
         if ((rc = encode(&vm.tyz, fbase[F_TYZ], g, TX, yh))) return rc;
+        if ((rc = encode(&vm.c[0], fbase[F_VX], g, TX, TY3))) return rc;
+        if ((rc = encode(&vm.c[1], fbase[F_VZ], g, TX, TY3))) return rc;
+        if ((rc = encode(&vm.c[2], fbase[F_VY], g, TX, TY3))) return rc;
+        if ((rc = encode(&vm.c[3], mbase[2], g, TX, TY3))) return rc;
+        if ((rc = encode(&vm.fr[0], fbase[F_TXZ], g, TX, TY3))) return rc;
+        if ((rc = encode(&vm.fr[1], fbase[F_TZZ], g, TX, TY3))) return rc;
+        if ((rc = encode(&vm.fr[2], fbase[F_TYZ], g, TX, TY3))) return rc;
     }
-    int n = 0;
-    if ((rc = encode(&vm.c[n++], fbase[F_VX], g, TX, g.tyb))) return rc;
-    if ((rc = encode(&vm.c[n++], fbase[F_VZ], g, TX, g.tyb))) return rc;
-    if (!two_d && (rc = encode(&vm.c[n++], fbase[F_VY], g, TX, g.tyb))) return rc;
-    if ((rc = encode(&vm.c[n++], mbase[2], g, TX, g.tyb))) return rc;
-    n = 0;
-    if ((rc = encode(&vm.fr[n++], fbase[F_TXZ], g, TX, g.tyb))) return rc;
-    if ((rc = encode(&vm.fr[n++], fbase[F_TZZ], g, TX, g.tyb))) return rc;
-    if (!two_d && (rc = encode(&vm.fr[n++], fbase[F_TYZ], g, TX, g.tyb))) return rc;
 
     // the modelling pass: record vx, vy, vz at the receivers for every step
     if (nrec > 0) NCK(cudaMemsetAsync(data_out, 0, 4 * 3 * (size_t)c.nt * nrec, st));
     NCK(launch_set_int(counters, 0, st));
     for (int step = 0; step < c.nt; step++) {
+        a.it_add = step;
         NCK(launch_stress(R, g, a, sm, cpml, false, st));
         NCK(launch_velocity(R, g, a, vm, cpml, EPI_NONE, nrec > 0, st));
-        NCK(launch_advance(counters, 1, st));
     }
     int err = 0;
     NCK(cudaMemcpyAsync(&err, counters + 4, sizeof(int), cudaMemcpyDeviceToHost, st));

@@ -1,6 +1,6 @@
 // Host set-up shared by every entry point that runs the step kernels: the
 // padded-volume geometry, the difference coefficients, the absorbing-boundary
-// profiles and the z-chunk rule.  The context path (ertm_api.cu) and the
+// profiles and the tile rules.  The context path (ertm_api.cu) and the
 // no-allocation modelling path (noalloc.cu) both call these, so the two can
 // never drift apart.
 #include <cuda_runtime.h>
@@ -14,6 +14,21 @@ namespace ertm {
 
 static long long rup(long long v, long long m) { return (v + m - 1) / m * m; }
 
+// Rows per thread of the 2D tile kernels: as many (1, 2 or 4) as still give every SM a
+// CTA (64 columns x 4 rows of threads).  More rows per thread share more of the z window
+// and re-read fewer halo rows, fewer rows give small grids more CTAs.  Measured on B200,
+// us per step (R = 4, C-PML, modelling) with 1 / 2 / 4 rows: 168 x 104 4.3 / 4.8 / 6.1,
+// 680 x 380 10.5 / 9.6 / 8.0, 4096 x 2048 201 / 166 / 154.  With R = 6 the four-row
+// kernels' registers leave one CTA less per SM, which costs a grid that streams from
+// HBM more than the window saves: 4096 x 2048 205 / 155 / 165 (1471 x 803: 30 / 23 / 22).
+static int rows2d(int nx, int nz, int R)
+{
+    const long long cols = (nx + TX2 - 1) / TX2;
+    for (int nr = R > 4 && (long long)nx * nz > (3 << 20) ? 2 : 4; nr > 1; nr /= 2)
+        if (cols * ((nz + 4 * nr - 1) / (4 * nr)) >= 148) return nr;
+    return 1;
+}
+
 Geom make_geom(int nx, int ny, int nz, int R)
 {
     Geom g{};
@@ -22,7 +37,8 @@ Geom make_geom(int nx, int ny, int nz, int R)
     g.nz = nz;
     g.R = R;
     g.two_d = (ny == 1);
-    g.tyb = g.two_d ? TY2 : TY3;
+    g.tyb = g.two_d ? 1 : TY3;
+    g.nr2 = rows2d(nx, nz, R);
     g.hx = XH;
     g.hy = g.two_d ? 0 : R;
     g.hz = R;
@@ -132,40 +148,18 @@ void sponge_profile(int n, int w0, int w1, int kind, float coe, int i0, int m, f
     }
 }
 
-// z planes per CTA.  3D: chunks of about 32 planes, balanced over nz.  Timed on
-// B200 at 480 x 480 x 380 (R = 4, C-PML), the step kernels get faster as the
+// z planes per CTA of the 3D kernels: chunks of about 32 planes, balanced over nz.
+// Timed on B200 at 480 x 480 x 380 (R = 4, C-PML), the step kernels get faster as the
 // chunk shrinks from the whole column (380 planes) down to 32-48 planes
 // (stress 1.92 -> 1.51 ms, velocity 1.98 -> 1.61 ms per launch), while below
 // ~24 planes the z-queue fill of each chunk starts to cost more than the finer
-// load balance gains.  2D: the chunk count minimises (waves of CTAs) x
-// (planes per chunk + start-up of ~2R planes).
-int choose_kchunk(const Geom& g, int R, int device)
+// load balance gains.
+int choose_kchunk(const Geom& g)
 {
-    if (!g.two_d) {
-        const int target = 32;
-        const int chunks = std::max(1, (g.nz + target / 2) / target);
-        return (g.nz + chunks - 1) / chunks;
-    }
-    const long long cols = (long long)((g.nx + TX - 1) / TX) * ((g.ny + g.tyb - 1) / g.tyb);
-    int sms = 148;
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) {
-        cudaGetLastError();
-        sms = 148;
-    }
-    const long long slots = (long long)sms * 8;
-    const double startup = 2.0 * R;
-    int best = g.nz;
-    double best_cost = 1e300;
-    for (int kc = g.nz; kc >= std::min(g.nz, 16); kc--) {
-        const long long chunks = (g.nz + kc - 1) / kc;
-        const long long waves = (cols * chunks + slots - 1) / slots;
-        const double cost = (double)waves * (kc + startup);
-        if (cost < best_cost - 1e-9) {
-            best_cost = cost;
-            best = kc;
-        }
-    }
-    return best;
+    if (g.two_d) return g.nz;
+    const int target = 32;
+    const int chunks = std::max(1, (g.nz + target / 2) / target);
+    return (g.nz + chunks - 1) / chunks;
 }
 
 }  // namespace ertm

@@ -59,6 +59,13 @@ __device__ __forceinline__ void damping(const KArgs& a, bool cpml, int i, int j,
     }
 }
 
+// step index of this launch (a plain load: a dependent launch may start before the
+// counter's last change, see step_kernels_2d.cuh)
+__device__ __forceinline__ int step_index(const KArgs& a)
+{
+    return *(volatile const int*)a.it_ptr + a.it_add;
+}
+
 __device__ __forceinline__ int receiver_index(const KArgs& a, int i, int j)
 {
     int di = i - a.rx0, dj = j - a.ry0;
@@ -150,11 +157,11 @@ __device__ __forceinline__ void tma3(float* dst, const CUtensorMap* map, int x, 
 }
 
 // Box geometry of the staged tiles
-template <int R, bool Y>
+template <int R>
 struct Boxes {
-    static constexpr int TYB = Y ? TY3 : TY2;
+    static constexpr int TYB = TY3;
     static constexpr int XB = xb_of(R);
-    static constexpr int YB = Y ? R : 0;
+    static constexpr int YB = R;
     static constexpr int C = TX * TYB;                         // centre box
     static constexpr int XW = TX + 2 * XB;                      // x-halo box width
     static constexpr int X = XW * TYB;
@@ -162,8 +169,7 @@ struct Boxes {
     static constexpr int Yb = TX * YH;
     static constexpr int XY = XW * YH;
     // shared-memory slot sizes: a TMA box must land on a 128-byte boundary, so
-    // slots round up to 32 floats (a no-op for the 3D tiles; one-row 2D tiles
-    // have 40- or 48-float halo boxes)
+    // slots round up to 32 floats
     static constexpr int XP = (X + 31) / 32 * 32;
     static constexpr int XYP = (XY + 31) / 32 * 32;
 };
@@ -201,13 +207,13 @@ __device__ __forceinline__ bool produce_planes(uint64_t* bars, int nk, unsigned 
 // ---------------------------------------------------------------------------
 // Stress kernel
 // ---------------------------------------------------------------------------
-template <int R, bool Y, bool CPML, bool PS>
+template <int R, bool CPML, bool PS>
 struct StressShape {
-    using B = Boxes<R, Y>;
-    static constexpr int NV = Y ? 3 : 2;                        // vx, vz, (vy)
-    static constexpr int NSIG = Y ? 6 : 3;                      // txx tzz txz (tyy txy tyz)
+    using B = Boxes<R>;
+    static constexpr int NV = 3;                                // vx, vz, vy
+    static constexpr int NSIG = 6;                              // txx tzz txz tyy txy tyz
     static constexpr int NC = NSIG + (PS ? 1 : 0) + 2;          // + tp + M + MU
-    static constexpr int NP = CPML ? (Y ? 9 : 4) : 0;
+    static constexpr int NP = CPML ? 9 : 0;
     // stage: v tiles (XY), fronts (C), cells (C)
     static constexpr int OFF_FR = NV * B::XYP;
     static constexpr int OFF_C = OFF_FR + NV * B::C;
@@ -222,10 +228,10 @@ struct StressShape {
 
 // The stress step of one CTA: tile (blockIdx.x, blockIdx.y) of the x-y plane, z
 // chunk bz of the grid described by `a`, whose TMA maps are `maps`.
-template <int R, bool Y, bool CPML, bool PS>
+template <int R, bool CPML, bool PS>
 __device__ __forceinline__ void stress_body(const StressMaps& maps, const KArgs& a, int bz)
 {
-    using SS = StressShape<R, Y, CPML, PS>;
+    using SS = StressShape<R, CPML, PS>;
     using B = typename SS::B;
     constexpr int NS = SS::NS;
     constexpr int TYB = B::TYB, XB = B::XB, XW = B::XW, CB = B::C;
@@ -244,13 +250,13 @@ __device__ __forceinline__ void stress_body(const StressMaps& maps, const KArgs&
     const int nk = k1 - k0;
     const int sy = (int)a.sy, sz = (int)a.sz;
     const bool act = (i < a.nx) && (j < a.ny);
-    const int it = __ldg(a.it_ptr);
+    const int it = step_index(a);
     const bool src_on = (it >= 0) && (it < a.nw);
     const bool src_here = src_on && (i == a.ssx) && (j == a.ssy);
     const float wsrc = src_on ? __ldg(a.wavelet + it) : 0.f;
     const int cell = ty * TX + tx;
     // padded-volume coordinates of the tile
-    const int gx = i0 + XH, gy = j0 + (Y ? R : 0), gz0 = k0 + R;
+    const int gx = i0 + XH, gy = j0 + R, gz0 = k0 + R;
 
     float* sig[6] = {a.f[F_TXX], a.f[F_TZZ], a.f[F_TXZ], a.f[F_TYY], a.f[F_TXY], a.f[F_TYZ]};
     float* tp = a.f[F_TP];
@@ -279,7 +285,7 @@ __device__ __forceinline__ void stress_body(const StressMaps& maps, const KArgs&
     // C-PML: slab membership and profile coefficients of this column
     const int WX = a.w[0] + a.w[1], WY = a.w[2] + a.w[3];
     const bool inx = CPML && act && (i < a.w[0] || i >= a.nx - a.w[1]);
-    const bool iny = CPML && Y && act && (j < a.w[2] || j >= a.ny - a.w[3]);
+    const bool iny = CPML && act && (j < a.w[2] || j >= a.ny - a.w[3]);
     const int slx = i < a.w[0] ? i : i - a.nx + WX;
     const int sly = j < a.w[2] ? j : j - a.ny + WY;
     float axf = 0.f, bxf = 1.f, axh = 0.f, bxh = 1.f, ayf = 0.f, byf = 1.f, ayh = 0.f, byh = 1.f;
@@ -292,7 +298,7 @@ __device__ __forceinline__ void stress_body(const StressMaps& maps, const KArgs&
         ayh = __ldg(a.pa[1][1] + j); byh = __ldg(a.pb[1][1] + j);
     }
     // psi slots: x: EXX DXVZ (DXVY), y: EYY DYVX DYVZ, z: EZZ DZVX (DZVY)
-    constexpr int PX = 0, PY = Y ? 3 : 2, PZ = Y ? 6 : 2;
+    constexpr int PX = 0, PY = 3, PZ = 6;
     auto issue_psi = [&](int p, int buf) {
         if (!CPML) return;
         float* Ps = psibuf + buf * SS::PSI;
@@ -300,7 +306,7 @@ __device__ __forceinline__ void stress_body(const StressMaps& maps, const KArgs&
             const int x = (p * a.ny + j) * WX + slx;
             cpa4(&Ps[(PX + 0) * CB + cell], a.psi[P_EXX] + x);
             cpa4(&Ps[(PX + 1) * CB + cell], a.psi[P_DXVZ] + x);
-            if (Y) cpa4(&Ps[(PX + 2) * CB + cell], a.psi[P_DXVY] + x);
+            cpa4(&Ps[(PX + 2) * CB + cell], a.psi[P_DXVY] + x);
         }
         if (iny) {
             const int y = (p * WY + sly) * a.nx + i;
@@ -313,7 +319,7 @@ __device__ __forceinline__ void stress_body(const StressMaps& maps, const KArgs&
             const int z = (sl * a.ny + j) * a.nx + i;
             cpa4(&Ps[(PZ + 0) * CB + cell], a.psi[P_EZZ] + z);
             cpa4(&Ps[(PZ + 1) * CB + cell], a.psi[P_DZVX] + z);
-            if (Y) cpa4(&Ps[(PZ + 2) * CB + cell], a.psi[P_DZVY] + z);
+            cpa4(&Ps[(PZ + 2) * CB + cell], a.psi[P_DZVY] + z);
         }
         cpa_commit();
     };
@@ -340,7 +346,7 @@ __device__ __forceinline__ void stress_body(const StressMaps& maps, const KArgs&
         const int cc = (k0 + q - R) * sz + cj;
         qx[q] = vsrc[0][cc];
         qz[q] = vsrc[1][cc];
-        if (Y) qy[q] = vsrc[2][cc];
+        qy[q] = vsrc[2][cc];
     }
     issue_psi(k0, 0);
     if (nk > 1) issue_psi(k0 + 1, 1);
@@ -364,7 +370,7 @@ __device__ __forceinline__ void stress_body(const StressMaps& maps, const KArgs&
         const float* Ps = psibuf + (t % 3) * SS::PSI;
         qx[2 * R] = S[SS::OFF_FR + 0 * CB + cell];
         qz[2 * R] = S[SS::OFF_FR + 1 * CB + cell];
-        if (Y) qy[2 * R] = S[SS::OFF_FR + 2 * CB + cell];
+        qy[2 * R] = S[SS::OFF_FR + 2 * CB + cell];
         // tiles: (TX+2XB) wide, (TYB+2YB) high; the cell sits at row ty+YB, column tx+XB
         const float* Tx = S + 0 * B::XYP + (ty + B::YB) * XW + tx + XB;
         const float* Tz = S + 1 * B::XYP + (ty + B::YB) * XW + tx + XB;
@@ -378,13 +384,11 @@ __device__ __forceinline__ void stress_body(const StressMaps& maps, const KArgs&
             dxvz = fmaf(a.cx[n], Tz[n - 1] - Tz[-n], dxvz);
             ezz = fmaf(a.cz[n], qz[R + n - 1] - qz[R - n], ezz);
             dzvx = fmaf(a.cz[n], qx[R + n] - qx[R - n + 1], dzvx);
-            if (Y) {
-                dxvy = fmaf(a.cx[n], Ty[n - 1] - Ty[-n], dxvy);
-                eyy = fmaf(a.cy[n], Ty[n * XW] - Ty[(1 - n) * XW], eyy);
-                dyvx = fmaf(a.cy[n], Tx[(n - 1) * XW] - Tx[-n * XW], dyvx);
-                dyvz = fmaf(a.cy[n], Tz[(n - 1) * XW] - Tz[-n * XW], dyvz);
-                dzvy = fmaf(a.cz[n], qy[R + n] - qy[R - n + 1], dzvy);
-            }
+            dxvy = fmaf(a.cx[n], Ty[n - 1] - Ty[-n], dxvy);
+            eyy = fmaf(a.cy[n], Ty[n * XW] - Ty[(1 - n) * XW], eyy);
+            dyvx = fmaf(a.cy[n], Tx[(n - 1) * XW] - Tx[-n * XW], dyvx);
+            dyvz = fmaf(a.cy[n], Tz[(n - 1) * XW] - Tz[-n * XW], dyvz);
+            dzvy = fmaf(a.cz[n], qy[R + n] - qy[R - n + 1], dzvy);
         }
 
         if (act) {
@@ -398,11 +402,9 @@ __device__ __forceinline__ void stress_body(const StressMaps& maps, const KArgs&
                     a.psi[P_DXVZ][x] = p1;
                     exx += p0;
                     dxvz += p1;
-                    if (Y) {
-                        float p2 = fmaf(bxh, Ps[(PX + 2) * CB + cell], axh * dxvy);
-                        a.psi[P_DXVY][x] = p2;
-                        dxvy += p2;
-                    }
+                    float p2 = fmaf(bxh, Ps[(PX + 2) * CB + cell], axh * dxvy);
+                    a.psi[P_DXVY][x] = p2;
+                    dxvy += p2;
                 }
                 if (iny) {
                     const int y = (k * WY + sly) * a.nx + i;
@@ -427,39 +429,33 @@ __device__ __forceinline__ void stress_body(const StressMaps& maps, const KArgs&
                     a.psi[P_DZVX][z] = p1;
                     ezz += p0;
                     dzvx += p1;
-                    if (Y) {
-                        float p2 = fmaf(bzh, Ps[(PZ + 2) * CB + cell], azh * dzvy);
-                        a.psi[P_DZVY][z] = p2;
-                        dzvy += p2;
-                    }
+                    float p2 = fmaf(bzh, Ps[(PZ + 2) * CB + cell], azh * dzvy);
+                    a.psi[P_DZVY][z] = p2;
+                    dzvy += p2;
                 }
             }
             float g1, g2;
-            damping<Y>(a, CPML, i, j, k, g1, g2);
+            damping<true>(a, CPML, i, j, k, g1, g2);
             const float M = Cc[C_M * CB + cell], U = Cc[C_MU * CB + cell];
             const float L = M - 2.f * U;
             const float dt = a.dt;
             float oxx = Cc[0 * CB + cell], ozz = Cc[1 * CB + cell], oxz = Cc[2 * CB + cell];
             float oyy = 0.f, oxy = 0.f, oyz = 0.f;
-            if (Y) {
-                oyy = Cc[3 * CB + cell];
-                oxy = Cc[4 * CB + cell];
-                oyz = Cc[5 * CB + cell];
-            }
+            oyy = Cc[3 * CB + cell];
+            oxy = Cc[4 * CB + cell];
+            oyz = Cc[5 * CB + cell];
             if (src_here && k == a.ssz) {     // add_source_3D into txx, tyy, tzz
                 oxx += wsrc;
                 ozz += wsrc;
-                if (Y) oyy += wsrc;
+                oyy += wsrc;
             }
             if (ok) {
                 sig[0][c] = g1 * (g2 * oxx + dt * (M * exx + L * (eyy + ezz)));
                 sig[1][c] = g1 * (g2 * ozz + dt * (M * ezz + L * (exx + eyy)));
                 sig[2][c] = g1 * (g2 * oxz + dt * U * (dzvx + dxvz));
-                if (Y) {
-                    sig[3][c] = g1 * (g2 * oyy + dt * (M * eyy + L * (exx + ezz)));
-                    sig[4][c] = g1 * (g2 * oxy + dt * U * (dyvx + dxvy));
-                    sig[5][c] = g1 * (g2 * oyz + dt * U * (dzvy + dyvz));
-                }
+                sig[3][c] = g1 * (g2 * oyy + dt * (M * eyy + L * (exx + ezz)));
+                sig[4][c] = g1 * (g2 * oxy + dt * U * (dyvx + dxvy));
+                sig[5][c] = g1 * (g2 * oyz + dt * U * (dzvy + dyvz));
                 if (PS) tp[c] = g1 * (g2 * Cc[C_TP * CB + cell] + dt * M * (exx + eyy + ezz));
             }
         }
@@ -468,7 +464,7 @@ __device__ __forceinline__ void stress_body(const StressMaps& maps, const KArgs&
         for (int q = 0; q < 2 * R; q++) {
             qx[q] = qx[q + 1];
             qz[q] = qz[q + 1];
-            if (Y) qy[q] = qy[q + 1];
+            qy[q] = qy[q + 1];
         }
         cpa_wait_1();   // plane t+1's memory variables have landed
         __syncwarp();
@@ -480,47 +476,47 @@ __device__ __forceinline__ void stress_body(const StressMaps& maps, const KArgs&
 // ---------------------------------------------------------------------------
 // Velocity kernel
 // ---------------------------------------------------------------------------
-template <int R, bool Y, bool CPML, int EPI>
+template <int R, bool CPML, int EPI>
 struct VelShape {
-    using B = Boxes<R, Y>;
+    using B = Boxes<R>;
     static constexpr bool PS = (EPI != EPI_NONE);
-    // tiles: txx (X), txz (X), txy (XY), tyy (Y), tyz (Y), tp (XY; X in 2D)
+    // tiles: txx (X), txz (X), txy (XY), tyy (Y), tyz (Y), tp (XY)
     static constexpr int O_TXX = 0;
     static constexpr int O_TXZ = O_TXX + B::XP;
     static constexpr int O_TXY = O_TXZ + B::XP;
-    static constexpr int O_TYY = O_TXY + (Y ? B::XYP : 0);
-    static constexpr int O_TYZ = O_TYY + (Y ? B::Yb : 0);
-    static constexpr int O_TP = O_TYZ + (Y ? B::Yb : 0);
+    static constexpr int O_TYY = O_TXY + B::XYP;
+    static constexpr int O_TYZ = O_TYY + B::Yb;
+    static constexpr int O_TP = O_TYZ + B::Yb;
     static constexpr int O_FR = O_TP + (PS ? B::XYP : 0);
     // fronts: txz, tzz, (tyz), (tp)
-    static constexpr int NFR = 2 + (Y ? 1 : 0) + (PS ? 1 : 0);
-    static constexpr int FR_TYZ = 2, FR_TP = Y ? 3 : 2;
+    static constexpr int NFR = PS ? 4 : 3;
+    static constexpr int FR_TYZ = 2, FR_TP = 3;
     // cells: vx, vz, (vy), (vxp, vzp, (vyp)), b, (excitation)
     static constexpr int C_VX = 0, C_VZ = 1, C_VY = 2;
-    static constexpr int C_PX = Y ? 3 : 2;
+    static constexpr int C_PX = 3;
     static constexpr int C_PZ = C_PX + 1, C_PY = C_PX + 2;
-    static constexpr int C_B = PS ? C_PX + (Y ? 3 : 2) : C_PX;
+    static constexpr int C_B = PS ? C_PX + 3 : C_PX;
     static constexpr int C_EX = C_B + 1;
     static constexpr int NC = C_B + 1 + (PS ? 1 : 0);
     static constexpr int O_C = O_FR + NFR * B::C;
     static constexpr int STAGE = O_C + NC * B::C;
     static constexpr unsigned TX_BYTES =    // box bytes (slots may be padded)
-        4u * (2 * B::X + (Y ? B::XY + 2 * B::Yb : 0) + (PS ? B::XY : 0) + NFR * B::C + NC * B::C);
+        4u * (2 * B::X + B::XY + 2 * B::Yb + (PS ? B::XY : 0) + NFR * B::C + NC * B::C);
     static_assert(B::C % 32 == 0 && O_TXZ % 32 == 0 && O_TXY % 32 == 0 && O_TYY % 32 == 0 &&
                       O_TYZ % 32 == 0 && O_TP % 32 == 0 && O_FR % 32 == 0 && O_C % 32 == 0 &&
                       STAGE % 32 == 0,
                   "TMA boxes must start on 128-byte boundaries");
-    static constexpr int NP = CPML ? (Y ? 9 : 4) : 0;
+    static constexpr int NP = CPML ? 9 : 0;
     static constexpr int PSI = NP * B::C;
     static constexpr int NS = 3;   // ring stages (4 would not leave room for 2 CTAs per SM)
     static constexpr size_t BYTES = 4 * (size_t)(NS * STAGE + 3 * PSI) + 16 * NS;
 };
 
 // The velocity step of one CTA (tile and chunk as in stress_body).
-template <int R, bool Y, bool CPML, int EPI, bool REC>
+template <int R, bool CPML, int EPI, bool REC>
 __device__ __forceinline__ void velocity_body(const VelMaps& maps, const KArgs& a, int bz)
 {
-    using VS = VelShape<R, Y, CPML, EPI>;
+    using VS = VelShape<R, CPML, EPI>;
     using B = typename VS::B;
     constexpr int NS = VS::NS;
     constexpr bool PS = VS::PS;
@@ -538,11 +534,11 @@ __device__ __forceinline__ void velocity_body(const VelMaps& maps, const KArgs& 
     const int nk = k1 - k0;
     const int sy = (int)a.sy, sz = (int)a.sz;
     const bool act = (i < a.nx) && (j < a.ny);
-    const int it = __ldg(a.it_ptr);
+    const int it = step_index(a);
     const int rec = ((REC || EPI == EPI_IMAGE) && act) ? receiver_index(a, i, j) : -1;
     const long long nrec = (long long)a.nrx * a.nry;
     const int cell = ty * TX + tx;
-    const int gx = i0 + XH, gy = j0 + (Y ? R : 0), gz0 = k0 + R;
+    const int gx = i0 + XH, gy = j0 + R, gz0 = k0 + R;
     const int cj = j * sy + i;
 
     float* vx = a.f[F_VX];
@@ -561,11 +557,9 @@ __device__ __forceinline__ void velocity_body(const VelMaps& maps, const KArgs& 
         mbar_expect_tx(bar, VS::TX_BYTES);
         tma3(S + VS::O_TXX, &maps.txx, gx - XB, gy, z, bar);
         tma3(S + VS::O_TXZ, &maps.txz, gx - XB, gy, z, bar);
-        if (Y) {
-            tma3(S + VS::O_TXY, &maps.txy, gx - XB, gy - R, z, bar);
-            tma3(S + VS::O_TYY, &maps.tyy, gx, gy - R, z, bar);
-            tma3(S + VS::O_TYZ, &maps.tyz, gx, gy - R, z, bar);
-        }
+        tma3(S + VS::O_TXY, &maps.txy, gx - XB, gy - R, z, bar);
+        tma3(S + VS::O_TYY, &maps.tyy, gx, gy - R, z, bar);
+        tma3(S + VS::O_TYZ, &maps.tyz, gx, gy - R, z, bar);
         if (PS) tma3(S + VS::O_TP, &maps.tp, gx - XB, gy - B::YB, z, bar);
 #pragma unroll
         for (int f = 0; f < VS::NFR; f++) tma3(S + VS::O_FR + f * CB, &maps.fr[f], gx, gy, z + R, bar);
@@ -576,7 +570,7 @@ __device__ __forceinline__ void velocity_body(const VelMaps& maps, const KArgs& 
 
     const int WX = a.w[0] + a.w[1], WY = a.w[2] + a.w[3];
     const bool inx = CPML && act && (i < a.w[0] || i >= a.nx - a.w[1]);
-    const bool iny = CPML && Y && act && (j < a.w[2] || j >= a.ny - a.w[3]);
+    const bool iny = CPML && act && (j < a.w[2] || j >= a.ny - a.w[3]);
     const int slx = i < a.w[0] ? i : i - a.nx + WX;
     const int sly = j < a.w[2] ? j : j - a.ny + WY;
     float axf = 0.f, bxf = 1.f, axh = 0.f, bxh = 1.f, ayf = 0.f, byf = 1.f, ayh = 0.f, byh = 1.f;
@@ -589,7 +583,7 @@ __device__ __forceinline__ void velocity_body(const VelMaps& maps, const KArgs& 
         ayh = __ldg(a.pa[1][1] + j); byh = __ldg(a.pb[1][1] + j);
     }
     // psi slots: x: DXTXX DXTXZ (DXTXY), y: DYTXY DYTYY DYTYZ, z: DZTXZ DZTZZ (DZTYZ)
-    constexpr int PX = 0, PY = Y ? 3 : 2, PZ = Y ? 6 : 2;
+    constexpr int PX = 0, PY = 3, PZ = 6;
     auto issue_psi = [&](int p, int buf) {
         if (!CPML) return;
         float* Ps = psibuf + buf * VS::PSI;
@@ -597,7 +591,7 @@ __device__ __forceinline__ void velocity_body(const VelMaps& maps, const KArgs& 
             const int x = (p * a.ny + j) * WX + slx;
             cpa4(&Ps[(PX + 0) * CB + cell], a.psi[P_DXTXX] + x);
             cpa4(&Ps[(PX + 1) * CB + cell], a.psi[P_DXTXZ] + x);
-            if (Y) cpa4(&Ps[(PX + 2) * CB + cell], a.psi[P_DXTXY] + x);
+            cpa4(&Ps[(PX + 2) * CB + cell], a.psi[P_DXTXY] + x);
         }
         if (iny) {
             const int y = (p * WY + sly) * a.nx + i;
@@ -610,7 +604,7 @@ __device__ __forceinline__ void velocity_body(const VelMaps& maps, const KArgs& 
             const int z = (sl * a.ny + j) * a.nx + i;
             cpa4(&Ps[(PZ + 0) * CB + cell], a.psi[P_DZTXZ] + z);
             cpa4(&Ps[(PZ + 1) * CB + cell], a.psi[P_DZTZZ] + z);
-            if (Y) cpa4(&Ps[(PZ + 2) * CB + cell], a.psi[P_DZTYZ] + z);
+            cpa4(&Ps[(PZ + 2) * CB + cell], a.psi[P_DZTYZ] + z);
         }
         cpa_commit();
     };
@@ -639,7 +633,7 @@ __device__ __forceinline__ void velocity_body(const VelMaps& maps, const KArgs& 
         const int cc = (k0 + q - R) * sz + cj;
         qxz[q] = txz[cc];
         qzz[q] = tzz[cc];
-        if (Y) qyz[q] = tyz[cc];
+        qyz[q] = tyz[cc];
         if (PS) qtp[q] = tp[cc];
     }
     issue_psi(k0, 0);
@@ -664,7 +658,7 @@ __device__ __forceinline__ void velocity_body(const VelMaps& maps, const KArgs& 
         const float* Ps = psibuf + (t % 3) * VS::PSI;
         qxz[2 * R] = S[VS::O_FR + 0 * CB + cell];
         qzz[2 * R] = S[VS::O_FR + 1 * CB + cell];
-        if (Y) qyz[2 * R] = S[VS::O_FR + VS::FR_TYZ * CB + cell];
+        qyz[2 * R] = S[VS::O_FR + VS::FR_TYZ * CB + cell];
         if (PS) qtp[2 * R] = S[VS::O_FR + VS::FR_TP * CB + cell];
         const float* Txx = S + VS::O_TXX + ty * XW + tx + XB;
         const float* Txz = S + VS::O_TXZ + ty * XW + tx + XB;
@@ -683,17 +677,15 @@ __device__ __forceinline__ void velocity_body(const VelMaps& maps, const KArgs& 
             dxtxz = fmaf(a.cx[n], Txz[n] - Txz[1 - n], dxtxz);
             dztxz = fmaf(a.cz[n], qxz[R + n - 1] - qxz[R - n], dztxz);
             dztzz = fmaf(a.cz[n], qzz[R + n] - qzz[R - n + 1], dztzz);
-            if (Y) {
-                dytxy = fmaf(a.cy[n], Txy[n * XW] - Txy[(1 - n) * XW], dytxy);
-                dxtxy = fmaf(a.cx[n], Txy[n] - Txy[1 - n], dxtxy);
-                dytyy = fmaf(a.cy[n], Tyy[(n - 1) * TX] - Tyy[-n * TX], dytyy);
-                dztyz = fmaf(a.cz[n], qyz[R + n - 1] - qyz[R - n], dztyz);
-                dytyz = fmaf(a.cy[n], Tyz[n * TX] - Tyz[(1 - n) * TX], dytyz);
-            }
+            dytxy = fmaf(a.cy[n], Txy[n * XW] - Txy[(1 - n) * XW], dytxy);
+            dxtxy = fmaf(a.cx[n], Txy[n] - Txy[1 - n], dxtxy);
+            dytyy = fmaf(a.cy[n], Tyy[(n - 1) * TX] - Tyy[-n * TX], dytyy);
+            dztyz = fmaf(a.cz[n], qyz[R + n - 1] - qyz[R - n], dztyz);
+            dytyz = fmaf(a.cy[n], Tyz[n * TX] - Tyz[(1 - n) * TX], dytyz);
             if (PS) {
                 dxtp = fmaf(a.cx[n], Ttp[n - 1] - Ttp[-n], dxtp);
                 dztp = fmaf(a.cz[n], qtp[R + n] - qtp[R - n + 1], dztp);
-                if (Y) dytp = fmaf(a.cy[n], Ttp[(n - 1) * XW] - Ttp[-n * XW], dytp);
+                dytp = fmaf(a.cy[n], Ttp[(n - 1) * XW] - Ttp[-n * XW], dytp);
             }
         }
 
@@ -708,11 +700,9 @@ __device__ __forceinline__ void velocity_body(const VelMaps& maps, const KArgs& 
                     a.psi[P_DXTXZ][x] = p1;
                     dxtxx += p0;
                     dxtxz += p1;
-                    if (Y) {
-                        float p2 = fmaf(bxf, Ps[(PX + 2) * CB + cell], axf * dxtxy);
-                        a.psi[P_DXTXY][x] = p2;
-                        dxtxy += p2;
-                    }
+                    float p2 = fmaf(bxf, Ps[(PX + 2) * CB + cell], axf * dxtxy);
+                    a.psi[P_DXTXY][x] = p2;
+                    dxtxy += p2;
                 }
                 if (iny) {
                     const int y = (k * WY + sly) * a.nx + i;
@@ -737,32 +727,30 @@ __device__ __forceinline__ void velocity_body(const VelMaps& maps, const KArgs& 
                     a.psi[P_DZTZZ][z] = p1;
                     dztxz += p0;
                     dztzz += p1;
-                    if (Y) {
-                        float p2 = fmaf(bzf, Ps[(PZ + 2) * CB + cell], azf * dztyz);
-                        a.psi[P_DZTYZ][z] = p2;
-                        dztyz += p2;
-                    }
+                    float p2 = fmaf(bzf, Ps[(PZ + 2) * CB + cell], azf * dztyz);
+                    a.psi[P_DZTYZ][z] = p2;
+                    dztyz += p2;
                 }
             }
             float g1, g2;
-            damping<Y>(a, CPML, i, j, k, g1, g2);
+            damping<true>(a, CPML, i, j, k, g1, g2);
             const float b = Cc[VS::C_B * CB + cell];
             const float db = a.dt * b;
             float nvx = g1 * (g2 * Cc[VS::C_VX * CB + cell] + db * (dxtxx + dytxy + dztxz));
             float nvz = g1 * (g2 * Cc[VS::C_VZ * CB + cell] + db * (dxtxz + dytyz + dztzz));
             float nvy = 0.f;
-            if (Y) nvy = g1 * (g2 * Cc[VS::C_VY * CB + cell] + db * (dxtxy + dytyy + dztyz));
+            nvy = g1 * (g2 * Cc[VS::C_VY * CB + cell] + db * (dxtxy + dytyy + dztyz));
             float npx = 0.f, npy = 0.f, npz = 0.f;
             if (PS) {
                 // decoupled P velocity from the P-stress gradient (role of fwd_vxp_vzp_3D,
                 // 3D_forward_or_back_together.cu:118); S velocity = v - v_P
                 npx = g1 * (g2 * Cc[VS::C_PX * CB + cell] + db * dxtp);
                 npz = g1 * (g2 * Cc[VS::C_PZ * CB + cell] + db * dztp);
-                if (Y) npy = g1 * (g2 * Cc[VS::C_PY * CB + cell] + db * dytp);
+                npy = g1 * (g2 * Cc[VS::C_PY * CB + cell] + db * dytp);
                 if (ok) {
                     vxp[c] = npx;
                     vzp[c] = npz;
-                    if (Y) vyp[c] = npy;
+                    vyp[c] = npy;
                 }
             }
             if (EPI == EPI_EXCITE && ok) {
@@ -773,7 +761,7 @@ __device__ __forceinline__ void velocity_body(const VelMaps& maps, const KArgs& 
                     a.ex_amp2[c] = a2;
                     a.ex_time[c] = it;
                     a.ex_v[0][c] = npx;
-                    if (Y) a.ex_v[1][c] = npy;
+                    a.ex_v[1][c] = npy;
                     a.ex_v[2][c] = npz;
                     a.ex_tp[c] = qtp[R];
                 }
@@ -782,7 +770,7 @@ __device__ __forceinline__ void velocity_body(const VelMaps& maps, const KArgs& 
                 // imaging_inner_product_ex / imaging_correlation_ex
                 // (2D_elastic_RTM/elastic_2D_kernel_3.cu:542-576) at it == excitation time
                 if (__float_as_int(Cc[VS::C_EX * CB + cell]) == it) {
-                    float ex = a.ex_v[0][c], ey = Y ? a.ex_v[1][c] : 0.f, ez = a.ex_v[2][c];
+                    float ex = a.ex_v[0][c], ey = a.ex_v[1][c], ez = a.ex_v[2][c];
                     float den = ex * ex + ey * ey + ez * ez;
                     if (den > 0.f) {   // a true division: 1/den overflows for denormal den
                         if (a.img[0]) a.img[0][c] = (ex * npx + ey * npy + ez * npz) / den;
@@ -799,18 +787,18 @@ __device__ __forceinline__ void velocity_body(const VelMaps& maps, const KArgs& 
                     if (a.inject_mode == 2) {
                         nvx = d[0];
                         nvz = d[2 * cs];
-                        if (Y) nvy = d[cs];
+                        nvy = d[cs];
                     } else {
                         nvx += d[0];
                         nvz += d[2 * cs];
-                        if (Y) nvy += d[cs];
+                        nvy += d[cs];
                     }
                 }
             }
             if (ok) {
                 vx[c] = nvx;
                 vz[c] = nvz;
-                if (Y) vy[c] = nvy;
+                vy[c] = nvy;
             }
             if (REC && ok && rec >= 0 && k == a.rz) {
                 // write_or_add_shot_3D_surface_three, record flag 0 (:127)
@@ -826,7 +814,7 @@ __device__ __forceinline__ void velocity_body(const VelMaps& maps, const KArgs& 
         for (int q = 0; q < 2 * R; q++) {
             qxz[q] = qxz[q + 1];
             qzz[q] = qzz[q + 1];
-            if (Y) qyz[q] = qyz[q + 1];
+            qyz[q] = qyz[q + 1];
             if (PS) qtp[q] = qtp[q + 1];
         }
         cpa_wait_1();   // plane t+1's memory variables have landed
@@ -839,18 +827,18 @@ __device__ __forceinline__ void velocity_body(const VelMaps& maps, const KArgs& 
 // ---------------------------------------------------------------------------
 // Kernels
 // ---------------------------------------------------------------------------
-template <int R, bool Y, bool CPML, bool PS>
-__global__ void __launch_bounds__(TX * ((Y ? TY3 : TY2) + 1), Y ? CTAS3 : 1)
+template <int R, bool CPML, bool PS>
+__global__ void __launch_bounds__(TX * (TY3 + 1), CTAS3)
 k_stress(const __grid_constant__ StressMaps maps, const __grid_constant__ KArgs a)
 {
-    stress_body<R, Y, CPML, PS>(maps, a, blockIdx.z);
+    stress_body<R, CPML, PS>(maps, a, blockIdx.z);
 }
 
-template <int R, bool Y, bool CPML, int EPI, bool REC>
-__global__ void __launch_bounds__(TX * ((Y ? TY3 : TY2) + 1), Y ? CTAS3 : 1)
+template <int R, bool CPML, int EPI, bool REC>
+__global__ void __launch_bounds__(TX * (TY3 + 1), CTAS3)
 k_velocity(const __grid_constant__ VelMaps maps, const __grid_constant__ KArgs a)
 {
-    velocity_body<R, Y, CPML, EPI, REC>(maps, a, blockIdx.z);
+    velocity_body<R, CPML, EPI, REC>(maps, a, blockIdx.z);
 }
 
 // Several 3D shots in one launch (the RTM passes: P/S split on, excitation or
@@ -864,8 +852,8 @@ __global__ void __launch_bounds__(TX * (TY3 + 1), CTAS3) k_stress_multi(const __
 {
     const int shot = blockIdx.z / P.chunks;
     const KArgs& a = P.a[shot];
-    if ((int)blockIdx.x * TX >= a.nx || (int)blockIdx.y * TY3 >= a.ny || __ldg(a.it_ptr) >= a.it_hi) return;
-    stress_body<R, true, CPML, true>(P.m[shot], a, blockIdx.z - shot * P.chunks);
+    if ((int)blockIdx.x * TX >= a.nx || (int)blockIdx.y * TY3 >= a.ny || step_index(a) >= a.it_hi) return;
+    stress_body<R, CPML, true>(P.m[shot], a, blockIdx.z - shot * P.chunks);
 }
 
 template <int R, bool CPML, int EPI>
@@ -873,8 +861,8 @@ __global__ void __launch_bounds__(TX * (TY3 + 1), CTAS3) k_velocity_multi(const 
 {
     const int shot = blockIdx.z / P.chunks;
     const KArgs& a = P.a[shot];
-    if ((int)blockIdx.x * TX >= a.nx || (int)blockIdx.y * TY3 >= a.ny || __ldg(a.it_ptr) >= a.it_hi) return;
-    velocity_body<R, true, CPML, EPI, false>(P.m[shot], a, blockIdx.z - shot * P.chunks);
+    if ((int)blockIdx.x * TX >= a.nx || (int)blockIdx.y * TY3 >= a.ny || step_index(a) >= a.it_hi) return;
+    velocity_body<R, CPML, EPI, false>(P.m[shot], a, blockIdx.z - shot * P.chunks);
 }
 
 // ---------------------------------------------------------------------------
@@ -893,66 +881,49 @@ static cudaError_t launch_dyn(dim3 grid, dim3 block, size_t smem, const MAPS& m,
     return cudaGetLastError();
 }
 
-template <int R, bool Y, bool C, bool P>
-static cudaError_t launch_stress_y(dim3 grid, dim3 block, const StressMaps& m, const KArgs& a,
-                                   cudaStream_t st)
+inline dim3 step_grid(const Geom& g, const KArgs& a)
 {
-    return launch_dyn<StressMaps, k_stress<R, Y, C, P>>(grid, block,
-                                                         StressShape<R, Y, C, P>::BYTES, m, a, st);
+    return dim3((g.nx + TX - 1) / TX, (g.ny + TY3 - 1) / TY3, (g.nz + a.kchunk - 1) / a.kchunk);
 }
 
-inline dim3 step_grid(const Geom& g, const KArgs& a, int tyb)
+template <int R, bool C, bool P>
+static cudaError_t launch_stress_c(const Geom& g, const StressMaps& m, const KArgs& a, cudaStream_t st)
 {
-    return dim3((g.nx + TX - 1) / TX, (g.ny + tyb - 1) / tyb, (g.nz + a.kchunk - 1) / a.kchunk);
+    return launch_dyn<StressMaps, k_stress<R, C, P>>(step_grid(g, a), dim3(TX, TY3 + 1),
+                                                     StressShape<R, C, P>::BYTES, m, a, st);
 }
 
 template <int R>
 cudaError_t launch_stress_t(const Geom& g, const KArgs& a, const StressMaps& m, bool cpml, bool ps,
                             cudaStream_t st)
 {
-    const bool Y = !g.two_d;
-    const int tyb = Y ? TY3 : TY2;
-    dim3 block(TX, tyb + 1), grid = step_grid(g, a, tyb);
-    if (Y) {
-        if (cpml) return ps ? launch_stress_y<R, true, true, true>(grid, block, m, a, st)
-                            : launch_stress_y<R, true, true, false>(grid, block, m, a, st);
-        return ps ? launch_stress_y<R, true, false, true>(grid, block, m, a, st)
-                  : launch_stress_y<R, true, false, false>(grid, block, m, a, st);
-    }
-    if (cpml) return ps ? launch_stress_y<R, false, true, true>(grid, block, m, a, st)
-                        : launch_stress_y<R, false, true, false>(grid, block, m, a, st);
-    return ps ? launch_stress_y<R, false, false, true>(grid, block, m, a, st)
-              : launch_stress_y<R, false, false, false>(grid, block, m, a, st);
+    if (cpml) return ps ? launch_stress_c<R, true, true>(g, m, a, st) : launch_stress_c<R, true, false>(g, m, a, st);
+    return ps ? launch_stress_c<R, false, true>(g, m, a, st) : launch_stress_c<R, false, false>(g, m, a, st);
 }
 
-template <int R, bool Y, bool C>
-static cudaError_t launch_velocity_y(dim3 grid, dim3 block, const VelMaps& m, const KArgs& a,
-                                     int epi, bool rec, cudaStream_t st)
+template <int R, bool C, int EPI, bool REC>
+static cudaError_t launch_velocity_e(const Geom& g, const VelMaps& m, const KArgs& a, cudaStream_t st)
 {
-    if (epi == EPI_EXCITE)
-        return launch_dyn<VelMaps, k_velocity<R, Y, C, EPI_EXCITE, false>>(
-            grid, block, VelShape<R, Y, C, EPI_EXCITE>::BYTES, m, a, st);
-    if (epi == EPI_IMAGE)
-        return launch_dyn<VelMaps, k_velocity<R, Y, C, EPI_IMAGE, false>>(
-            grid, block, VelShape<R, Y, C, EPI_IMAGE>::BYTES, m, a, st);
-    if (rec)
-        return launch_dyn<VelMaps, k_velocity<R, Y, C, EPI_NONE, true>>(
-            grid, block, VelShape<R, Y, C, EPI_NONE>::BYTES, m, a, st);
-    return launch_dyn<VelMaps, k_velocity<R, Y, C, EPI_NONE, false>>(
-        grid, block, VelShape<R, Y, C, EPI_NONE>::BYTES, m, a, st);
+    return launch_dyn<VelMaps, k_velocity<R, C, EPI, REC>>(step_grid(g, a), dim3(TX, TY3 + 1),
+                                                           VelShape<R, C, EPI>::BYTES, m, a, st);
+}
+
+template <int R, bool C>
+static cudaError_t launch_velocity_c(const Geom& g, const VelMaps& m, const KArgs& a, int epi, bool rec,
+                                     cudaStream_t st)
+{
+    if (epi == EPI_EXCITE) return launch_velocity_e<R, C, EPI_EXCITE, false>(g, m, a, st);
+    if (epi == EPI_IMAGE) return launch_velocity_e<R, C, EPI_IMAGE, false>(g, m, a, st);
+    if (rec) return launch_velocity_e<R, C, EPI_NONE, true>(g, m, a, st);
+    return launch_velocity_e<R, C, EPI_NONE, false>(g, m, a, st);
 }
 
 template <int R>
 cudaError_t launch_velocity_t(const Geom& g, const KArgs& a, const VelMaps& m, bool cpml, int epi,
                               bool rec, cudaStream_t st)
 {
-    const bool Y = !g.two_d;
-    const int tyb = Y ? TY3 : TY2;
-    dim3 block(TX, tyb + 1), grid = step_grid(g, a, tyb);
-    if (Y) return cpml ? launch_velocity_y<R, true, true>(grid, block, m, a, epi, rec, st)
-                       : launch_velocity_y<R, true, false>(grid, block, m, a, epi, rec, st);
-    return cpml ? launch_velocity_y<R, false, true>(grid, block, m, a, epi, rec, st)
-                : launch_velocity_y<R, false, false>(grid, block, m, a, epi, rec, st);
+    return cpml ? launch_velocity_c<R, true>(g, m, a, epi, rec, st)
+                : launch_velocity_c<R, false>(g, m, a, epi, rec, st);
 }
 
 template <typename P, void (*K)(P)>
@@ -969,8 +940,8 @@ template <int R>
 cudaError_t launch_stress_multi_t(dim3 grid, const StressMulti& P, bool cpml, cudaStream_t st)
 {
     if (cpml)
-        return launch_dyn_multi<StressMulti, k_stress_multi<R, true>>(grid, StressShape<R, true, true, true>::BYTES, P, st);
-    return launch_dyn_multi<StressMulti, k_stress_multi<R, false>>(grid, StressShape<R, true, false, true>::BYTES, P, st);
+        return launch_dyn_multi<StressMulti, k_stress_multi<R, true>>(grid, StressShape<R, true, true>::BYTES, P, st);
+    return launch_dyn_multi<StressMulti, k_stress_multi<R, false>>(grid, StressShape<R, false, true>::BYTES, P, st);
 }
 
 template <int R>
@@ -978,14 +949,14 @@ cudaError_t launch_velocity_multi_t(dim3 grid, const VelMulti& P, bool cpml, int
 {
     if (epi == EPI_EXCITE)
         return cpml ? launch_dyn_multi<VelMulti, k_velocity_multi<R, true, EPI_EXCITE>>(
-                          grid, VelShape<R, true, true, EPI_EXCITE>::BYTES, P, st)
+                          grid, VelShape<R, true, EPI_EXCITE>::BYTES, P, st)
                     : launch_dyn_multi<VelMulti, k_velocity_multi<R, false, EPI_EXCITE>>(
-                          grid, VelShape<R, true, false, EPI_EXCITE>::BYTES, P, st);
+                          grid, VelShape<R, false, EPI_EXCITE>::BYTES, P, st);
     if (epi == EPI_IMAGE)
         return cpml ? launch_dyn_multi<VelMulti, k_velocity_multi<R, true, EPI_IMAGE>>(
-                          grid, VelShape<R, true, true, EPI_IMAGE>::BYTES, P, st)
+                          grid, VelShape<R, true, EPI_IMAGE>::BYTES, P, st)
                     : launch_dyn_multi<VelMulti, k_velocity_multi<R, false, EPI_IMAGE>>(
-                          grid, VelShape<R, true, false, EPI_IMAGE>::BYTES, P, st);
+                          grid, VelShape<R, false, EPI_IMAGE>::BYTES, P, st);
     return cudaErrorInvalidValue;
 }
 

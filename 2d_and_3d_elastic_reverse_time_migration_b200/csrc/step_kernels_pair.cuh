@@ -28,6 +28,7 @@
 #pragma once
 
 #include "step_kernels.cuh"
+#include "step_kernels_2d.cuh"
 
 namespace ertm {
 
@@ -121,7 +122,7 @@ template <int R, bool CPML, bool PS>
 __global__ void __launch_bounds__(32 * (PAIR_WARPS + 1), CTAS3)
 k_stress2(const __grid_constant__ StressMaps maps, const KArgs a)
 {
-    using SS = StressShape<R, true, CPML, PS>;
+    using SS = StressShape<R, CPML, PS>;
     using B = typename SS::B;
     constexpr int NS = SS::NS;
     constexpr int XB = B::XB, XW = B::XW, CB = B::C;
@@ -143,7 +144,7 @@ k_stress2(const __grid_constant__ StressMaps maps, const KArgs a)
     const int nk = k1 - k0;
     const int sy = (int)a.sy, sz = (int)a.sz;
     const bool act[2] = {(i < a.nx) && (j < a.ny), (i + 1 < a.nx) && (j < a.ny)};
-    const int it = __ldg(a.it_ptr);
+    const int it = step_index(a);
     const bool src_on = (it >= 0) && (it < a.nw);
     const float wsrc = src_on ? __ldg(a.wavelet + it) : 0.f;
     const int cell = r * TX + ci;                // C-box index of the first cell
@@ -408,7 +409,7 @@ template <int R, bool CPML, int EPI, bool REC>
 __global__ void __launch_bounds__(32 * (PAIR_WARPS + 1), CTAS3)
 k_velocity2(const __grid_constant__ VelMaps maps, const KArgs a)
 {
-    using VS = VelShape<R, true, CPML, EPI>;
+    using VS = VelShape<R, CPML, EPI>;
     using B = typename VS::B;
     constexpr int NS = VS::NS;
     constexpr bool PS = VS::PS;
@@ -429,7 +430,7 @@ k_velocity2(const __grid_constant__ VelMaps maps, const KArgs a)
     const int nk = k1 - k0;
     const int sy = (int)a.sy, sz = (int)a.sz;
     const bool act[2] = {(i < a.nx) && (j < a.ny), (i + 1 < a.nx) && (j < a.ny)};
-    const int it = __ldg(a.it_ptr);
+    const int it = step_index(a);
     int rec[2];
 #pragma unroll
     for (int e = 0; e < 2; e++) rec[e] = ((REC || EPI == EPI_IMAGE) && act[e]) ? receiver_index(a, i + e, j) : -1;
@@ -767,7 +768,7 @@ template <int R, bool C, bool P>
 static cudaError_t launch_stress_pair(dim3 grid, const StressMaps& m, const KArgs& a, cudaStream_t st)
 {
     return launch_dyn<StressMaps, k_stress2<R, C, P>>(grid, dim3(32, PAIR_WARPS + 1),
-                                                      StressShape<R, true, C, P>::BYTES, m, a, st);
+                                                      StressShape<R, C, P>::BYTES, m, a, st);
 }
 
 template <int R, bool C>
@@ -777,25 +778,26 @@ static cudaError_t launch_velocity_pair(dim3 grid, const VelMaps& m, const KArgs
     const dim3 block(32, PAIR_WARPS + 1);
     if (epi == EPI_EXCITE)
         return launch_dyn<VelMaps, k_velocity2<R, C, EPI_EXCITE, false>>(
-            grid, block, VelShape<R, true, C, EPI_EXCITE>::BYTES, m, a, st);
+            grid, block, VelShape<R, C, EPI_EXCITE>::BYTES, m, a, st);
     if (epi == EPI_IMAGE)
         return launch_dyn<VelMaps, k_velocity2<R, C, EPI_IMAGE, false>>(
-            grid, block, VelShape<R, true, C, EPI_IMAGE>::BYTES, m, a, st);
+            grid, block, VelShape<R, C, EPI_IMAGE>::BYTES, m, a, st);
     if (rec)
         return launch_dyn<VelMaps, k_velocity2<R, C, EPI_NONE, true>>(
-            grid, block, VelShape<R, true, C, EPI_NONE>::BYTES, m, a, st);
+            grid, block, VelShape<R, C, EPI_NONE>::BYTES, m, a, st);
     return launch_dyn<VelMaps, k_velocity2<R, C, EPI_NONE, false>>(
-        grid, block, VelShape<R, true, C, EPI_NONE>::BYTES, m, a, st);
+        grid, block, VelShape<R, C, EPI_NONE>::BYTES, m, a, st);
 }
 
 // 3D grids: the pair kernels when KArgs::pairs is set, else the single-cell kernels;
-// 2D grids: the single-cell kernels (one tile row)
+// 2D grids: the tile kernels
 template <int R>
 cudaError_t launch_stress_any(const Geom& g, const KArgs& a, const StressMaps& m, bool cpml, bool ps,
                               cudaStream_t st)
 {
-    if (g.two_d || !a.pairs) return launch_stress_t<R>(g, a, m, cpml, ps, st);
-    const dim3 grid = step_grid(g, a, TY3);
+    if (g.two_d) return launch_stress2d<R>(g, a, m, cpml, ps, st);
+    if (!a.pairs) return launch_stress_t<R>(g, a, m, cpml, ps, st);
+    const dim3 grid = step_grid(g, a);
     if (cpml) return ps ? launch_stress_pair<R, true, true>(grid, m, a, st)
                         : launch_stress_pair<R, true, false>(grid, m, a, st);
     return ps ? launch_stress_pair<R, false, true>(grid, m, a, st)
@@ -806,8 +808,9 @@ template <int R>
 cudaError_t launch_velocity_any(const Geom& g, const KArgs& a, const VelMaps& m, bool cpml, int epi,
                                 bool rec, cudaStream_t st)
 {
-    if (g.two_d || !a.pairs) return launch_velocity_t<R>(g, a, m, cpml, epi, rec, st);
-    const dim3 grid = step_grid(g, a, TY3);
+    if (g.two_d) return launch_velocity2d<R>(g, a, m, cpml, epi, rec, st);
+    if (!a.pairs) return launch_velocity_t<R>(g, a, m, cpml, epi, rec, st);
+    const dim3 grid = step_grid(g, a);
     return cpml ? launch_velocity_pair<R, true>(grid, m, a, epi, rec, st)
                 : launch_velocity_pair<R, false>(grid, m, a, epi, rec, st);
 }
