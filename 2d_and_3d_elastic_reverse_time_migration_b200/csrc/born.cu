@@ -23,139 +23,122 @@
 //
 // The adjoint applies the transpose of every step in reverse order (D+ and D-
 // transpose to -D- and -D+ on the zero-padded grid).  Per reverse step:
-//   k_adj_vel : h_s <- g2 g1 h_s (completes the previous reverse step) + velocity^T
-//               contribution; rho gradient from a0
-//   k_adj_str : stress^T: velocity adjoint update, M/L/U gradients from e0
+//   k_adj_vm  : velocity^T into the stress adjoint and the rho gradient from a0, then
+//               (cell by cell, in registers) stress and memory variables^T with the
+//               pi and mu gradients from e0 and the strain adjoint S
+//   k_adj_str : velocity adjoint update with the stencils of S
 // The background history (v0 at the start of each step, a0 of each step) is
 // rebuilt per segment from checkpoints of the background state.
 //
-// Compact 2D layout: cell (i,k) at (k+R)*px + (i+XH), zero halos.
+// Compact 2D layout: cell (i,k) at (k+R)*px + (i+BXH), zero halos; the per-shot volumes
+// of a group are [type][shot][n], one 4D tensor (column, row, shot, type) to TMA.
+//
+// Every kernel is one tile of the x-z plane of one shot per CTA (blockIdx.z: shot), in
+// the manner of step_kernels_2d.cuh: the fields that a stencil reads arrive as TMA boxes
+// with halos under one mbarrier, each thread meanwhile loads the values of its own NR
+// rows of one column into registers (up to 30 per cell with three mechanisms), and all
+// stores come last.  A CTA makes one round trip to memory and others on the SM
+// fill its wait, so a grid in L2 costs little more than the launch and a large group
+// streams.  Before, each warp marched down 8-32 rows with one round trip per row.
+// Measured on B200, ms per call before -> now: Born forward, 10 shots of 880 x 480, three
+// mechanisms, 100 steps 34.4 -> 22.5 (4.96 TB/s of the 264 B per shot-cell and step that
+// the pair of kernels cannot do without); adjoint, 8 shots of 592 x 336, elastic, 240
+// steps 37.5 -> 21.2.
+//
+// Tiles start at allocated columns 64 b (cell 64 b - BXH): every row access is whole
+// 128-byte lines.  Lanes on the zero halo columns load and compute and store nothing.
 #include <cuda_runtime.h>
 
 #include "born.cuh"
+#include "step_kernels_2d.cuh"
 
 namespace ertm {
 
 namespace {
 
-template <int R>
-__device__ __forceinline__ float dpx(const float* __restrict__ f, long long c, const BornArgs& a)
+// box of a tile: columns of one shot's volume, halo rows, shot, type
+__device__ __forceinline__ void tma4(float* dst, const CUtensorMap* map, int x, int z, int shot, int type,
+                                     uint64_t* bar)
 {
-    float s = 0.f;
-#pragma unroll
-    for (int n = 1; n <= R; n++) s = fmaf(a.cx[n], __ldg(f + c + n) - __ldg(f + c - n + 1), s);
-    return s;
-}
-template <int R>
-__device__ __forceinline__ float dmx(const float* __restrict__ f, long long c, const BornArgs& a)
-{
-    float s = 0.f;
-#pragma unroll
-    for (int n = 1; n <= R; n++) s = fmaf(a.cx[n], __ldg(f + c + n - 1) - __ldg(f + c - n), s);
-    return s;
-}
-// Rows k-R .. k+R of one field at the thread's column, carried down the warp's z
-// chunk: each row is loaded once (one aligned 128-byte line per warp) and every
-// z stencil reads registers.  dpz / dmz are the forward / backward z differences
-// at row k with the same terms in the same order as the x differences above.
-template <int R>
-struct ZWin {
-    float w[2 * R + 1];
-    template <typename F>
-    __device__ __forceinline__ void init(F f, long long c, long long p)
-    {
-#pragma unroll
-        for (int j = 0; j <= 2 * R; j++) w[j] = f(c + (long long)(j - R) * p);
-    }
-    // c: the next row's cell
-    template <typename F>
-    __device__ __forceinline__ void shift(F f, long long c, long long p)
-    {
-#pragma unroll
-        for (int j = 0; j < 2 * R; j++) w[j] = w[j + 1];
-        w[2 * R] = f(c + (long long)R * p);
-    }
-    __device__ __forceinline__ float dpz(const float* cz) const
-    {
-        float s = 0.f;
-#pragma unroll
-        for (int n = 1; n <= R; n++) s = fmaf(cz[n], w[R + n] - w[R - n + 1], s);
-        return s;
-    }
-    __device__ __forceinline__ float dmz(const float* cz) const
-    {
-        float s = 0.f;
-#pragma unroll
-        for (int n = 1; n <= R; n++) s = fmaf(cz[n], w[R + n - 1] - w[R - n], s);
-        return s;
-    }
-};
-
-// read-only field (not written by the kernel that reads it)
-struct Ld {
-    const float* p;
-    __device__ __forceinline__ float operator()(long long c) const { return __ldg(p + c); }
-};
-// product of the shared B g1 (shot-independent, index c - zo) and the shot's own
-// field w: the velocity update's transposed operand
-struct Prod {
-    const float* bg;
-    const float* w;
-    long long zo;
-    __device__ __forceinline__ float operator()(long long c) const { return __ldg(bg + (c - zo)) * __ldg(w + c); }
-};
-template <int R, typename F>
-__device__ __forceinline__ float tdpx(F f, long long c, const BornArgs& a)
-{
-    float s = 0.f;
-#pragma unroll
-    for (int n = 1; n <= R; n++) s = fmaf(a.cx[n], f(c + n) - f(c - n + 1), s);
-    return s;
-}
-template <int R, typename F>
-__device__ __forceinline__ float tdmx(F f, long long c, const BornArgs& a)
-{
-    float s = 0.f;
-#pragma unroll
-    for (int n = 1; n <= R; n++) s = fmaf(a.cx[n], f(c + n - 1) - f(c - n), s);
-    return s;
+    asm volatile(
+        "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes"
+        " [%0], [%1, {%2, %3, %4, %5}], [%6];\n" ::"r"(smem_u32(dst)),
+        "l"(map), "r"(x), "r"(z), "r"(shot), "r"(type), "r"(smem_u32(bar))
+        : "memory");
 }
 
-// Work of one warp: a strip of 32 allocated columns (cells i = 32 w + lane - BXH, so
-// every row access is one aligned 128-byte line) and a chunk of a.kc rows, marched
-// top to bottom; blockIdx.z is the shot.  Lanes outside the grid (i < 0 or
-// i >= nx: zero halo columns) load and compute like the others and store nothing.
-constexpr int WPB = 4;       // warps per block: adjacent strips
-struct Strip {
-    int i, k0, k1;
-    bool act;                // the lane's cell is inside the grid
-    long long c;             // cell (i, k0) of the shared volumes
+// The thread's place: column i (cell; the tile's columns are allocated columns 64 b ..),
+// rows r0 .. r0 + NR - 1, and offsets of cell (i, r0) in the shared and per-shot volumes.
+template <int R, int NR>
+struct Place {
+    using T = Tile2<R, NR>;
+    int i, r0, kt, ax, tr;
+    bool act;
+    int c;                   // offset of cell (i, r0) in a volume
     long long zo;            // shot offset of the per-shot volumes
+    __device__ __forceinline__ explicit Place(const BornArgs& a)
+    {
+        const int tx = threadIdx.x & (TX2 - 1);
+        tr = threadIdx.x / TX2;
+        ax = blockIdx.x * TX2;
+        i = ax + tx - BXH;
+        kt = blockIdx.y * T::TZ;
+        r0 = kt + tr * NR;
+        act = i >= 0 && i < a.nx;
+        c = (int)((r0 + R) * a.px) + ax + tx;
+        zo = (long long)blockIdx.z * a.ss;
+    }
+    // shared-memory addresses of the thread's first cell in a tile with both halos, with
+    // the x halo only and with the z halo only
+    __device__ __forceinline__ int xz() const { return (tr * NR + R) * T::XW + (threadIdx.x & (TX2 - 1)) + T::XB; }
+    __device__ __forceinline__ int x() const { return tr * NR * T::XW + (threadIdx.x & (TX2 - 1)) + T::XB; }
+    __device__ __forceinline__ int z() const { return (tr * NR + R) * TX2 + (threadIdx.x & (TX2 - 1)); }
 };
-__device__ __forceinline__ bool strip_of(const BornArgs& a, Strip& s)
-{
-    const int w = blockIdx.x * WPB + threadIdx.y;
-    s.k0 = blockIdx.y * a.kc;
-    if (32 * w - BXH >= a.nx || s.k0 >= a.nz) return false;
-    s.k1 = min(s.k0 + a.kc, a.nz);
-    s.i = 32 * w + (int)threadIdx.x - BXH;
-    s.act = s.i >= 0 && s.i < a.nx;
-    s.c = (long long)(s.k0 + a.R) * a.px + 32 * w + threadIdx.x;
-    s.zo = (long long)blockIdx.z * a.ss;
-    return true;
-}
 
-// cell (i, k) of the launch's shot blockIdx.z: c indexes the shared volumes,
-// c + zo (zo = shot * ss) the shot's own volumes
-__device__ __forceinline__ bool cell_of(const BornArgs& a, int& i, int& k, long long& c, long long& zo)
+// x differences at f[0] and z differences from a column window w, w[q] = row q - R (dm)
+// or q + 1 - R (dp) of the thread's first row
+template <int R>
+__device__ __forceinline__ float dpx(const float* f, const float* cx)
 {
-    i = blockIdx.x * blockDim.x + threadIdx.x;
-    k = blockIdx.y * blockDim.y + threadIdx.y;
-    if (i >= a.nx || k >= a.nz) return false;
-    c = (long long)(k + a.R) * a.px + i + BXH;
-    zo = (long long)blockIdx.z * a.ss;
-    return true;
+    float s = 0.f;
+#pragma unroll
+    for (int n = 1; n <= R; n++) s = fmaf(cx[n], f[n] - f[1 - n], s);
+    return s;
 }
+template <int R>
+__device__ __forceinline__ float dmx(const float* f, const float* cx)
+{
+    float s = 0.f;
+#pragma unroll
+    for (int n = 1; n <= R; n++) s = fmaf(cx[n], f[n - 1] - f[-n], s);
+    return s;
+}
+template <int R, int NR>
+struct Win {
+    float w[NR + 2 * R - 1];
+    // f: the thread's first cell in a tile of pitch p; first: the window's first row
+    __device__ __forceinline__ void load(const float* f, int p, int first)
+    {
+#pragma unroll
+        for (int q = 0; q < NR + 2 * R - 1; q++) w[q] = f[(q + first) * p];
+    }
+    // forward difference at row r of a window that starts at row 1 - R
+    __device__ __forceinline__ float dp(int r, const float* cz) const
+    {
+        float s = 0.f;
+#pragma unroll
+        for (int n = 1; n <= R; n++) s = fmaf(cz[n], w[r + R - 1 + n] - w[r + R - n], s);
+        return s;
+    }
+    // backward difference at row r of a window that starts at row -R
+    __device__ __forceinline__ float dm(int r, const float* cz) const
+    {
+        float s = 0.f;
+#pragma unroll
+        for (int n = 1; n <= R; n++) s = fmaf(cz[n], w[r + R + n - 1] - w[r + R - n], s);
+        return s;
+    }
+};
 
 // the shot's parameters: sx, sz, rx0, nrx, drx, rz
 __device__ __forceinline__ int shot_par(const BornArgs& a, int q) { return __ldg(a.shot_tab + blockIdx.z * 8 + q); }
@@ -181,199 +164,213 @@ __device__ __forceinline__ void iso(float m, float u, float exx, float ezz, floa
 }
 
 // ---- forward ---------------------------------------------------------------
-template <int R, bool BORN, int NM>
-__global__ void __launch_bounds__(32 * WPB) k_born_stress(BornArgs a, int it)
+template <int R, bool BORN, int NM, int NR>
+__global__ void __launch_bounds__(256, 2) k_born_stress(const __grid_constant__ BornMaps maps,
+                                                        const __grid_constant__ BornArgs a, int it)
 {
-    Strip S;
-    if (!strip_of(a, S)) return;
-    const long long p = a.px, zo = S.zo;
-    const float dt = a.dt;
-    const float* v0x = a.v0x + zo;
-    const float* v0z = a.v0z + zo;
-    const float* vx = a.vx + zo;
-    const float* vz = a.vz + zo;
-    // z windows: v0x and vx feed forward z differences, v0z and vz backward ones
-    ZWin<R> w0x, w0z, wx, wz;
-    w0x.init(Ld{v0x}, S.c, p);
-    w0z.init(Ld{v0z}, S.c, p);
-    if (BORN) {
-        wx.init(Ld{vx}, S.c, p);
-        wz.init(Ld{vz}, S.c, p);
+    using T = Tile2<R, NR>;
+    constexpr int P = T::pad(T::XZ);
+    extern __shared__ __align__(128) float sm[];
+    __shared__ uint64_t bar;
+    const Place<R, NR> S(a);
+    tile2_begin(&bar);
+    if (threadIdx.x == 0) {
+        const int gx = S.ax - T::XB, sh = blockIdx.z;
+        mbar_expect_tx(&bar, 4u * (BORN ? 4 : 2) * T::XZ);
+        tma4(sm, &maps.xz, gx, S.kt, sh, a.t_v0, &bar);
+        tma4(sm + P, &maps.xz, gx, S.kt, sh, a.t_v0 + 1, &bar);
+        if (BORN) {
+            tma4(sm + 2 * P, &maps.xz, gx, S.kt, sh, a.t_v, &bar);
+            tma4(sm + 3 * P, &maps.xz, gx, S.kt, sh, a.t_v + 1, &bar);
+        }
+    }
+    const int px = (int)a.px;
+    float* s0[3] = {a.s0xx + S.zo, a.s0zz + S.zo, a.s0xz + S.zo};
+    float* sc[3] = {a.sxx + S.zo, a.szz + S.zo, a.sxz + S.zo};
+    constexpr int ND = NM > 0 ? NM : 1;
+    float o[3][NR], so[3][NR], r0v[3][ND][NR], rv[3][ND][NR];
+    float g1[NR], g2[NR], pi[NR], mu[NR], dpi[NR], dmu[NR];
+#pragma unroll
+    for (int r = 0; r < NR; r++) {
+        if (!S.act || S.r0 + r >= a.nz) continue;
+        const int c = S.c + r * px;
+#pragma unroll
+        for (int q = 0; q < 3; q++) {
+            o[q][r] = s0[q][c];
+            if (BORN) so[q][r] = sc[q][c];
+#pragma unroll
+            for (int l = 0; l < NM; l++) {
+                r0v[q][l][r] = a.r0[q * 3 + l][S.zo + c];
+                if (BORN) rv[q][l][r] = a.r[q * 3 + l][S.zo + c];
+            }
+        }
+        g1[r] = __ldg(a.g1 + c);
+        g2[r] = __ldg(a.g2 + c);
+        pi[r] = __ldg(a.M + c);
+        mu[r] = __ldg(a.U + c);
+        if (BORN) {
+            dpi[r] = __ldg(a.dM + c);
+            dmu[r] = __ldg(a.dU + c);
+        }
     }
     const bool src_step = it >= 0 && it < a.nw;
-    const int sx = shot_par(a, 0), sz = shot_par(a, 1);
-    long long c = S.c;
-    for (int k = S.k0; k < S.k1; k++, c += p) {
-        const long long cz = c + zo;
-        const float e0xx = dpx<R>(v0x, c, a), e0zz = w0z.dmz(a.cz);
-        const float e0xz = w0x.dpz(a.cz) + dmx<R>(v0z, c, a);
-        if (S.act) {
-            // every load of the row before any store: a store through one of the
-            // state pointers could alias a later load, which would serialise the
-            // memory-variable updates into one round trip each
-            const float g1 = __ldg(a.g1 + c), g2 = __ldg(a.g2 + c), pi = __ldg(a.M + c), mu = __ldg(a.U + c);
-            float o[3] = {a.s0xx[cz], a.s0zz[cz], a.s0xz[cz]};
-            float r0v[3][NM > 0 ? NM : 1], rv[3][NM > 0 ? NM : 1], so[3] = {0.f, 0.f, 0.f};
+    const bool src_col = src_step && S.i == shot_par(a, 0);
+    const int srcz = shot_par(a, 1);
+    if (!tile2_wait(&bar, kWaitPolls, a.err, false)) return;
+    if (!S.act || S.r0 >= a.nz) return;
+    const float* v0x = sm + S.xz();
+    const float* v0z = v0x + P;
+    const float* vx = v0x + 2 * P;
+    const float* vz = v0x + 3 * P;
+    Win<R, NR> w0x, w0z, wx, wz;      // v_x feeds forward z differences, v_z backward ones
+    w0x.load(v0x, T::XW, 1 - R);
+    w0z.load(v0z, T::XW, -R);
+    if (BORN) {
+        wx.load(vx, T::XW, 1 - R);
+        wz.load(vz, T::XW, -R);
+    }
+    const float dt = a.dt;
 #pragma unroll
-            for (int q = 0; q < 3; q++)
+    for (int r = 0; r < NR; r++) {
+        const int k = S.r0 + r;
+        if (k >= a.nz) break;
+        const int c = S.c + r * px;
+        const float e0xx = dpx<R>(v0x + r * T::XW, a.cx), e0zz = w0z.dm(r, a.cz);
+        const float e0xz = w0x.dp(r, a.cz) + dmx<R>(v0z + r * T::XW, a.cx);
+        float ov[3] = {o[0][r], o[1][r], o[2][r]};
+        if (src_col && k == srcz) {
+            // explosive source into the background
+            const float w = __ldg(a.wavelet + (long long)blockIdx.z * a.wstride + it);
+            ov[0] += w;
+            ov[1] += w;
+        }
+        float E0[3], F0[3];
+        iso(pi[r] * a.kp, mu[r] * a.ks, e0xx, e0zz, e0xz, E0);
+        if (NM) iso(pi[r] * a.tp, mu[r] * a.ts, e0xx, e0zz, e0xz, F0);
 #pragma unroll
-                for (int l = 0; l < NM; l++) r0v[q][l] = a.r0[q * 3 + l][cz];
-            float exx = 0.f, ezz = 0.f, exz = 0.f, dpi = 0.f, dmu = 0.f;
-            if (BORN) {
-                so[0] = a.sxx[cz];
-                so[1] = a.szz[cz];
-                so[2] = a.sxz[cz];
+        for (int q = 0; q < 3; q++) {
+            float sum = 0.f;
 #pragma unroll
-                for (int q = 0; q < 3; q++)
-#pragma unroll
-                    for (int l = 0; l < NM; l++) rv[q][l] = a.r[q * 3 + l][cz];
-                exx = dpx<R>(vx, c, a);
-                ezz = wz.dmz(a.cz);
-                exz = wx.dpz(a.cz) + dmx<R>(vz, c, a);
-                dpi = __ldg(a.dM + c);
-                dmu = __ldg(a.dU + c);
+            for (int l = 0; l < NM; l++) {
+                const float t = a.ra[l] * r0v[q][l][r] + a.rb[l] * F0[q];
+                a.r0[q * 3 + l][S.zo + c] = t;
+                sum += t;
             }
-            if (src_step && S.i == sx && k == sz) {
-                // explosive source into the background
-                const float w = __ldg(a.wavelet + (long long)blockIdx.z * a.wstride + it);
-                o[0] += w;
-                o[1] += w;
+            s0[q][c] = g1[r] * (g2[r] * ov[q] + dt * (E0[q] + sum));
+        }
+        if (BORN) {
+            const float exx = dpx<R>(vx + r * T::XW, a.cx), ezz = wz.dm(r, a.cz);
+            const float exz = wx.dp(r, a.cz) + dmx<R>(vz + r * T::XW, a.cx);
+            float E[3], dE[3], F[3], dF[3];
+            iso(pi[r] * a.kp, mu[r] * a.ks, exx, ezz, exz, E);
+            // the reference's stress sources (dem_p), scaled by the GSLS strengths
+            iso(dpi[r] * a.kp, dmu[r] * a.ks, e0xx, e0zz, e0xz, dE);
+            if (NM) {
+                iso(pi[r] * a.tp, mu[r] * a.ts, exx, ezz, exz, F);
+                iso(dpi[r] * a.tp, dmu[r] * a.ts, e0xx, e0zz, e0xz, dF);
             }
-            float E0[3], F0[3];
-            iso(pi * a.kp, mu * a.ks, e0xx, e0zz, e0xz, E0);
-            if (NM) iso(pi * a.tp, mu * a.ts, e0xx, e0zz, e0xz, F0);
-            float ns0[3];
 #pragma unroll
             for (int q = 0; q < 3; q++) {
                 float sum = 0.f;
 #pragma unroll
                 for (int l = 0; l < NM; l++) {
-                    r0v[q][l] = a.ra[l] * r0v[q][l] + a.rb[l] * F0[q];
-                    sum += r0v[q][l];
+                    const float t = a.ra[l] * rv[q][l][r] + a.rb[l] * (F[q] + dF[q]);
+                    a.r[q * 3 + l][S.zo + c] = t;
+                    sum += t;
                 }
-                ns0[q] = g1 * (g2 * o[q] + dt * (E0[q] + sum));
-            }
-            float nsc[3];
-            if (BORN) {
-                float E[3], dE[3], F[3], dF[3];
-                iso(pi * a.kp, mu * a.ks, exx, ezz, exz, E);
-                // the reference's stress sources (dem_p), scaled by the GSLS strengths
-                iso(dpi * a.kp, dmu * a.ks, e0xx, e0zz, e0xz, dE);
-                if (NM) {
-                    iso(pi * a.tp, mu * a.ts, exx, ezz, exz, F);
-                    iso(dpi * a.tp, dmu * a.ts, e0xx, e0zz, e0xz, dF);
-                }
-#pragma unroll
-                for (int q = 0; q < 3; q++) {
-                    float sum = 0.f;
-#pragma unroll
-                    for (int l = 0; l < NM; l++) {
-                        rv[q][l] = a.ra[l] * rv[q][l] + a.rb[l] * (F[q] + dF[q]);
-                        sum += rv[q][l];
-                    }
-                    nsc[q] = g1 * (g2 * so[q] + dt * (E[q] + dE[q] + sum));
-                }
-            }
-            // stores
-            a.s0xx[cz] = ns0[0];
-            a.s0zz[cz] = ns0[1];
-            a.s0xz[cz] = ns0[2];
-#pragma unroll
-            for (int q = 0; q < 3; q++)
-#pragma unroll
-                for (int l = 0; l < NM; l++) a.r0[q * 3 + l][cz] = r0v[q][l];
-            if (BORN) {
-                a.sxx[cz] = nsc[0];
-                a.szz[cz] = nsc[1];
-                a.sxz[cz] = nsc[2];
-#pragma unroll
-                for (int q = 0; q < 3; q++)
-#pragma unroll
-                    for (int l = 0; l < NM; l++) a.r[q * 3 + l][cz] = rv[q][l];
-            }
-        }
-        if (k + 1 < S.k1) {
-            w0x.shift(Ld{v0x}, c + p, p);
-            w0z.shift(Ld{v0z}, c + p, p);
-            if (BORN) {
-                wx.shift(Ld{vx}, c + p, p);
-                wz.shift(Ld{vz}, c + p, p);
+                sc[q][c] = g1[r] * (g2[r] * so[q][r] + dt * (E[q] + dE[q] + sum));
             }
         }
     }
 }
 
-template <int R, bool BORN, bool KEEP>
-__global__ void __launch_bounds__(32 * WPB) k_born_velocity(BornArgs a, int it)
+template <int R, bool BORN, bool KEEP, int NR>
+__global__ void __launch_bounds__(256, 2) k_born_velocity(const __grid_constant__ BornMaps maps,
+                                                          const __grid_constant__ BornArgs a, int it)
 {
-    Strip S;
-    if (!strip_of(a, S)) return;
-    const long long p = a.px, zo = S.zo;
-    const float dt = a.dt;
-    const float* s0xx = a.s0xx + zo;
-    const float* s0xz = a.s0xz + zo;
-    const float* s0zz = a.s0zz + zo;
-    const float* sxx = a.sxx + zo;
-    const float* sxz = a.sxz + zo;
-    const float* szz = a.szz + zo;
-    ZWin<R> w0xz, w0zz, wxz, wzz;      // sigma_xz: backward z difference; sigma_zz: forward
-    w0xz.init(Ld{s0xz}, S.c, p);
-    w0zz.init(Ld{s0zz}, S.c, p);
-    if (BORN) {
-        wxz.init(Ld{sxz}, S.c, p);
-        wzz.init(Ld{szz}, S.c, p);
+    using T = Tile2<R, NR>;
+    constexpr int O_ZZ = T::pad(T::X), O_XZ = O_ZZ + T::pad(T::Z), FLD = O_XZ + T::pad(T::XZ);
+    extern __shared__ __align__(128) float sm[];
+    __shared__ uint64_t bar;
+    const Place<R, NR> S(a);
+    tile2_begin(&bar);
+    if (threadIdx.x == 0) {
+        const int gx = S.ax - T::XB, sh = blockIdx.z;
+        mbar_expect_tx(&bar, 4u * (BORN ? 2 : 1) * (T::X + T::Z + T::XZ));
+#pragma unroll
+        for (int f = 0; f < (BORN ? 2 : 1); f++) {
+            float* d = sm + f * FLD;
+            const int t = f ? a.t_v + 2 : a.t_v0 + 2;      // sigma_xx, zz, xz
+            tma4(d, &maps.x, gx, S.kt + R, sh, t, &bar);
+            tma4(d + O_ZZ, &maps.z, S.ax, S.kt, sh, t + 1, &bar);
+            tma4(d + O_XZ, &maps.xz, gx, S.kt, sh, t + 2, &bar);
+        }
     }
-    const int rz = a.traces ? shot_par(a, 5) : -1;
-    long long c = S.c;
-    for (int k = S.k0; k < S.k1; k++, c += p) {
-        const long long cz = c + zo;
-        const float b = __ldg(a.B + c);
-        const float a0x = b * (dmx<R>(s0xx, c, a) + w0xz.dmz(a.cz));
-        const float a0z = b * (dpx<R>(s0xz, c, a) + w0zz.dpz(a.cz));
-        float ax = 0.f, az = 0.f;
+    const int px = (int)a.px;
+    float* v0x = a.v0x + S.zo;
+    float* v0z = a.v0z + S.zo;
+    float* vx = a.vx + S.zo;
+    float* vz = a.vz + S.zo;
+    float ov0x[NR], ov0z[NR], ovx[NR], ovz[NR], b[NR], g1[NR], g2[NR], rr[NR];
+#pragma unroll
+    for (int r = 0; r < NR; r++) {
+        if (!S.act || S.r0 + r >= a.nz) continue;
+        const int c = S.c + r * px;
+        ov0x[r] = v0x[c];
+        ov0z[r] = v0z[c];
+        b[r] = __ldg(a.B + c);
+        g1[r] = __ldg(a.g1 + c);
+        g2[r] = __ldg(a.g2 + c);
         if (BORN) {
-            ax = b * (dmx<R>(sxx, c, a) + wxz.dmz(a.cz));
-            az = b * (dpx<R>(sxz, c, a) + wzz.dpz(a.cz));
+            ovx[r] = vx[c];
+            ovz[r] = vz[c];
+            rr[r] = __ldg(a.rr + c);
         }
-        if (S.act) {
-            // every load of the row before any store (see k_born_stress)
-            const float g1 = __ldg(a.g1 + c), g2 = __ldg(a.g2 + c);
-            const float ov0x = a.v0x[cz], ov0z = a.v0z[cz];
-            float ovx = 0.f, ovz = 0.f, r = 0.f;
-            if (BORN) {
-                ovx = a.vx[cz];
-                ovz = a.vz[cz];
-                r = __ldg(a.rr + c);
-            }
-            if (KEEP) {   // background history for the adjoint: v0 at the start of the step, a0
-                a.kv0x[cz] = ov0x;
-                a.kv0z[cz] = ov0z;
-                a.ka0x[cz] = a0x;
-                a.ka0z[cz] = a0z;
-            }
-            a.v0x[cz] = g1 * (g2 * ov0x + dt * a0x);
-            a.v0z[cz] = g1 * (g2 * ov0z + dt * a0z);
-            if (BORN) {
-                const float nvx = g1 * (g2 * ovx + dt * (ax - r * a0x));
-                const float nvz = g1 * (g2 * ovz + dt * (az - r * a0z));
-                a.vx[cz] = nvx;
-                a.vz[cz] = nvz;
-                const int rec = k == rz ? recv_of(a, S.i, k) : -1;
-                if (rec >= 0) {
-                    const long long nrec = a.nrx, cs = (long long)a.nt * nrec;
-                    float* d = shot_traces(a) + (long long)it * nrec + rec;
-                    d[0] = nvx;
-                    d[cs] = 0.f;
-                    d[2 * cs] = nvz;
-                }
-            }
+    }
+    const int rz = BORN && a.traces ? shot_par(a, 5) : -1;
+    if (!tile2_wait(&bar, kWaitPolls, a.err, false)) return;
+    if (!S.act || S.r0 >= a.nz) return;
+    // sigma_xz: backward z difference; sigma_zz: forward
+    const float* s0xx = sm + S.x();
+    const float* s0xz = sm + O_XZ + S.xz();
+    Win<R, NR> w0xz, w0zz, wxz, wzz;
+    w0xz.load(s0xz, T::XW, -R);
+    w0zz.load(sm + O_ZZ + S.z(), TX2, 1 - R);
+    if (BORN) {
+        wxz.load(s0xz + FLD, T::XW, -R);
+        wzz.load(sm + FLD + O_ZZ + S.z(), TX2, 1 - R);
+    }
+    const float dt = a.dt;
+#pragma unroll
+    for (int r = 0; r < NR; r++) {
+        const int k = S.r0 + r;
+        if (k >= a.nz) break;
+        const int c = S.c + r * px;
+        const float a0x = b[r] * (dmx<R>(s0xx + r * T::XW, a.cx) + w0xz.dm(r, a.cz));
+        const float a0z = b[r] * (dpx<R>(s0xz + r * T::XW, a.cx) + w0zz.dp(r, a.cz));
+        if (KEEP) {   // background history for the adjoint: v0 at the start of the step, a0
+            const long long h = S.zo + c;
+            a.kv0x[h] = ov0x[r];
+            a.kv0z[h] = ov0z[r];
+            a.ka0x[h] = a0x;
+            a.ka0z[h] = a0z;
         }
-        if (k + 1 < S.k1) {
-            w0xz.shift(Ld{s0xz}, c + p, p);
-            w0zz.shift(Ld{s0zz}, c + p, p);
-            if (BORN) {
-                wxz.shift(Ld{sxz}, c + p, p);
-                wzz.shift(Ld{szz}, c + p, p);
+        v0x[c] = g1[r] * (g2[r] * ov0x[r] + dt * a0x);
+        v0z[c] = g1[r] * (g2[r] * ov0z[r] + dt * a0z);
+        if (BORN) {
+            const float ax = b[r] * (dmx<R>(s0xx + FLD + r * T::XW, a.cx) + wxz.dm(r, a.cz));
+            const float az = b[r] * (dpx<R>(s0xz + FLD + r * T::XW, a.cx) + wzz.dp(r, a.cz));
+            const float nvx = g1[r] * (g2[r] * ovx[r] + dt * (ax - rr[r] * a0x));
+            const float nvz = g1[r] * (g2[r] * ovz[r] + dt * (az - rr[r] * a0z));
+            vx[c] = nvx;
+            vz[c] = nvz;
+            const int rec = k == rz ? recv_of(a, S.i, k) : -1;
+            if (rec >= 0) {
+                const long long nrec = a.nrx, cs = (long long)a.nt * nrec;
+                float* d = shot_traces(a) + (long long)it * nrec + rec;
+                d[0] = nvx;
+                d[cs] = 0.f;
+                d[2 * cs] = nvz;
             }
         }
     }
@@ -397,150 +394,193 @@ __global__ void k_adj_inject(BornArgs a, int it)
     a.az[c] += d[2 * cs];
 }
 
-// velocity update^T: h (the stress adjoint, already carried through g2 g1 by
-// k_adj_mem) gains the velocity update's stencil transposed, applied to the
-// products B g1 a^; rho gradient from a0
-template <int R>
-__global__ void __launch_bounds__(32 * WPB) k_adj_vel(BornArgs a)
-{
-    Strip S;
-    if (!strip_of(a, S)) return;
-    const long long p = a.px, zo = S.zo;
-    const float dt = a.dt;
-    const Prod tx{a.Bg1, a.ax, zo}, tz{a.Bg1, a.az, zo};
-    ZWin<R> wx, wz;                    // products: forward z difference of x, backward of z
-    wx.init(tx, S.c + zo, p);
-    wz.init(tz, S.c + zo, p);
-    long long c = S.c;
-    for (int k = S.k0; k < S.k1; k++, c += p) {
-        const long long cz = c + zo;
-        const float dxx = tdpx<R>(tx, cz, a);
-        const float dxz = wx.dpz(a.cz) + tdmx<R>(tz, cz, a);
-        const float dzz = wz.dmz(a.cz);
-        if (S.act) {
-            // every load of the row before any store (see k_born_stress)
-            const float g1 = __ldg(a.g1 + c);
-            const float gr = a.gR[cz], hxx = a.hxx[cz], hxz = a.hxz[cz], hzz = a.hzz[cz];
-            const float vax = __ldg(a.ax + cz), vaz = __ldg(a.az + cz);
-            const float h0x = __ldg(a.ha0x + cz), h0z = __ldg(a.ha0z + cz);
-            // rho gradient: -dt g1 (vx^ a0x + vz^ a0z)
-            a.gR[cz] = gr + -dt * (g1 * vax * h0x + g1 * vaz * h0z);
-            a.hxx[cz] = hxx - dt * dxx;
-            a.hxz[cz] = hxz - dt * dxz;
-            a.hzz[cz] = hzz - dt * dzz;
-        }
-        if (k + 1 < S.k1) {
-            wx.shift(tx, cz + p, p);
-            wz.shift(tz, cz + p, p);
-        }
-    }
-}
-
-// stress and memory-variable update^T of one cell: Q = g1 h is the adjoint of
-// the stress bracket, Lambda_l = lr_l + dt Q that of r_l', P = sum_l rb_l Lambda_l
-// that of f; writes the strain adjoint S = iso(pi kp, mu ks; dt Q) + iso(pi tp,
+// velocity update^T, then stress and memory-variable update^T of one reverse step.
+//
+// h (the stress adjoint, already carried through g2 g1 by the previous reverse step)
+// gains the velocity update's stencil transposed, applied to the products B g1 a^
+// (formed in the staged tiles); rho gradient from a0.  Then, cell by cell: Q = g1 h is
+// the adjoint of the stress bracket, Lambda_l = lr_l + dt Q that of r_l', P = sum_l rb_l
+// Lambda_l that of f; writes the strain adjoint S = iso(pi kp, mu ks; dt Q) + iso(pi tp,
 // mu ts; P) (both maps are symmetric), carries lr_l = ra_l Lambda_l and h = g2 Q,
-// and accumulates the pi and mu gradients from the background strain rates.
-template <int R, int NM>
-__global__ void __launch_bounds__(32 * WPB) k_adj_mem(BornArgs a)
+// and accumulates the pi and mu gradients from the background strain rates.  One kernel:
+// h passes between the two parts in registers (24 B per cell less, one launch less).
+template <int R, int NM, int NR>
+__global__ void __launch_bounds__(256, 2) k_adj_vm(const __grid_constant__ BornMaps maps,
+                                                   const __grid_constant__ BornArgs a)
 {
-    Strip S;
-    if (!strip_of(a, S)) return;
-    const long long p = a.px, zo = S.zo;
-    const float dt = a.dt;
-    const float* hv0x = a.hv0x + zo;
-    const float* hv0z = a.hv0z + zo;
-    ZWin<R> wx, wz;
-    wx.init(Ld{hv0x}, S.c, p);
-    wz.init(Ld{hv0z}, S.c, p);
-    long long c = S.c;
-    for (int k = S.k0; k < S.k1; k++, c += p) {
-        const long long cz = c + zo;
-        const float e0xx = dpx<R>(hv0x, c, a), e0zz = wz.dmz(a.cz);
-        const float e0xz = wx.dpz(a.cz) + dmx<R>(hv0z, c, a);
-        if (S.act) {
-            // every load of the row before any store (see k_born_stress)
-            const float g1 = __ldg(a.g1 + c), g2 = __ldg(a.g2 + c), pi = __ldg(a.M + c), mu = __ldg(a.U + c);
-            const float Q[3] = {g1 * a.hxx[cz], g1 * a.hzz[cz], g1 * a.hxz[cz]};
-            float lv[3][NM > 0 ? NM : 1];
+    using T = Tile2<R, NR>;
+    constexpr int P = T::pad(T::XZ);
+    extern __shared__ __align__(128) float sm[];
+    __shared__ uint64_t bar;
+    const Place<R, NR> S(a);
+    tile2_begin(&bar);
+    if (threadIdx.x == 0) {
+        const int gx = S.ax - T::XB, sh = blockIdx.z;
+        mbar_expect_tx(&bar, 4u * 5 * T::XZ);
+        tma4(sm, &maps.xz, gx, S.kt, sh, a.t_adj, &bar);
+        tma4(sm + P, &maps.xz, gx, S.kt, sh, a.t_adj + 1, &bar);
+        tma4(sm + 2 * P, &maps.bg1, gx, S.kt, 0, 0, &bar);
+        tma4(sm + 3 * P, &maps.hist, gx, S.kt, sh, a.t_hist, &bar);
+        tma4(sm + 4 * P, &maps.hist, gx, S.kt, sh, a.t_hist + 1, &bar);
+    }
+    const int px = (int)a.px;
+    constexpr int ND = NM > 0 ? NM : 1;
+    float* h[3] = {a.hxx + S.zo, a.hzz + S.zo, a.hxz + S.zo};
+    float* Sg[3] = {a.Sxx + S.zo, a.Szz + S.zo, a.Sxz + S.zo};
+    float hv[3][NR], lv[3][ND][NR], gM[NR], gU[NR], gR[NR], h0x[NR], h0z[NR], vax[NR], vaz[NR];
+    float g1[NR], g2[NR], pi[NR], mu[NR];
 #pragma unroll
-            for (int q = 0; q < 3; q++)
+    for (int r = 0; r < NR; r++) {
+        if (!S.act || S.r0 + r >= a.nz) continue;
+        const int c = S.c + r * px;
+        const long long cz = S.zo + c;
 #pragma unroll
-                for (int l = 0; l < NM; l++) lv[q][l] = a.lr[q * 3 + l][cz];
-            const float gm = a.gM[cz], gu = a.gU[cz];
-            float P[3] = {0.f, 0.f, 0.f};
+        for (int q = 0; q < 3; q++) {
+            hv[q][r] = h[q][c];
 #pragma unroll
-            for (int q = 0; q < 3; q++)
-#pragma unroll
-                for (int l = 0; l < NM; l++) {
-                    const float lam = lv[q][l] + dt * Q[q];
-                    P[q] += a.rb[l] * lam;
-                    lv[q][l] = a.ra[l] * lam;
-                }
-            const float tq0 = dt * Q[0], tq1 = dt * Q[1], tq2 = dt * Q[2];
-            const float ngm = gm + (a.kp * (tq0 + tq1) + a.tp * (P[0] + P[1])) * (e0xx + e0zz);
-            const float ngu = gu + (a.ks * (-2.f * tq0 * e0zz - 2.f * tq1 * e0xx + tq2 * e0xz) +
-                                    a.ts * (-2.f * P[0] * e0zz - 2.f * P[1] * e0xx + P[2] * e0xz));
-            float E[3], F[3] = {0.f, 0.f, 0.f};
-            iso(pi * a.kp, mu * a.ks, tq0, tq1, tq2, E);
-            if (NM) iso(pi * a.tp, mu * a.ts, P[0], P[1], P[2], F);
-#pragma unroll
-            for (int q = 0; q < 3; q++)
-#pragma unroll
-                for (int l = 0; l < NM; l++) a.lr[q * 3 + l][cz] = lv[q][l];
-            a.gM[cz] = ngm;
-            a.gU[cz] = ngu;
-            a.Sxx[cz] = E[0] + F[0];
-            a.Szz[cz] = E[1] + F[1];
-            a.Sxz[cz] = E[2] + F[2];
-            a.hxx[cz] = g2 * Q[0];
-            a.hzz[cz] = g2 * Q[1];
-            a.hxz[cz] = g2 * Q[2];
+            for (int l = 0; l < NM; l++) lv[q][l][r] = a.lr[q * 3 + l][cz];
         }
-        if (k + 1 < S.k1) {
-            wx.shift(Ld{hv0x}, c + p, p);
-            wz.shift(Ld{hv0z}, c + p, p);
+        gM[r] = a.gM[cz];
+        gU[r] = a.gU[cz];
+        gR[r] = a.gR[cz];
+        h0x[r] = a.ha0x[cz];
+        h0z[r] = a.ha0z[cz];
+        g1[r] = __ldg(a.g1 + c);
+        g2[r] = __ldg(a.g2 + c);
+        pi[r] = __ldg(a.M + c);
+        mu[r] = __ldg(a.U + c);
+    }
+    const bool landed = tile2_wait(&bar, kWaitPolls, a.err, false);
+    float* fx = sm + S.xz();
+    float* fz = fx + P;
+#pragma unroll
+    for (int r = 0; r < NR; r++) {
+        vax[r] = fx[r * T::XW];
+        vaz[r] = fz[r * T::XW];
+    }
+    __syncthreads();
+    for (int q = threadIdx.x; q < T::XZ; q += 256) {      // the products B g1 a^
+        const float b = sm[2 * P + q];
+        sm[q] *= b;
+        sm[P + q] *= b;
+    }
+    if (!__syncthreads_and(landed)) return;
+    if (!S.act || S.r0 >= a.nz) return;
+    const float* v0x = fx + 3 * P;
+    const float* v0z = fx + 4 * P;
+    Win<R, NR> wx, wz, w0x, w0z;
+    wx.load(fx, T::XW, 1 - R);
+    wz.load(fz, T::XW, -R);
+    w0x.load(v0x, T::XW, 1 - R);
+    w0z.load(v0z, T::XW, -R);
+    const float dt = a.dt;
+#pragma unroll
+    for (int r = 0; r < NR; r++) {
+        const int k = S.r0 + r;
+        if (k >= a.nz) break;
+        const int c = S.c + r * px;
+        const long long cz = S.zo + c;
+        const float dxx = dpx<R>(fx + r * T::XW, a.cx);
+        const float dxz = wx.dp(r, a.cz) + dmx<R>(fz + r * T::XW, a.cx);
+        const float dzz = wz.dm(r, a.cz);
+        // rho gradient: -dt g1 (vx^ a0x + vz^ a0z)
+        a.gR[cz] = gR[r] + -dt * (g1[r] * vax[r] * h0x[r] + g1[r] * vaz[r] * h0z[r]);
+        const float nxx = hv[0][r] - dt * dxx, nzz = hv[1][r] - dt * dzz, nxz = hv[2][r] - dt * dxz;
+        const float e0xx = dpx<R>(v0x + r * T::XW, a.cx), e0zz = w0z.dm(r, a.cz);
+        const float e0xz = w0x.dp(r, a.cz) + dmx<R>(v0z + r * T::XW, a.cx);
+        const float Q[3] = {g1[r] * nxx, g1[r] * nzz, g1[r] * nxz};
+        float Pm[3] = {0.f, 0.f, 0.f};
+#pragma unroll
+        for (int q = 0; q < 3; q++)
+#pragma unroll
+            for (int l = 0; l < NM; l++) {
+                const float lam = lv[q][l][r] + dt * Q[q];
+                Pm[q] += a.rb[l] * lam;
+                a.lr[q * 3 + l][cz] = a.ra[l] * lam;
+            }
+        const float tq0 = dt * Q[0], tq1 = dt * Q[1], tq2 = dt * Q[2];
+        a.gM[cz] = gM[r] + (a.kp * (tq0 + tq1) + a.tp * (Pm[0] + Pm[1])) * (e0xx + e0zz);
+        a.gU[cz] = gU[r] + (a.ks * (-2.f * tq0 * e0zz - 2.f * tq1 * e0xx + tq2 * e0xz) +
+                            a.ts * (-2.f * Pm[0] * e0zz - 2.f * Pm[1] * e0xx + Pm[2] * e0xz));
+        float E[3], F[3] = {0.f, 0.f, 0.f};
+        iso(pi[r] * a.kp, mu[r] * a.ks, tq0, tq1, tq2, E);
+        if (NM) iso(pi[r] * a.tp, mu[r] * a.ts, Pm[0], Pm[1], Pm[2], F);
+#pragma unroll
+        for (int q = 0; q < 3; q++) {
+            Sg[q][c] = E[q] + F[q];
+            h[q][c] = g2[r] * Q[q];
         }
     }
 }
 
 // velocity adjoint: a <- g2 g1 a (the velocity update^T) - D^T S (the stress
 // update's stencils transposed), plus the next (earlier) step's residual
-template <int R>
-__global__ void __launch_bounds__(32 * WPB) k_adj_str(BornArgs a, int it_next)
+template <int R, int NR>
+__global__ void __launch_bounds__(256, 2) k_adj_str(const __grid_constant__ BornMaps maps,
+                                                    const __grid_constant__ BornArgs a, int it_next)
 {
-    Strip S;
-    if (!strip_of(a, S)) return;
-    const long long p = a.px, zo = S.zo;
-    const Ld sxx{a.Sxx + zo}, szz{a.Szz + zo}, sxz{a.Sxz + zo};
-    ZWin<R> wxz, wzz;                  // S_xz: backward z difference; S_zz: forward
-    wxz.init(sxz, S.c, p);
-    wzz.init(szz, S.c, p);
-    const int rz = it_next >= 0 ? shot_par(a, 5) : -1;
-    long long c = S.c;
-    for (int k = S.k0; k < S.k1; k++, c += p) {
-        const long long cz = c + zo;
-        const float dx = tdmx<R>(sxx, c, a) + wxz.dmz(a.cz);
-        const float dz = wzz.dpz(a.cz) + tdpx<R>(sxz, c, a);
-        if (S.act) {
-            const float g12 = __ldg(a.g2 + c) * __ldg(a.g1 + c);
-            float nx = g12 * a.ax[cz] - dx;
-            float nz = g12 * a.az[cz] - dz;
-            const int rec = k == rz ? recv_of(a, S.i, k) : -1;
-            if (rec >= 0) {
-                const long long nrec = a.nrx, cs = (long long)a.nt * nrec;
-                const float* d = shot_traces(a) + (long long)it_next * nrec + rec;
-                nx += d[0];
-                nz += d[2 * cs];
-            }
-            a.ax[cz] = nx;
-            a.az[cz] = nz;
-        }
-        if (k + 1 < S.k1) {
-            wxz.shift(sxz, c + p, p);
-            wzz.shift(szz, c + p, p);
-        }
+    using T = Tile2<R, NR>;
+    constexpr int O_ZZ = T::pad(T::X), O_XZ = O_ZZ + T::pad(T::Z);
+    extern __shared__ __align__(128) float sm[];
+    __shared__ uint64_t bar;
+    const Place<R, NR> S(a);
+    tile2_begin(&bar);
+    if (threadIdx.x == 0) {
+        const int gx = S.ax - T::XB, sh = blockIdx.z;
+        mbar_expect_tx(&bar, 4u * (T::X + T::Z + T::XZ));
+        tma4(sm, &maps.x, gx, S.kt + R, sh, a.t_s, &bar);
+        tma4(sm + O_ZZ, &maps.z, S.ax, S.kt, sh, a.t_s + 1, &bar);
+        tma4(sm + O_XZ, &maps.xz, gx, S.kt, sh, a.t_s + 2, &bar);
     }
+    const int px = (int)a.px;
+    float* ax = a.ax + S.zo;
+    float* az = a.az + S.zo;
+    float ox[NR], oz[NR], g12[NR];
+#pragma unroll
+    for (int r = 0; r < NR; r++) {
+        if (!S.act || S.r0 + r >= a.nz) continue;
+        const int c = S.c + r * px;
+        ox[r] = ax[c];
+        oz[r] = az[c];
+        g12[r] = __ldg(a.g2 + c) * __ldg(a.g1 + c);
+    }
+    const int rz = it_next >= 0 ? shot_par(a, 5) : -1;
+    if (!tile2_wait(&bar, kWaitPolls, a.err, false)) return;
+    if (!S.act || S.r0 >= a.nz) return;
+    const float* sxx = sm + S.x();
+    const float* sxz = sm + O_XZ + S.xz();
+    Win<R, NR> wxz, wzz;                  // S_xz: backward z difference; S_zz: forward
+    wxz.load(sxz, T::XW, -R);
+    wzz.load(sm + O_ZZ + S.z(), TX2, 1 - R);
+#pragma unroll
+    for (int r = 0; r < NR; r++) {
+        const int k = S.r0 + r;
+        if (k >= a.nz) break;
+        const int c = S.c + r * px;
+        const float dx = dmx<R>(sxx + r * T::XW, a.cx) + wxz.dm(r, a.cz);
+        const float dz = wzz.dp(r, a.cz) + dpx<R>(sxz + r * T::XW, a.cx);
+        float nx = g12[r] * ox[r] - dx;
+        float nz = g12[r] * oz[r] - dz;
+        const int rec = k == rz ? recv_of(a, S.i, k) : -1;
+        if (rec >= 0) {
+            const long long nrec = a.nrx, cs = (long long)a.nt * nrec;
+            const float* d = shot_traces(a) + (long long)it_next * nrec + rec;
+            nx += d[0];
+            nz += d[2 * cs];
+        }
+        ax[c] = nx;
+        az[c] = nz;
+    }
+}
+
+// cell (i, k) of the small kernels below
+__device__ __forceinline__ bool cell_of(const BornArgs& a, int& i, int& k, long long& c)
+{
+    i = blockIdx.x * blockDim.x + threadIdx.x;
+    k = blockIdx.y * blockDim.y + threadIdx.y;
+    if (i >= a.nx || k >= a.nz) return false;
+    c = (long long)(k + a.R) * a.px + i + BXH;
+    return true;
 }
 
 // gradients w.r.t. (r_vp, r_vs, r_rho) on the contiguous nz x nx grid, summed over
@@ -548,8 +588,8 @@ __global__ void __launch_bounds__(32 * WPB) k_adj_str(BornArgs a, int it_next)
 __global__ void k_born_final(BornArgs a, float* gvp, float* gvs, float* grho, int accumulate)
 {
     int i, k;
-    long long c, zo;
-    if (!cell_of(a, i, k, c, zo)) return;
+    long long c;
+    if (!cell_of(a, i, k, c)) return;
     const long long m = (long long)k * a.nx + i;
     float gp = 0.f, gu = 0.f, gr = 0.f;
     for (int sh = 0; sh < a.nshot; sh++) {
@@ -573,8 +613,7 @@ __global__ void k_born_model(BornArgs a, const float* Mc, const float* Uc, const
 {
     int i, k;
     long long c;
-    long long zo;
-    if (!cell_of(a, i, k, c, zo)) return;
+    if (!cell_of(a, i, k, c)) return;
     const long long m = (long long)k * csz + i;
     M[c] = Mc[m];
     U[c] = Uc[m];
@@ -591,39 +630,14 @@ __global__ void k_born_pert(BornArgs a, const float* rvp, const float* rvs, cons
 {
     int i, k;
     long long c;
-    long long zo;
-    if (!cell_of(a, i, k, c, zo)) return;
+    if (!cell_of(a, i, k, c)) return;
     const long long m = (long long)k * a.nx + i;
     dM[c] = a.M[c] * (rrho[m] + 2.f * rvp[m]);
     dU[c] = a.U[c] * (rrho[m] + 2.f * rvs[m]);
     rr[c] = rrho[m];
 }
 
-dim3 born_grid(const BornArgs& a, int shots = 1) { return dim3((a.nx + 31) / 32, (a.nz + 7) / 8, shots); }
-
-// The marching kernels' arguments and grid: WPB strips per block, chunks of kc
-// rows, one grid layer per shot.  kc is the longest chunk (32, 16 or 8 rows) that
-// still gives about two waves of blocks on the device (a shorter chunk reloads
-// the 2R rows of its z windows more often).
-BornArgs march(const BornArgs& a, dim3& grid)
-{
-    static const int sms = [] {
-        int dev = 0, n = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-        return n > 0 ? n : 148;
-    }();
-    BornArgs b = a;
-    const long long xb = ((a.nx + BXH + 31) / 32 + WPB - 1) / WPB;
-    b.kc = 8;
-    for (int kc = 32; kc > 8; kc /= 2)
-        if (xb * ((a.nz + kc - 1) / kc) * a.nshot >= 2LL * 7 * sms) {
-            b.kc = kc;
-            break;
-        }
-    grid = dim3((unsigned)xb, (a.nz + b.kc - 1) / b.kc, a.nshot);
-    return b;
-}
+dim3 born_grid(const BornArgs& a) { return dim3((a.nx + 31) / 32, (a.nz + 7) / 8); }
 
 }  // namespace
 
@@ -644,62 +658,109 @@ cudaError_t born_launch_pert(const BornArgs& a, const float* rvp, const float* r
 }
 
 namespace {
-template <int R, int NM>
-void step_r(const BornArgs& a0, int it, bool born, bool keep, cudaStream_t s)
+dim3 tile_grid(const BornArgs& a)
 {
-    dim3 g;
-    const BornArgs a = march(a0, g);
-    const dim3 b(32, WPB);
-    if (born) k_born_stress<R, true, NM><<<g, b, 0, s>>>(a, it);
-    else k_born_stress<R, false, NM><<<g, b, 0, s>>>(a, it);
-    if (born) k_born_velocity<R, true, false><<<g, b, 0, s>>>(a, it);
-    else if (keep) k_born_velocity<R, false, true><<<g, b, 0, s>>>(a, it);
-    else k_born_velocity<R, false, false><<<g, b, 0, s>>>(a, it);
+    return dim3((a.nx + BXH + TX2 - 1) / TX2, (a.nz + 4 * a.nr - 1) / (4 * a.nr), a.nshot);
+}
+template <typename... P, typename... A>
+cudaError_t launch_tile(void (*K)(P...), unsigned long long* opted, const BornArgs& a, size_t smem, cudaStream_t s,
+                        const A&... args)
+{
+    const cudaError_t e = smem > 48 * 1024 ? smem_opt_in(K, smem, opted) : cudaSuccess;
+    return e != cudaSuccess ? e : launch_pdl(K, tile_grid(a), 256, smem, s, args...);
+}
+
+template <int R, int NR>
+constexpr size_t xz_bytes(int n) { return 4 * (size_t)n * Tile2<R, NR>::pad(Tile2<R, NR>::XZ); }
+template <int R, int NR>
+constexpr size_t sig_bytes(int n)
+{
+    using T = Tile2<R, NR>;
+    return 4 * (size_t)n * (T::pad(T::X) + T::pad(T::Z) + T::pad(T::XZ));
+}
+
+template <int R, int NM, int NR, bool BORN>
+cudaError_t stress_r(const BornMaps& m, const BornArgs& a, int it, cudaStream_t s)
+{
+    static unsigned long long opted = 0;
+    return launch_tile(k_born_stress<R, BORN, NM, NR>, &opted, a, xz_bytes<R, NR>(BORN ? 4 : 2), s, m, a, it);
+}
+template <int R, int NR, bool BORN, bool KEEP>
+cudaError_t velocity_r(const BornMaps& m, const BornArgs& a, int it, cudaStream_t s)
+{
+    static unsigned long long opted = 0;
+    return launch_tile(k_born_velocity<R, BORN, KEEP, NR>, &opted, a, sig_bytes<R, NR>(BORN ? 2 : 1), s, m, a, it);
+}
+template <int R, int NM, int NR>
+cudaError_t step_r(const BornMaps& m, const BornArgs& a, int it, bool born, bool keep, cudaStream_t s)
+{
+    cudaError_t e = born ? stress_r<R, NM, NR, true>(m, a, it, s) : stress_r<R, NM, NR, false>(m, a, it, s);
+    if (e != cudaSuccess) return e;
+    if (born) return velocity_r<R, NR, true, false>(m, a, it, s);
+    return keep ? velocity_r<R, NR, false, true>(m, a, it, s) : velocity_r<R, NR, false, false>(m, a, it, s);
+}
+template <int R, int NM, int NR>
+cudaError_t adj_r(const BornMaps& m, const BornArgs& a, int it, cudaStream_t s)
+{
+    static unsigned long long opted = 0, opted2 = 0;
+    const cudaError_t e = launch_tile(k_adj_vm<R, NM, NR>, &opted, a, xz_bytes<R, NR>(5), s, m, a);
+    if (e != cudaSuccess) return e;
+    return launch_tile(k_adj_str<R, NR>, &opted2, a, sig_bytes<R, NR>(1), s, m, a, it - 1);
 }
 template <int R, int NM>
-void adj_r(const BornArgs& a0, int it, cudaStream_t s)
+cudaError_t step_nr(const BornMaps& m, const BornArgs& a, int it, bool born, bool keep, cudaStream_t s)
 {
-    dim3 g;
-    const BornArgs a = march(a0, g);
-    const dim3 b(32, WPB);
-    k_adj_vel<R><<<g, b, 0, s>>>(a);
-    k_adj_mem<R, NM><<<g, b, 0, s>>>(a);
-    k_adj_str<R><<<g, b, 0, s>>>(a, it - 1);
+    if constexpr (NM == 0)
+        if (a.nr == 4) return step_r<R, NM, 4>(m, a, it, born, keep, s);
+    return a.nr == 1 ? step_r<R, NM, 1>(m, a, it, born, keep, s) : step_r<R, NM, 2>(m, a, it, born, keep, s);
+}
+template <int R, int NM>
+cudaError_t adj_nr(const BornMaps& m, const BornArgs& a, int it, cudaStream_t s)
+{
+    if constexpr (NM == 0)
+        if (a.nr == 4) return adj_r<R, NM, 4>(m, a, it, s);
+    return a.nr == 1 ? adj_r<R, NM, 1>(m, a, it, s) : adj_r<R, NM, 2>(m, a, it, s);
 }
 template <int R>
-void step_nm(const BornArgs& a, int it, bool born, bool keep, cudaStream_t s)
+cudaError_t step_nm(const BornMaps& m, const BornArgs& a, int it, bool born, bool keep, cudaStream_t s)
 {
     switch (a.nm) {
-    case 0: step_r<R, 0>(a, it, born, keep, s); break;
-    case 1: step_r<R, 1>(a, it, born, keep, s); break;
-    case 2: step_r<R, 2>(a, it, born, keep, s); break;
-    default: step_r<R, 3>(a, it, born, keep, s); break;
+    case 0: return step_nr<R, 0>(m, a, it, born, keep, s);
+    case 1: return step_nr<R, 1>(m, a, it, born, keep, s);
+    case 2: return step_nr<R, 2>(m, a, it, born, keep, s);
+    default: return step_nr<R, 3>(m, a, it, born, keep, s);
     }
 }
 template <int R>
-void adj_nm(const BornArgs& a, int it, cudaStream_t s)
+cudaError_t adj_nm(const BornMaps& m, const BornArgs& a, int it, cudaStream_t s)
 {
     switch (a.nm) {
-    case 0: adj_r<R, 0>(a, it, s); break;
-    case 1: adj_r<R, 1>(a, it, s); break;
-    case 2: adj_r<R, 2>(a, it, s); break;
-    default: adj_r<R, 3>(a, it, s); break;
+    case 0: return adj_nr<R, 0>(m, a, it, s);
+    case 1: return adj_nr<R, 1>(m, a, it, s);
+    case 2: return adj_nr<R, 2>(m, a, it, s);
+    default: return adj_nr<R, 3>(m, a, it, s);
     }
 }
 }  // namespace
 
-cudaError_t born_launch_step(const BornArgs& a, int it, bool born, bool keep, cudaStream_t s)
+// Rows per thread: as many (1, 2, or 4 without memory variables, which take up to 24
+// registers a row) as still give every SM a CTA.
+int born_rows(int nx, int nz, int nshot, int nm)
 {
-    if (a.R == 4) step_nm<4>(a, it, born, keep, s);
-    else step_nm<6>(a, it, born, keep, s);
-    return cudaGetLastError();
+    const long long cols = (nx + BXH + TX2 - 1) / TX2;
+    for (int nr = nm ? 2 : 4; nr > 1; nr /= 2)
+        if (cols * ((nz + 4 * nr - 1) / (4 * nr)) * nshot >= 148) return nr;
+    return 1;
 }
 
-cudaError_t born_launch_adjoint_step(const BornArgs& a, int it, cudaStream_t s)
+cudaError_t born_launch_step(const BornMaps& m, const BornArgs& a, int it, bool born, bool keep, cudaStream_t s)
 {
-    if (a.R == 4) adj_nm<4>(a, it, s);
-    else adj_nm<6>(a, it, s);
-    return cudaGetLastError();
+    return a.R == 4 ? step_nm<4>(m, a, it, born, keep, s) : step_nm<6>(m, a, it, born, keep, s);
+}
+
+cudaError_t born_launch_adjoint_step(const BornMaps& m, const BornArgs& a, int it, cudaStream_t s)
+{
+    return a.R == 4 ? adj_nm<4>(m, a, it, s) : adj_nm<6>(m, a, it, s);
 }
 
 cudaError_t born_launch_inject(const BornArgs& a, int it, cudaStream_t s)

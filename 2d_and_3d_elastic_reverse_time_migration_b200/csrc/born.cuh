@@ -2,6 +2,7 @@
 // viscoelastic): argument block and launchers.
 #pragma once
 
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 namespace ertm {
@@ -26,7 +27,7 @@ struct BornArgs {
     float tp, ts, kp, ks;                  // strengths; kp = 1 + nm tp, ks = 1 + nm ts
     float *r0[9], *r[9], *lr[9];           // background, scattered, adjoint memory variables
     float *Sxx, *Szz, *Sxz;                // strain adjoint of the reverse step (scratch)
-    const float *hv0x, *hv0z, *ha0x, *ha0z;// background history read by the adjoint step
+    const float *ha0x, *ha0z;              // background history read by the adjoint step (v0: t_hist)
     float *kv0x, *kv0z, *ka0x, *ka0z;      // history slot written by a recording step
     int nw;
     const float* wavelet;                  // shot s's wavelet at wavelet + s * wstride
@@ -43,16 +44,30 @@ struct BornArgs {
     long long ss;
     const int* shot_tab;
     long long tstride;
-    int kc;                                // rows per warp of the step kernels (set by the launcher)
+    int nr;                                // rows per thread of the step kernels (born_rows), as the maps' boxes
+    // TMA types (BornMaps): v0x, v0z, sigma0 xx, zz, xz in a row from t_v0, the scattered
+    // ones from t_v; ax, az from t_adj; Sxx, Szz, Sxz from t_s; the history slot's v0x,
+    // v0z from t_hist
+    int t_v0, t_v, t_adj, t_s, t_hist;
+    int* err;                              // device error word
 };
+
+// TMA maps over the per-shot volumes (column, row, shot, type), boxes of one type's tile:
+// 64 columns x 4 nr rows with halos in both directions (xz), in x only, in z only; the
+// history volumes and the shared B g1, both with xz boxes.
+struct BornMaps {
+    CUtensorMap xz, x, z, hist, bg1;
+};
+
+int born_rows(int nx, int nz, int nshot, int nm);
 
 cudaError_t born_launch_model(const BornArgs& a, const float* Mc, const float* Uc, const float* Bc,
                               long long csz, const float* att_x, const float* att_z, float* M,
                               float* U, float* Bg1, float* B, float* g1, float* g2, cudaStream_t s);
 cudaError_t born_launch_pert(const BornArgs& a, const float* rvp, const float* rvs,
                              const float* rrho, float* dM, float* dU, float* rr, cudaStream_t s);
-cudaError_t born_launch_step(const BornArgs& a, int it, bool born, bool keep, cudaStream_t s);
-cudaError_t born_launch_adjoint_step(const BornArgs& a, int it, cudaStream_t s);
+cudaError_t born_launch_step(const BornMaps& m, const BornArgs& a, int it, bool born, bool keep, cudaStream_t s);
+cudaError_t born_launch_adjoint_step(const BornMaps& m, const BornArgs& a, int it, cudaStream_t s);
 cudaError_t born_launch_inject(const BornArgs& a, int it, cudaStream_t s);
 // gradients summed over the launch's shots, written to (or, with accumulate, added to)
 // the nz x nx outputs

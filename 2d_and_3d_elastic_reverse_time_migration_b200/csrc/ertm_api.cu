@@ -1590,6 +1590,7 @@ int born_prepare(ertm_ctx* c, BornArgs& a)
     a.nt = c->cfg.nt;
     a.nshot = 1;
     a.ss = B.n;
+    a.err = c->err_d;
     CK(c, born_launch_model(a, c->m[1][0], c->m[1][1], c->m[1][2], g.sz, c->att[0], c->att[2],
                             B.sv[SV_M], B.sv[SV_U], B.sv[SV_BG1], B.sv[SV_B], B.sv[SV_G1], B.sv[SV_G2],
                             c->stream));
@@ -1683,6 +1684,44 @@ int born_zero_types(ertm_ctx* c, int first, int count, int G)
     return ERTM_OK;
 }
 
+// Tile maps of the group's volumes: `types` volumes [shot][n] each, G shots, at `base`;
+// boxes of bx columns x bz rows of one shot and type.
+int born_map(ertm_ctx* c, CUtensorMap* m, const void* base, int G, int types, int bx, int bz)
+{
+    auto enc = tensor_map_encoder();
+    if (!enc) return fail(c, ERTM_ECUDA, "cuTensorMapEncodeTiled unavailable");
+    const auto& B = c->born;
+    const cuuint64_t dims[4] = {(cuuint64_t)B.px, (cuuint64_t)(B.n / B.px), (cuuint64_t)G, (cuuint64_t)types};
+    const cuuint64_t strides[3] = {(cuuint64_t)B.px * 4, (cuuint64_t)B.n * 4, (cuuint64_t)B.n * 4 * G};
+    const cuuint32_t box[4] = {(cuuint32_t)bx, (cuuint32_t)bz, 1, 1}, es[4] = {1, 1, 1, 1};
+    CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<void*>(base), dims, strides, box, es,
+                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return fail(c, ERTM_ECUDA, "cuTensorMapEncodeTiled failed (%d)", (int)r);
+    return ERTM_OK;
+}
+
+// rows per thread and maps for a group of G shots; hist_slots: history slots (adjoint), or 0
+int born_group_maps(ertm_ctx* c, BornArgs& a, BornMaps& m, int G, int hist_slots)
+{
+    const auto& B = c->born;
+    a.nr = born_rows(a.nx, a.nz, G, a.nm);
+    a.t_v0 = PV_BG;
+    a.t_v = PV_SC;
+    a.t_adj = PV_ADJ;
+    a.t_s = PV_S;
+    a.t_hist = 0;
+    const int xw = TX2 + 2 * xb_of(a.R), tz = 4 * a.nr, zh = tz + 2 * a.R;
+    std::memset(&m, 0, sizeof m);
+    int rc;
+    if ((rc = born_map(c, &m.xz, B.block, G, PV_N, xw, zh))) return rc;
+    if ((rc = born_map(c, &m.x, B.block, G, PV_N, xw, tz))) return rc;
+    if ((rc = born_map(c, &m.z, B.block, G, PV_N, TX2, zh))) return rc;
+    if (!hist_slots) return ERTM_OK;
+    if ((rc = born_map(c, &m.hist, B.hist, G, 4 * hist_slots, xw, zh))) return rc;
+    return born_map(c, &m.bg1, B.sv[SV_BG1], 1, 1, xw, zh);
+}
+
 // contiguous nz*nx device copies of up to three caller arrays (stage)
 int born_stage_in(ertm_ctx* c, const float* const* src, int count, const float** out)
 {
@@ -1705,13 +1744,15 @@ int born_stage_in(ertm_ctx* c, const float* const* src, int count, const float**
 // adjoint, its checkpoints and history) take at most about 60 % of the free memory.
 int born_group_size(ertm_ctx* c, int want, long long floats_per_shot)
 {
+    // memory the context already holds for a group counts as available; a call whose
+    // volumes all fit in it asks the driver nothing
+    const long long held = (long long)c->born.G * c->born.n * PV_N + c->born.ckpt_floats + c->born.hist_floats;
+    if (want <= kBornMaxShots && held >= want * floats_per_shot) return want;
     size_t free_b = 0, total_b = 0;
     if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
         cudaGetLastError();
         return 1;
     }
-    // memory the context already holds for a group counts as available
-    const long long held = (long long)c->born.G * c->born.n * PV_N + c->born.ckpt_floats + c->born.hist_floats;
     const double avail = 0.6 * (double)free_b + 4.0 * (double)held;
     long long g = (long long)(avail / (4.0 * (double)floats_per_shot));
     if (g > want) g = want;
@@ -1750,19 +1791,20 @@ int ertm_born_forward_shots(ertm_ctx* c, const ertm_shot* shots, int nshots, con
         const int g = std::min(G, nshots - s0);
         born_group_args(c, a, g);
         if ((rc = born_group_shots(c, a, shots + s0, g))) return rc;
+        BornMaps maps;
+        if ((rc = born_group_maps(c, a, maps, g, 0))) return rc;
         a.tstride = nd;
         a.traces = dev_out ? data_out + (size_t)s0 * nd : c->traces;
         // background and scattered states of the group (types BG .. R, contiguous)
         if ((rc = born_zero_types(c, PV_BG, PV_ADJ - PV_BG, g))) return rc;
         CK(c, cudaMemsetAsync(a.traces, 0, sizeof(float) * nd * g, c->stream));
-        for (int it = 0; it < nt; it++) CK(c, born_launch_step(a, it, true, false, c->stream));
+        for (int it = 0; it < nt; it++) CK(c, born_launch_step(maps, a, it, true, false, c->stream));
         c->launches += 2LL * nt;
         if (!dev_out)
             CK(c, cudaMemcpyAsync(data_out + (size_t)s0 * nd, a.traces, sizeof(float) * nd * g,
                                   cudaMemcpyDeviceToHost, c->stream));
     }
-    CK(c, cudaStreamSynchronize(c->stream));
-    return ERTM_OK;
+    return check_device_error(c);
 }
 
 int ertm_born_forward(ertm_ctx* c, const ertm_shot* s, const float* r_vp, const float* r_vs,
@@ -1820,6 +1862,8 @@ int ertm_born_adjoint_shots(ertm_ctx* c, const ertm_shot* shots, int nshots, con
         const int g = std::min(G, nshots - s0);
         born_group_args(c, a, g);
         if ((rc = born_group_shots(c, a, shots + s0, g))) return rc;
+        BornMaps maps;
+        if ((rc = born_group_maps(c, a, maps, g, K))) return rc;
         a.tstride = nd;
         if (dev_res) a.traces = const_cast<float*>(residual) + (size_t)s0 * nd;
         else {
@@ -1841,7 +1885,7 @@ int ertm_born_adjoint_shots(ertm_ctx* c, const ertm_shot* shots, int nshots, con
         };
         for (int it = 0; it < nt; it++) {
             if (it % K == 0) CK(c, save(it / K));
-            CK(c, born_launch_step(a, it, false, false, c->stream));
+            CK(c, born_launch_step(maps, a, it, false, false, c->stream));
         }
         // 2. reverse sweep, one checkpoint segment at a time
         if ((rc = born_zero_types(c, PV_ADJ, PV_N - PV_ADJ, g))) return rc;   // adjoint, gradients, scratch
@@ -1855,18 +1899,17 @@ int ertm_born_adjoint_shots(ertm_ctx* c, const ertm_shot* shots, int nshots, con
                 a.kv0z = h + g * B.n;
                 a.ka0x = h + 2 * g * B.n;
                 a.ka0z = h + 3 * g * B.n;
-                CK(c, born_launch_step(a, it, false, true, c->stream));
+                CK(c, born_launch_step(maps, a, it, false, true, c->stream));
             }
             for (int it = t1 - 1; it >= t0; it--) {
                 const float* h = B.hist + (size_t)(it - t0) * 4 * g * B.n;
-                a.hv0x = h;
-                a.hv0z = h + g * B.n;
                 a.ha0x = h + 2 * g * B.n;
                 a.ha0z = h + 3 * g * B.n;
-                CK(c, born_launch_adjoint_step(a, it, c->stream));
+                a.t_hist = 4 * (it - t0);
+                CK(c, born_launch_adjoint_step(maps, a, it, c->stream));
             }
         }
-        c->launches += 2LL * nt * 2 + 3LL * nt + 1;
+        c->launches += 2LL * nt * 2 + 2LL * nt + 1;
         // 3. gradients w.r.t. the relative perturbations, summed over the group's shots
         CK(c, born_launch_final(a, tgt[0], tgt[1], tgt[2], s0 > 0, c->stream));
         c->launches++;
@@ -1874,8 +1917,7 @@ int ertm_born_adjoint_shots(ertm_ctx* c, const ertm_shot* shots, int nshots, con
     for (int q = 0; q < 3; q++)
         if (!dev[q])
             CK(c, cudaMemcpyAsync(outs[q], tgt[q], sizeof(float) * n, cudaMemcpyDeviceToHost, c->stream));
-    CK(c, cudaStreamSynchronize(c->stream));
-    return ERTM_OK;
+    return check_device_error(c);
 }
 
 int ertm_born_adjoint(ertm_ctx* c, const ertm_shot* s, const float* residual, float* g_vp,
