@@ -178,6 +178,10 @@ inline cudaError_t launch_pdl(void (*K)(P...), dim3 grid, dim3 block, size_t sme
     return cudaLaunchKernelEx(&cf, K, args...);
 }
 
+// In-kernel side of it: wait for the previous launch's memory; let the next one start.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // Host set-up shared by the context path and the no-allocation path (setup.cu).
 Geom make_geom(int nx, int ny, int nz, int R);
 // difference coefficients c_0..c_R (c_0 = 0) for ERTM_COEF_* `coef_kind`

@@ -35,11 +35,6 @@ struct Tile2 {
     static constexpr int XZ = XW * ZH, X = XW * TZ, Z = TX2 * ZH;
 };
 
-// Programmatic dependent launch: let the next step kernel set up while this one still
-// runs, and wait for the previous one's memory before touching any.
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-
 // Shared by both kernels: barrier set-up before, and memory access after, the wait for
 // the previous launch.
 __device__ __forceinline__ void tile2_begin(uint64_t* bar)
