@@ -684,7 +684,7 @@ int run_pass(ertm_ctx* c, int which, const ertm_shot* s, int mode, int nsteps, f
     int rc;
     float vmax = c->cfg.pml_vmax > 0 ? c->cfg.pml_vmax : c->vpmax[which];
     if ((rc = upload_profiles(c, vmax))) return rc;
-    int kchunk = choose_kchunk(c->g);
+    int kchunk = choose_kchunk(step_tiles(c->g), c->g.nz);
     if (c->cfg.autotune == 1 && (rc = autotune_kchunk(c, which, &kchunk))) return rc;
     if ((rc = reset_state(c))) return rc;
     if (mode != MODE_RECEIVER && (rc = upload_wavelet(c, s))) return rc;
@@ -1204,14 +1204,16 @@ int ertm_rtm_multi(ertm_ctx* const* ctx, int n, const ertm_shot* shots, const fl
         ertm_ctx* c = ctx[q];
         if ((rc = upload_profiles(c, c->cfg.pml_vmax > 0 ? c->cfg.pml_vmax : c->vpmax[1]))) return rc;
     }
-    int kchunk = choose_kchunk(c0->g);
-    if (c0->cfg.autotune == 1 && (rc = autotune_kchunk(c0, 1, &kchunk))) return rc;
-    const int chunks = (c0->g.nz + kchunk - 1) / kchunk;
+    long long tiles = 0;
     unsigned gx = 0, gy = 0;
     for (int q = 0; q < n; q++) {
+        tiles += step_tiles(ctx[q]->g);
         gx = std::max(gx, (unsigned)((ctx[q]->g.nx + TX - 1) / TX));
         gy = std::max(gy, (unsigned)((ctx[q]->g.ny + TY3 - 1) / TY3));
     }
+    int kchunk = choose_kchunk(tiles, c0->g.nz);
+    if (c0->cfg.autotune == 1 && (rc = autotune_kchunk(c0, 1, &kchunk))) return rc;
+    const int chunks = (c0->g.nz + kchunk - 1) / kchunk;
     const dim3 grid(gx, gy, (unsigned)(n * chunks));
     // the argument blocks travel by value in the kernels' parameter space
     std::unique_ptr<StressMulti> SP(new StressMulti());
@@ -1429,7 +1431,7 @@ int ertm_time_kernels(ertm_ctx* c, const ertm_shot* s, int nsteps, float* ms)
     if ((rc = upload_wavelet(c, s))) return rc;
     KArgs a;
     fill_args(c, 1, s, a);
-    a.kchunk = choose_kchunk(c->g);
+    a.kchunk = choose_kchunk(step_tiles(c->g), c->g.nz);
     const bool cpml = c->cfg.boundary == ERTM_BOUNDARY_CPML;
     cudaEvent_t ev[3];
     for (int q = 0; q < 3; q++) CK(c, cudaEventCreate(&ev[q]));

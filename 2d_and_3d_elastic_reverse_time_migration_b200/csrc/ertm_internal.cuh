@@ -193,8 +193,9 @@ void cpml_profile(int n, int w0, int w1, int stg, double h, double vmax, double 
 // sponge damping (1/s, ERTM_BOUNDARY_SPONGE_COS or _CUBIC ramps) of one axis of n
 // cells, for cells i0 .. i0+m-1 into v[0..m)
 void sponge_profile(int n, int w0, int w1, int kind, float coe, int i0, int m, float* v);
-// z planes per CTA of the 3D step kernels for grid g
-int choose_kchunk(const Geom& g);
+// tiles of the x-y plane of a 3D grid, and z planes per CTA of a launch over `tiles` of them
+long long step_tiles(const Geom& g);
+int choose_kchunk(long long tiles, int nz);
 
 // Launchers (one translation unit per stencil radius).
 cudaError_t launch_stress(int R, const Geom& g, const KArgs& a, const StressMaps& m, bool cpml,

@@ -357,7 +357,7 @@ int run_noalloc(const ertm_config* cfg, const float* vp, const float* vs, const 
     a.err = counters + 4;
 
     // z planes per CTA (3D): the context path's rule
-    a.kchunk = choose_kchunk(g);
+    a.kchunk = choose_kchunk(step_tiles(g), g.nz);
 
     // tensor maps over the scratch volumes
     StressMaps sm;

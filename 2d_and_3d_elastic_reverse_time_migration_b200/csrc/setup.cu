@@ -148,18 +148,37 @@ void sponge_profile(int n, int w0, int w1, int kind, float coe, int i0, int m, f
     }
 }
 
-// z planes per CTA of the 3D kernels: chunks of about 32 planes, balanced over nz.
-// Timed on B200 at 480 x 480 x 380 (R = 4, C-PML), the step kernels get faster as the
-// chunk shrinks from the whole column (380 planes) down to 32-48 planes
-// (stress 1.92 -> 1.51 ms, velocity 1.98 -> 1.61 ms per launch), while below
-// ~24 planes the z-queue fill of each chunk starts to cost more than the finer
-// load balance gains.
-int choose_kchunk(const Geom& g)
+// z planes per CTA of the 3D kernels for `tiles` tiles of the x-y plane (of every shot of a
+// launch).  From eight waves of CTAs on, balanced chunks of about 32 planes: the time is flat
+// from there to 40-48 (480 x 480 x 380, RTM: 235.0, 234.8, 234.6 ms for 32, 40, 48; five
+// windows of different sizes in one launch: 120.5, 120.7, 121.5) and grows above (236.1, 245.2
+// and 123.5, 128.7 for 64, 96) and below (237.5 and 121.3 for 24).  A smaller launch needs its
+// last wave full: the chunk of 8 to 48 planes with the least waves x (planes + start-up),
+// start-up being the fill of the z queues and of the ring, about 8 planes' time (151 x 133 x
+// 117, modelling, 80 steps: 9.45 ms in chunks of 30 planes, 340 CTAs on 296 places, and 8.19
+// in chunks of 39, 255 CTAs).
+int choose_kchunk(long long tiles, int nz)
 {
-    if (g.two_d) return g.nz;
-    const int target = 32;
-    const int chunks = std::max(1, (g.nz + target / 2) / target);
-    return (g.nz + chunks - 1) / chunks;
+    constexpr long long places = CTAS3 * 148;
+    const int n32 = std::max(1, (nz + 16) / 32);
+    int best = (nz + n32 - 1) / n32;
+    if (tiles * n32 >= 8 * places) return best;
+    double best_cost = 1e300;
+    for (int n = (nz + 47) / 48; n <= (nz + 7) / 8; n++) {
+        const int kc = (nz + n - 1) / n, chunks = (nz + kc - 1) / kc;
+        const long long waves = (tiles * chunks + places - 1) / places;
+        const double cost = (double)waves * (kc + 8);
+        if (cost < best_cost) {
+            best_cost = cost;
+            best = kc;
+        }
+    }
+    return best;
+}
+
+long long step_tiles(const Geom& g)
+{
+    return (long long)((g.nx + TX - 1) / TX) * ((g.ny + TY3 - 1) / TY3);
 }
 
 }  // namespace ertm

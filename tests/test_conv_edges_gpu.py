@@ -1,0 +1,125 @@
+"""The convolutions, their gradients and the elementwise kernels at the edges of their
+tiles, against PyTorch FP32 on the same BF16 inputs (GPU).
+
+Tolerances: a BF16 output is within half a unit in the last place of the FP32 result,
+2^-9 relative per element (2^-8 with room for a sum that rounds the other way), so 2^-8 in
+relative L2; FP32 weight gradients sum at most 5,000 products of exact BF16 factors here,
+each addition within 2^-24: 1e-4.  (PyTorch's TF32 convolutions are exact on BF16 factors.)"""
+import importlib
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+PKG = "2d_and_3d_elastic_reverse_time_migration_b200"
+BF16 = 2.0 ** -8
+
+
+@pytest.fixture(scope="module")
+def env():
+    import torch
+    nn = importlib.import_module(PKG + ".nn")
+    dev = torch.device("cuda", 0)
+    torch.manual_seed(1)
+    return torch, nn, nn.Ops(dev), dev
+
+
+def _rel(a, b):
+    a, b = a.detach().double(), b.detach().double()
+    return float((a - b).norm() / b.norm())
+
+
+def _nchw(t):
+    return t.permute(0, 3, 1, 2)
+
+
+# one pixel; images narrower, one short of, equal to and past the 254-pixel row of a tile;
+# channel counts that fill no swizzle span, one, several, and more than one output block
+@pytest.mark.parametrize("n,h,w,ci,co", [
+    (1, 1, 1, 32, 48), (3, 5, 13, 8, 16), (2, 7, 61, 24, 40), (1, 3, 253, 16, 64), (1, 2, 255, 48, 272),
+    (1, 3, 300, 64, 32), (2, 2, 31, 288, 16), (5, 9, 17, 128, 128), (1, 65, 3, 40, 8)])
+def test_conv_edges(env, n, h, w, ci, co):
+    torch, nn, ops, dev = env
+    F = torch.nn.functional
+    off, cs = 8, co + 16                       # outputs inside a wider tensor
+    x = torch.randn(n, h, w, ci, device=dev).bfloat16()
+    wt = (torch.randn(co, 9 * ci, device=dev) * 0.1).bfloat16()
+    bias = torch.randn(co, device=dev)
+    y = torch.full((n, h, w, cs), 7.0, device=dev, dtype=torch.bfloat16)
+    ops.conv(nn.act(x, n, h, w), wt, bias, nn.act(y, n, h, w, co, off), relu=True)
+    w4 = wt.float().view(co, 3, 3, ci).permute(0, 3, 1, 2).clone().requires_grad_(True)
+    xr = _nchw(x.float()).requires_grad_(True)
+    pre = F.conv2d(xr, w4, None, padding=1)
+    ref = F.relu(pre.detach() + bias.view(1, -1, 1, 1))
+    assert _rel(_nchw(y[..., off:off + co].float()), ref) <= BF16
+    assert bool((y[..., :off] == 7).all()) and bool((y[..., off + co:] == 7).all())
+    y32 = torch.zeros(n, h, w, co, device=dev)
+    ops.conv(nn.act(x, n, h, w), wt, bias, nn.act(y32, n, h, w), relu=False, y32=y32)
+    assert _rel(_nchw(y32), pre.detach() + bias.view(1, -1, 1, 1)) <= 1e-5
+    dy = torch.zeros(n, h, w, cs, device=dev, dtype=torch.bfloat16)
+    dy[..., off:off + co] = torch.randn(n, h, w, co, device=dev)
+    dyv = dy[..., off:off + co].float()
+    pre.backward(_nchw(dyv))
+    wf = torch.zeros(ci, 9 * co, device=dev, dtype=torch.bfloat16)
+    ops.flip3(wt, wf, co, ci)
+    dx = torch.zeros_like(x)
+    ops.conv_dgrad(nn.act(dy, n, h, w, co, off), wf, nn.act(dx, n, h, w), mask=nn.act(x, n, h, w))
+    assert _rel(_nchw(dx.float()), xr.grad * (xr.detach() > 0)) <= BF16
+    dw = torch.ones(co, 9 * ci, device=dev)    # accumulated
+    ops.conv_wgrad(nn.act(x, n, h, w), nn.act(dy, n, h, w, co, off), dw)
+    assert _rel(dw.view(co, 3, 3, ci).permute(0, 3, 1, 2) - 1, w4.grad) <= 1e-4
+    db = torch.zeros(co, device=dev)
+    ops.bias_grad(nn.act(dy, n, h, w, co, off), db)
+    assert _rel(db, dyv.sum(dim=(0, 1, 2))) <= 1e-4
+    assert int(ops.err.item()) == 0
+
+
+@pytest.mark.parametrize("n,h,w,ci,co", [(1, 1, 1, 8, 8), (2, 3, 7, 24, 40), (1, 2, 129, 64, 32), (3, 9, 33, 128, 64)])
+def test_up2_edges(env, n, h, w, ci, co):
+    torch, nn, ops, dev = env
+    F = torch.nn.functional
+    off, cs = 8, co + 24
+    x = torch.randn(n, h, w, ci, device=dev).bfloat16()
+    u = (torch.randn(4 * co, ci, device=dev) * 0.1).bfloat16()
+    bias = torch.randn(co, device=dev)
+    y = torch.full((n, 2 * h, 2 * w, cs), 7.0, device=dev, dtype=torch.bfloat16)
+    ops.up(nn.act(x, n, h, w), u, bias, nn.act(y, n, 2 * h, 2 * w, co, off), relu=False)
+    wt = u.float().view(2, 2, co, ci).permute(3, 2, 0, 1).contiguous().requires_grad_(True)
+    xr = _nchw(x.float()).requires_grad_(True)
+    ref = F.conv_transpose2d(xr, wt, None, stride=2)
+    assert _rel(_nchw(y[..., off:off + co].float()), ref + bias.view(1, -1, 1, 1)) <= BF16
+    assert bool((y[..., :off] == 7).all()) and bool((y[..., off + co:] == 7).all())
+    dy = torch.randn(n, 2 * h, 2 * w, cs, device=dev).bfloat16()
+    ref.backward(_nchw(dy[..., off:off + co].float()))
+    ut = torch.zeros(ci, 4 * co, device=dev, dtype=torch.bfloat16)
+    ops.transpose(u, ut, 4 * co, ci)
+    dx = torch.zeros_like(x)
+    dya = nn.act(dy, n, 2 * h, 2 * w, co, off)
+    ops.up_dgrad(dya, ut, nn.act(dx, n, h, w), mask=nn.act(x, n, h, w))
+    assert _rel(_nchw(dx.float()), xr.grad * (xr.detach() > 0)) <= BF16
+    du = torch.zeros(4 * co, ci, device=dev)
+    ops.up_wgrad(nn.act(x, n, h, w), dya, du)
+    assert _rel(du.view(2, 2, co, ci).permute(3, 2, 0, 1), wt.grad) <= 1e-4
+    assert int(ops.err.item()) == 0
+
+
+# the vector kernels (16-byte aligned dense operand) against the scalar ones, bit for bit
+@pytest.mark.parametrize("n,h,w,c", [(1, 2, 2, 8), (2, 6, 10, 24), (3, 4, 130, 136)])
+def test_pool_vector_equals_scalar(env, n, h, w, c):
+    torch, nn, ops, dev = env
+    x = torch.randn(n, h, w, c + 8, device=dev).bfloat16()
+    x[0, 0, :2] = -3.0e38                      # below every other value: the window has no maximum
+    xa = nn.act(x, n, h, w, c, 8)
+    size = n * (h // 2) * (w // 2) * c
+    flat = [torch.zeros(size + 1, device=dev, dtype=torch.bfloat16)[k:k + size] for k in (0, 1)]
+    for f in flat:
+        ops.pool(xa, f)
+    assert torch.equal(*flat)
+    dy = torch.randn(size, device=dev).bfloat16()
+    off = torch.zeros(size + 1, device=dev, dtype=torch.bfloat16)[1:]
+    off.copy_(dy)
+    for mask in (False, True):
+        dx = [torch.ones_like(x) for _ in range(2)]
+        for d, g in zip(dx, (dy, off)):
+            ops.pool_bwd(xa, g, nn.act(d, n, h, w, c, 8), relu_mask=mask)
+        assert torch.equal(*dx)
