@@ -1833,10 +1833,10 @@ int ertm_born_adjoint_shots(ertm_ctx* c, const ertm_shot* shots, int nshots, con
     const int nbg = 5 + (a.nm ? 9 : 0);   // background volume types in a checkpoint
     const long long nd = 3LL * nt * shots[0].nrx;
     const bool dev_res = is_device_ptr(residual);
-    const long long per_shot = B.n * ((long long)PV_N + 14LL * nck + 4LL * K) + (dev_res ? 0 : nd);
+    const long long per_shot = B.n * ((long long)PV_N + 14LL * (nck - 1) + 4LL * K) + (dev_res ? 0 : nd);
     const int G = born_group_size(c, nshots, per_shot);
     if ((rc = born_group_volumes(c, G))) return rc;
-    const long long ck_need = 14LL * nck * G * B.n, hist_need = 4LL * K * G * B.n;
+    const long long ck_need = 14LL * (nck - 1) * G * B.n, hist_need = 4LL * K * G * B.n;
     if (B.ckpt_floats < ck_need) {
         cudaFree(B.ckpt);
         B.ckpt = nullptr;
@@ -1885,23 +1885,40 @@ int ertm_born_adjoint_shots(ertm_ctx* c, const ertm_shot* shots, int nshots, con
             return cudaMemcpyAsync(B.pv[PV_BG], B.ckpt + seg * ck_seg, sizeof(float) * ck_seg,
                                    cudaMemcpyDeviceToDevice, c->stream);
         };
-        for (int it = 0; it < nt; it++) {
-            if (it % K == 0) CK(c, save(it / K));
-            CK(c, born_launch_step(maps, a, it, false, false, c->stream));
-        }
-        // 2. reverse sweep, one checkpoint segment at a time
-        if ((rc = born_zero_types(c, PV_ADJ, PV_N - PV_ADJ, g))) return rc;   // adjoint, gradients, scratch
-        CK(c, born_launch_inject(a, nt - 1, c->stream));
-        for (int sg = nck - 1; sg >= 0; sg--) {
-            const int t0 = sg * K, t1 = std::min(nt, t0 + K);
-            CK(c, load(sg));
-            for (int it = t0; it < t1; it++) {
+        // The segments end at nt, nt - K, ...: the last one is a full one, and its steps, which
+        // the reverse sweep needs first, record their history as they are made.  Only the
+        // earlier ones are made twice, once for the checkpoints and once for the history
+        // (592 x 336, 8 shots, 240 steps in segments of 100: 18.9 ms, 21.3 with every segment made
+        // twice).
+        auto seg_begin = [&](int seg) { return std::max(0, nt - (nck - seg) * K); };
+        auto seg_end = [&](int seg) { return nt - (nck - 1 - seg) * K; };
+        auto record = [&](int seg) {
+            const int t0 = seg_begin(seg);
+            for (int it = t0; it < seg_end(seg); it++) {
                 float* h = B.hist + (size_t)(it - t0) * 4 * g * B.n;
                 a.kv0x = h;
                 a.kv0z = h + g * B.n;
                 a.ka0x = h + 2 * g * B.n;
                 a.ka0z = h + 3 * g * B.n;
-                CK(c, born_launch_step(maps, a, it, false, true, c->stream));
+                const cudaError_t e = born_launch_step(maps, a, it, false, true, c->stream);
+                if (e != cudaSuccess) return e;
+            }
+            return cudaSuccess;
+        };
+        for (int sg = 0; sg < nck - 1; sg++) {
+            CK(c, save(sg));
+            for (int it = seg_begin(sg); it < seg_end(sg); it++)
+                CK(c, born_launch_step(maps, a, it, false, false, c->stream));
+        }
+        CK(c, record(nck - 1));
+        // 2. reverse sweep, one checkpoint segment at a time
+        if ((rc = born_zero_types(c, PV_ADJ, PV_N - PV_ADJ, g))) return rc;   // adjoint, gradients, scratch
+        CK(c, born_launch_inject(a, nt - 1, c->stream));
+        for (int sg = nck - 1; sg >= 0; sg--) {
+            const int t0 = seg_begin(sg), t1 = seg_end(sg);
+            if (sg < nck - 1) {
+                CK(c, load(sg));
+                CK(c, record(sg));
             }
             for (int it = t1 - 1; it >= t0; it--) {
                 const float* h = B.hist + (size_t)(it - t0) * 4 * g * B.n;
@@ -1911,7 +1928,7 @@ int ertm_born_adjoint_shots(ertm_ctx* c, const ertm_shot* shots, int nshots, con
                 CK(c, born_launch_adjoint_step(maps, a, it, c->stream));
             }
         }
-        c->launches += 2LL * nt * 2 + 2LL * nt + 1;
+        c->launches += 2LL * (2 * nt - K) + 2LL * nt + 1;
         // 3. gradients w.r.t. the relative perturbations, summed over the group's shots
         CK(c, born_launch_final(a, tgt[0], tgt[1], tgt[2], s0 > 0, c->stream));
         c->launches++;
