@@ -74,6 +74,11 @@ class _NnAct(C.Structure):
                 ("cstride", C.c_int), ("coff", C.c_int), ("c", C.c_int)]
 
 
+class _NnOp(C.Structure):
+    _fields_ = [("kind", C.c_int), ("flag", C.c_int), ("p", C.c_int * 3), ("n", C.c_longlong),
+                ("a", _NnAct), ("b", _NnAct), ("m", _NnAct)]
+
+
 # every entry point of include/ertm.h: name -> (restype, argtypes)
 _P = C.c_void_p
 SIGNATURES = {
@@ -140,6 +145,7 @@ SIGNATURES = {
     "ertm_nn_flip3": (C.c_int, [_P, _P, C.c_int, C.c_int, _P]),
     "ertm_nn_transpose": (C.c_int, [_P, _P, C.c_int, C.c_int, _P]),
     "ertm_nn_to_bf16": (C.c_int, [_P, _P, C.c_longlong, _P]),
+    "ertm_nn_run": (C.c_int, [C.POINTER(_NnOp), C.c_int, C.POINTER(_P), C.c_int, C.POINTER(C.c_int), _P, _P]),
     "ertm_forward_together_using_real_model_noalloc": (
         C.c_int, [C.POINTER(_Config), _P, _P, _P, C.POINTER(_Shot), _P, _P, C.c_char_p, C.c_size_t]),
 }

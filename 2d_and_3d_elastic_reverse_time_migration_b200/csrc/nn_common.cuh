@@ -119,4 +119,22 @@ inline bool mask_ok(const ertm_nn_act* mask, const ertm_nn_act* dx)
                      mask->c == dx->c);
 }
 
+// 8 BF16 values of a 16-byte chunk
+__device__ __forceinline__ void unpack8(const uint4& u, float* f)
+{
+    const uint32_t* w = &u.x;
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        f[2 * q] = __uint_as_float(w[q] << 16);
+        f[2 * q + 1] = __uint_as_float(w[q] & 0xffff0000u);
+    }
+}
+
 }  // namespace
+
+namespace ertm {
+// ertm_nn_conv3x3_wgrad and ertm_nn_up2_wgrad with the bias gradient of the same dy, db += its
+// sum over the pixels, in the same kernel (db NULL: none).
+int nn_conv3x3_wgrad(const ertm_nn_act* x, const ertm_nn_act* dy, float* dw, float* db, int* err, void* stream);
+int nn_up2_wgrad(const ertm_nn_act* x, const ertm_nn_act* dy, float* du, float* db, int* err, void* stream);
+}  // namespace ertm

@@ -28,12 +28,13 @@
 //
 // Measured on B200 against cp.async-staged im2col tiles (and, for widths in multiples of
 // 128, rows of 128 pixels), one tile per CTA: loss and gradients of a 16 x 256 x 512 batch
-// 14.08 -> 2.53 ms, one 256 x 512 image forward 595 -> 218 us (bit-identical), a single
+// 14.08 -> 2.32 ms, one 256 x 512 image forward 595 -> 157 us (bit-identical), a single
 // 32 -> 48 layer on 5 x 61 x 107 with its gradients 264 -> 50 us.  Of the batch's way:
 // 16-byte planes and one thread computing every descriptor 3.86 ms; swizzled blocks 4.07
 // (no line bound yet, more arithmetic per MMA), the warp computing them in uniform registers
 // 3.60, MMA tables 2.86, four epilogue warps per lane quarter with the mask read ahead and
-// the 2x2 sums through shared memory 2.53.
+// the 2x2 sums through shared memory 2.53, the bias gradients taken by the weight gradients'
+// idle warps and one call per pass 2.32 (the 18 separate bias kernels took 212 us).
 //
 // What bounds them: at 16-32 channels a layer moves 64-200 bytes per pixel for 5-18 kFLOP,
 // the HBM side; next to it the lines of the boxes (TMA moves one in 1.6, 2.7, 3.4 or 7
@@ -577,7 +578,8 @@ struct WgMaps {
 // chain.  x and dy are read past the last column and row as zeros, so an infinite
 // activation in the last column meets a zero gradient there.
 __global__ void __launch_bounds__(CTHREADS, 1) k_wgrad(const __grid_constant__ WgMaps maps,
-                                                       const __grid_constant__ WgP p, float* __restrict__ dw, int* err)
+                                                       const __grid_constant__ WgP p, float* __restrict__ dw,
+                                                       float* __restrict__ db, int* err)
 {
     extern __shared__ __align__(1024) uint8_t sm[];
     __shared__ uint64_t full[MAXSLOT], empty[MAXSLOT], done;
@@ -586,10 +588,11 @@ __global__ void __launch_bounds__(CTHREADS, 1) k_wgrad(const __grid_constant__ W
     const int kx0 = blockIdx.y * p.nkx;
     const int c0 = (int)(blockIdx.z % p.cparts) * p.CB * p.cx, o0 = (int)(blockIdx.z / p.cparts) * p.OB * p.cy;
     const int ca = p.up ? p.cy : p.cx, cn = p.up ? p.cx : p.cy;   // channels per block of the M and N side
+    const bool bias = db && blockIdx.y == 0 && blockIdx.z % p.cparts == 0;   // each dy tile counts once
     if (threadIdx.x == 0) {
         for (int q = 0; q < p.stages; q++) {
             mbar_init(&full[q], 1);
-            mbar_init(&empty[q], 1);
+            mbar_init(&empty[q], bias ? 1 + EPW : 1);
         }
         mbar_init(&done, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -670,6 +673,53 @@ __global__ void __launch_bounds__(CTHREADS, 1) k_wgrad(const __grid_constant__ W
         if (el) umma_commit(&done);
         if (!mbar_wait(&done, 0)) ok = false;
     }
+    // bias: these warps wait for the sums anyway and add up dy's staged pixels meanwhile.  A
+    // thread sums 8 channels over its pixels, neighbouring threads on neighbouring chunks.
+    const int cpb = p.cy / 8, nch = p.OB * cpb, lanes = 32 * EPW / nch;
+    const int ch = threadIdx.x % nch, ln = threadIdx.x / nch;
+    float bs[8];
+#pragma unroll
+    for (int e = 0; e < 8; e++) bs[e] = 0.f;
+    if (bias && warp < EPW) {
+        const uint32_t pitch = p.up ? p.pitchA : p.rr * p.pitchB;    // bytes of a staged block
+        const uint32_t px = 2 * p.cy, swz = cpb - 1;                 // SWIZZLE_(2 cy)B: chunk ^ 128-byte line
+        const uint32_t from = su32(sm) + (p.up ? 0 : p.abytes) + (ch / cpb) * pitch + (ch % cpb) * 16;
+        const int npx = p.rr * p.tw;
+        auto load = [&](uint32_t at, float* f) {
+            uint4 v;
+            at ^= (at >> 7 & swz) << 4;
+            asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(at));
+            unpack8(v, f);
+        };
+        int i = 0;
+        for (int u = blockIdx.x; u < p.units; u += gridDim.x, i++) {
+            const int sl = i % p.stages;
+            if (!all_lanes(mbar_wait(&full[sl], (i / p.stages) & 1))) {
+                ok = false;
+                break;
+            }
+            if (ln < lanes)
+                for (int ab = 0; ab < (p.up ? 4 : 1); ab++) {
+                    const uint32_t at = from + (uint32_t)sl * p.stage + (uint32_t)(ab * p.OB) * pitch;
+                    int q = ln;
+                    for (; q + 3 * lanes < npx; q += 4 * lanes) {
+                        float f[4][8];
+#pragma unroll
+                        for (int k = 0; k < 4; k++) load(at + (uint32_t)(q + k * lanes) * px, f[k]);
+#pragma unroll
+                        for (int e = 0; e < 8; e++) bs[e] += (f[0][e] + f[1][e]) + (f[2][e] + f[3][e]);
+                    }
+                    for (; q < npx; q += lanes) {
+                        float f[8];
+                        load(at + (uint32_t)q * px, f);
+#pragma unroll
+                        for (int e = 0; e < 8; e++) bs[e] += f[e];
+                    }
+                }
+            __syncwarp();
+            if (lane == 0) mbar_arrive1(&empty[sl]);
+        }
+    }
     // TMEM loads are warp-collective and shared memory is reused: the decision is the block's
     const bool all_ok = __syncthreads_and(ok ? 1 : 0) != 0;
     tc_fence_after();
@@ -684,6 +734,21 @@ __global__ void __launch_bounds__(CTHREADS, 1) k_wgrad(const __grid_constant__ W
         // in banks) to be added along them
         const int ups = cw + 1;
         const bool staged = p.up && p.staged;
+        if (bias) {
+            if (epi)
+#pragma unroll
+                for (int e = 0; e < 8; e++) acc[threadIdx.x * 9 + e] = bs[e];
+            __syncthreads();
+            // channel o of the CTA's 8 nch, one of S partial sums over the pixel lanes
+            const int no = 8 * nch, S = max(1, 32 * EPW / no);
+            for (int t = threadIdx.x; t < S * no; t += CTHREADS) {
+                const int o = t % no;
+                float v = 0.f;
+                for (int l = t / no; l < lanes; l += S) v += acc[(l * nch + o / 8) * 9 + o % 8];
+                if (o0 + o < p.co) atomicAdd(db + o0 + o, v);
+            }
+            __syncthreads();
+        }
         if (!direct) {
             for (int q = threadIdx.x; q < na; q += CTHREADS) acc[q] = 0.f;
             __syncthreads();
@@ -1075,7 +1140,8 @@ bool wgrad_plan(WgP& best, size_t& smem, dim3& grid, int nb, int h, int w, int c
                             best_cost = cost;
                             best = p;
                             best.toff = (uint32_t)stages * p.stage;
-                            smem = std::max((size_t)stages * p.stage + over + table, accb);
+                            // the bias's partial sums take 36 bytes of every summing thread
+                            smem = std::max({(size_t)stages * p.stage + over + table, accb, (size_t)32 * EPW * 36});
                             grid = dim3(splits, p.kgroups, p.cparts * div_up(oblk, p.OB));
                         }
                     }
@@ -1085,7 +1151,7 @@ bool wgrad_plan(WgP& best, size_t& smem, dim3& grid, int nb, int h, int w, int c
     return best_cost < 1e299;
 }
 
-cudaError_t wgrad_launch(const Act& x, const Act& dy, float* dw, bool up, int* err, cudaStream_t st)
+cudaError_t wgrad_launch(const Act& x, const Act& dy, float* dw, float* db, bool up, int* err, cudaStream_t st)
 {
     struct Plan {
         WgP p;
@@ -1118,10 +1184,31 @@ cudaError_t wgrad_launch(const Act& x, const Act& dy, float* dw, bool up, int* e
     static unsigned long long opted = 0;
     const cudaError_t e = ertm::smem_opt_in(k_wgrad, SMEM_MAX, &opted);
     if (e != cudaSuccess) return e;
-    return ertm::launch_pdl(k_wgrad, grid, dim3(CTHREADS), smem, st, maps, p, dw, err);
+    return ertm::launch_pdl(k_wgrad, grid, dim3(CTHREADS), smem, st, maps, p, dw, db, err);
 }
 
 }  // namespace
+
+namespace ertm {
+int nn_conv3x3_wgrad(const ertm_nn_act* x, const ertm_nn_act* dy, float* dw, float* db, int* err, void* stream)
+{
+    if (!act_ok(x) || !act_ok(dy) || !dw || (db && !same_grid(x, dy))) return ERTM_EINVAL;
+    Act da = act_of(dy);            // dy's pixels are taken in x's grid, in order
+    da.nb = x->n;
+    da.h = x->h;
+    da.w = x->w;
+    return rc_of(wgrad_launch(act_of(x), da, dw, db, false, err, (cudaStream_t)stream));
+}
+
+int nn_up2_wgrad(const ertm_nn_act* x, const ertm_nn_act* dy, float* du, float* db, int* err, void* stream)
+{
+    if (!act_ok(x) || !act_ok(dy) || !du || dy->h != 2 * x->h || dy->w != 2 * x->w || (db && dy->n != x->n))
+        return ERTM_EINVAL;
+    Act da = act_of(dy);
+    da.nb = x->n;
+    return rc_of(wgrad_launch(act_of(x), da, du, db, true, err, (cudaStream_t)stream));
+}
+}  // namespace ertm
 
 // ---------------------------------------------------------------------------
 // C ABI
@@ -1160,12 +1247,7 @@ int ertm_nn_conv3x3_dgrad(const ertm_nn_act* dy, const void* wflip, const ertm_n
 int ertm_nn_conv3x3_wgrad(const ertm_nn_act* x, const ertm_nn_act* dy, float* dw, int splitk, int* err, void* stream)
 {
     (void)splitk;   // a hint: the plan splits the pixels by itself
-    if (!act_ok(x) || !act_ok(dy) || !dw) return ERTM_EINVAL;
-    Act da = act_of(dy);            // dy's pixels are taken in x's grid, in order
-    da.nb = x->n;
-    da.h = x->h;
-    da.w = x->w;
-    return rc_of(wgrad_launch(act_of(x), da, dw, false, err, (cudaStream_t)stream));
+    return ertm::nn_conv3x3_wgrad(x, dy, dw, nullptr, err, stream);
 }
 
 int ertm_nn_up2(const ertm_nn_act* x, const void* u, const float* bias, const ertm_nn_act* y, int relu, int* err,
@@ -1196,10 +1278,7 @@ int ertm_nn_up2_dgrad(const ertm_nn_act* dy, const void* ut, const ertm_nn_act* 
 int ertm_nn_up2_wgrad(const ertm_nn_act* x, const ertm_nn_act* dy, float* du, int splitk, int* err, void* stream)
 {
     (void)splitk;
-    if (!act_ok(x) || !act_ok(dy) || !du || dy->h != 2 * x->h || dy->w != 2 * x->w) return ERTM_EINVAL;
-    Act da = act_of(dy);
-    da.nb = x->n;
-    return rc_of(wgrad_launch(act_of(x), da, du, true, err, (cudaStream_t)stream));
+    return ertm::nn_up2_wgrad(x, dy, du, nullptr, err, stream);
 }
 
 }  // extern "C"

@@ -21,7 +21,7 @@ from dataclasses import dataclass
 
 import numpy as np
 
-from . import ErtmError, _NnAct, lib
+from . import ErtmError, _NnAct, _NnOp, lib
 
 IN_C, OUT_C = 3, 3
 IN_P, OUT_P = 8, 16
@@ -122,6 +122,57 @@ class Ops:
 
     def to_bf16(self, a, b):
         _ck(self.L.ertm_nn_to_bf16(_p(a), _p(b), a.numel(), self.st), "to_bf16")
+
+
+# ertm_nn_op kinds, in the header's order
+(CONV, CONV_DGRAD, CONV_WGRAD, UP, UP_DGRAD, UP_WGRAD, POOL, POOL_BWD, ZERO, PACK) = range(10)
+
+
+class OpList:
+    """A list of operations for ertm_nn_run: their kinds and the views of the network's own
+    buffers are laid out once, the pointers of everything else are read at each call from the
+    tensors that `table` names at that time (entries: a tensor of the buffers, or the
+    parameter's name and its attribute).  One call from Python per pass: the calls one by one took
+    about 10 us of host time per layer, more than a layer of one 256 x 512 image runs
+    (its forward pass of 22 launches took 218 us, 157 as a list)."""
+
+    def __init__(self):
+        self.ops, self.table = [], []
+
+    def add(self, kind, a=None, b=None, m=None, p=(), flag=0, n=0):
+        o = _NnOp()
+        o.kind, o.n = kind, n
+        o.flag = int(m is not None) if kind in (CONV_DGRAD, UP_DGRAD) else int(flag)
+        for k in range(3):
+            o.p[k] = -1
+        for k, e in enumerate(p):
+            if e is not None:                    # table slot 0: the call's input, "x"
+                o.p[k] = 0 if isinstance(e, str) else 1 + len(self.table)
+                if not isinstance(e, str):
+                    self.table.append(e)
+        for name, v in (("a", a), ("b", b), ("m", m)):
+            if v is not None:
+                setattr(o, name, v)
+        self.ops.append(o)
+
+    def seal(self):
+        self.ops = (_NnOp * len(self.ops))(*self.ops)
+        return self
+
+    def run(self, o, params, x=None, first=0, ops=None):
+        """Runs the operations from `first` on, on torch's current stream; `ops`: a changed
+        copy of the list."""
+        ops = self.ops if ops is None else ops
+        ptrs = (C.c_void_p * (1 + len(self.table)))(
+            _p(x), *[(getattr(params[e[0]], e[1]) if type(e) is tuple else e).data_ptr() for e in self.table])
+        done = C.c_int(0)
+        rc = o.L.ertm_nn_run(C.byref(ops[0], first * C.sizeof(_NnOp)), len(ops) - first, ptrs, len(ptrs),
+                             C.byref(done), o.err.data_ptr(), o.st)
+        _ck(rc, f"operation {first + done.value} of the U-Net pass")
+
+
+class Buffers(tuple):
+    """(activations, gradients) of one input size, with the operation lists over them."""
 
 
 @dataclass
@@ -230,84 +281,111 @@ class UNet:
         B["out"] = self._new((n, h, w, OUT_P))
         G = {k: t.zeros_like(v) for k, v in B.items() if k != "out"}
         G["out"] = self._new((n, h, w, OUT_P), bf)
-        self.bufs[key] = (B, G)
-        return B, G
+        b = self.bufs[key] = Buffers((B, G))
+        b.fwd, b.bwd = self._forward_ops(B, n, h, w), self._backward_ops(B, G, n, h, w)
+        return b
 
     # ---- forward / backward -------------------------------------------------
-    def forward(self, x):
-        """x: (n, h, w, 3) float32 CUDA tensor, h and w multiples of 8 -> (n, h, w, 3) float32."""
-        n, h, w, _ = x.shape
-        assert h % 8 == 0 and w % 8 == 0
-        B, G = self._buffers(n, h, w)
-        o, P = self.ops, self.params
-        B["in0"].zero_()
-        B["in0"][..., :IN_C].copy_(x)
+    def _forward_ops(self, B, n, h, w):
+        L = OpList()
+        L.add(PACK, b=act(B["in0"], n, h, w), p=("x",), flag=IN_C)
+
+        def conv(x, name, y, relu=True, y32=None):
+            L.add(CONV, x, y, p=((name, "wb"), (name, "b"), y32), flag=relu)
+
         for l, c in enumerate(LEVELS):
             hh, ww = h >> l, w >> l
-            cin = B[f"in{l}"]
-            o.conv(act(cin, n, hh, ww), P[f"e{l}a"].wb, P[f"e{l}a"].b, act(B[f"e{l}a"], n, hh, ww))
+            ea = act(B[f"e{l}a"], n, hh, ww)
             eb = act(B[f"cat{l}"], n, hh, ww, c, c) if l < 3 else act(B["e3b"], n, hh, ww)
-            o.conv(act(B[f"e{l}a"], n, hh, ww), P[f"e{l}b"].wb, P[f"e{l}b"].b, eb)
+            conv(act(B[f"in{l}"], n, hh, ww), f"e{l}a", ea)
+            conv(ea, f"e{l}b", eb)
             if l < 3:
-                o.pool(eb, B[f"in{l + 1}"])
+                L.add(POOL, eb, p=(B[f"in{l + 1}"],))
         prev = act(B["e3b"], n, h >> 3, w >> 3)
         for l in (2, 1, 0):
             c, hh, ww = LEVELS[l], h >> l, w >> l
-            o.up(prev, P[f"u{l}"].wb, P[f"u{l}"].b, act(B[f"cat{l}"], n, hh, ww, c, 0))
-            o.conv(act(B[f"cat{l}"], n, hh, ww), P[f"d{l}a"].wb, P[f"d{l}a"].b, act(B[f"d{l}a"], n, hh, ww))
-            o.conv(act(B[f"d{l}a"], n, hh, ww), P[f"d{l}b"].wb, P[f"d{l}b"].b, act(B[f"d{l}b"], n, hh, ww))
-            prev = act(B[f"d{l}b"], n, hh, ww)
-        o.conv(prev, P["out"].wb, P["out"].b, _out_view(B["out"], n, h, w), relu=False, y32=B["out"])
+            da, db = act(B[f"d{l}a"], n, hh, ww), act(B[f"d{l}b"], n, hh, ww)
+            L.add(UP, prev, act(B[f"cat{l}"], n, hh, ww, c, 0), p=((f"u{l}", "wb"), (f"u{l}", "b")), flag=1)
+            conv(act(B[f"cat{l}"], n, hh, ww), f"d{l}a", da)
+            conv(da, f"d{l}b", db)
+            prev = db
+        conv(prev, "out", _out_view(B["out"], n, h, w), relu=False, y32=B["out"])
+        return L.seal()
+
+    def forward(self, x):
+        """x: (n, h, w, 3) float32 CUDA tensor, h and w multiples of 8 -> (n, h, w, 3) float32."""
+        n, h, w, c = x.shape
+        assert h % 8 == 0 and w % 8 == 0
+        bufs = self._buffers(n, h, w)
+        B = bufs[0]
+        # dense FP32 input on the network's device is packed by the list's first operation;
+        # anything else that a copy can convert goes through torch
+        if (c == IN_C and x.dtype is self.torch.float32 and x.device == B["in0"].device and x.is_contiguous()
+                and type(x) is self.torch.Tensor and not x.requires_grad):
+            bufs.fwd.run(self.ops, self.params, x)
+        else:
+            B["in0"].zero_()
+            B["in0"][..., :IN_C].copy_(x)
+            bufs.fwd.run(self.ops, self.params, first=1)
         return B["out"][..., :OUT_C]
 
-    def backward(self, gout):
-        """gout: BF16 (n, h, w, OUT_P) gradient of the loss w.r.t. the output; fills p.g, p.bg."""
-        n, h, w, _ = gout.shape
-        B, G = self._buffers(n, h, w)
-        o, P = self.ops, self.params
-        for p in P.values():
-            p.g.zero_()
-            p.bg.zero_()
-        # output convolution
+    def _backward_ops(self, B, G, n, h, w):
+        L = OpList()
+        for name, p in self.params.items():
+            L.add(ZERO, p=((name, "g"),), n=p.g.numel())
+            L.add(ZERO, p=((name, "bg"),), n=p.bg.numel())
+
+        def grads(kind, x, dy, name):
+            L.add(UP_WGRAD if kind == UP else CONV_WGRAD, x, dy, p=((name, "g"), (name, "bg")))
+
+        def dgrad(kind, dy, name, dx, mask=None):
+            L.add(UP_DGRAD if kind == UP else CONV_DGRAD, dy, dx, mask, p=((name, "aux"),))
+
+        # output convolution; `gout`: the view of the call's gradient
         d0b = act(B["d0b"], n, h, w)
-        go = act(gout, n, h, w)
-        o.conv_wgrad(d0b, go, P["out"].g)
-        o.bias_grad(go, P["out"].bg)
-        o.conv_dgrad(go, P["out"].aux, act(G["d0b"], n, h, w), mask=d0b)
+        go = act(G["out"], n, h, w)
+        L.gout = len(L.ops)
+        grads(CONV, d0b, go, "out")
+        dgrad(CONV, go, "out", act(G["d0b"], n, h, w), d0b)
         for l in (0, 1, 2):
             c, hh, ww = LEVELS[l], h >> l, w >> l
-            gdb = act(G[f"d{l}b"], n, hh, ww)
-            o.conv_wgrad(act(B[f"d{l}a"], n, hh, ww), gdb, P[f"d{l}b"].g)
-            o.bias_grad(gdb, P[f"d{l}b"].bg)
-            o.conv_dgrad(gdb, P[f"d{l}b"].aux, act(G[f"d{l}a"], n, hh, ww), mask=act(B[f"d{l}a"], n, hh, ww))
-            gda = act(G[f"d{l}a"], n, hh, ww)
-            o.conv_wgrad(act(B[f"cat{l}"], n, hh, ww), gda, P[f"d{l}a"].g)
-            o.bias_grad(gda, P[f"d{l}a"].bg)
-            o.conv_dgrad(gda, P[f"d{l}a"].aux, act(G[f"cat{l}"], n, hh, ww), mask=act(B[f"cat{l}"], n, hh, ww))
+            da, cat = act(B[f"d{l}a"], n, hh, ww), act(B[f"cat{l}"], n, hh, ww)
+            gdb, gda = act(G[f"d{l}b"], n, hh, ww), act(G[f"d{l}a"], n, hh, ww)
+            grads(CONV, da, gdb, f"d{l}b")
+            dgrad(CONV, gdb, f"d{l}b", gda, da)
+            grads(CONV, cat, gda, f"d{l}a")
+            dgrad(CONV, gda, f"d{l}a", act(G[f"cat{l}"], n, hh, ww), cat)
             # transposed convolution that produced cat[:, :c]
             gup = act(G[f"cat{l}"], n, hh, ww, c, 0)
             src = act(B["e3b"] if l == 2 else B[f"d{l + 1}b"], n, hh >> 1, ww >> 1)
-            o.up_wgrad(src, gup, P[f"u{l}"].g)
-            o.bias_grad(gup, P[f"u{l}"].bg)
-            gsrc = G["e3b"] if l == 2 else G[f"d{l + 1}b"]
-            o.up_dgrad(gup, P[f"u{l}"].aux, act(gsrc, n, hh >> 1, ww >> 1), mask=src)
+            gsrc = act(G["e3b"] if l == 2 else G[f"d{l + 1}b"], n, hh >> 1, ww >> 1)
+            grads(UP, src, gup, f"u{l}")
+            dgrad(UP, gup, f"u{l}", gsrc, src)
         # encoder, deepest first; the skip gradients already sit in cat[:, c:]
         for l in (3, 2, 1, 0):
             c, hh, ww = LEVELS[l], h >> l, w >> l
             if l == 3:
-                geb, eb = act(G["e3b"], n, hh, ww), act(B["e3b"], n, hh, ww)
+                geb = act(G["e3b"], n, hh, ww)
             else:
                 geb, eb = act(G[f"cat{l}"], n, hh, ww, c, c), act(B[f"cat{l}"], n, hh, ww, c, c)
                 # pooling of this level's output fed level l+1
-                o.pool_bwd(eb, G[f"in{l + 1}"], geb, relu_mask=True)
-            o.conv_wgrad(act(B[f"e{l}a"], n, hh, ww), geb, P[f"e{l}b"].g)
-            o.bias_grad(geb, P[f"e{l}b"].bg)
-            gea = act(G[f"e{l}a"], n, hh, ww)
-            o.conv_dgrad(geb, P[f"e{l}b"].aux, gea, mask=act(B[f"e{l}a"], n, hh, ww))
-            o.conv_wgrad(act(B[f"in{l}"], n, hh, ww), gea, P[f"e{l}a"].g)
-            o.bias_grad(gea, P[f"e{l}a"].bg)
+                L.add(POOL_BWD, eb, geb, p=(G[f"in{l + 1}"],), flag=1)
+            ea, gea = act(B[f"e{l}a"], n, hh, ww), act(G[f"e{l}a"], n, hh, ww)
+            grads(CONV, ea, geb, f"e{l}b")
+            dgrad(CONV, geb, f"e{l}b", gea, ea)
+            grads(CONV, act(B[f"in{l}"], n, hh, ww), gea, f"e{l}a")
             if l > 0:
-                o.conv_dgrad(gea, P[f"e{l}a"].aux, act(G[f"in{l}"], n, hh, ww))
+                dgrad(CONV, gea, f"e{l}a", act(G[f"in{l}"], n, hh, ww))
+        return L.seal()
+
+    def backward(self, gout):
+        """gout: BF16 (n, h, w, OUT_P) gradient of the loss w.r.t. the output; fills p.g, p.bg."""
+        n, h, w, _ = gout.shape
+        L = self._buffers(n, h, w).bwd
+        ops = type(L.ops).from_buffer_copy(L.ops)
+        go = act(gout, n, h, w)
+        ops[L.gout].b = ops[L.gout + 1].a = go
+        L.run(self.ops, self.params, ops=ops)
 
     def loss_grad(self, x, target):
         """Forward, mean-squared error against target ((n, h, w, 3) float32) and backward:

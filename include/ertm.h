@@ -463,6 +463,33 @@ int ertm_nn_flip3(const void *w, void *wf, int co, int ci, void *stream);
 int ertm_nn_transpose(const void *a, void *t, int rows, int cols, void *stream);
 int ertm_nn_to_bf16(const float *a, void *b, long long n, void *stream);
 
+/* A list of the operations above in one call, for a network whose layers are shorter than
+ * their calls: each entry names an operation, the views it takes and, by their place in the
+ * call's pointer table, its other operands (-1: NULL).
+ *   kind         a    b    m     p[0]   p[1]  p[2]  flag
+ *   CONV         x    y    -     w      bias  y32   relu
+ *   CONV_DGRAD   dy   dx   mask  wflip  -     -     1: m is a mask
+ *   CONV_WGRAD   x    dy   -     dw     db    -     -      (db: dy's bias gradient too)
+ *   UP           x    y    -     u      bias  -     relu
+ *   UP_DGRAD     dy   dx   mask  ut     -     -     1: m is a mask
+ *   UP_WGRAD     x    dy   -     du     db    -     -
+ *   POOL         x    -    -     y      -     -     -
+ *   POOL_BWD     x    dx   -     dy     -     -     relu_mask
+ *   ZERO         -    -    -     FP32 array of n elements; neighbours share a launch
+ *   PACK         -    y    -     FP32 array of flag <= 8 values per pixel of y, which is
+ *                                dense with 8 channels: BF16, padding zero
+ * Stops at the first operation that fails and returns its code; *done (may be NULL) is the
+ * number of operations that were launched. */
+enum { ERTM_NN_OP_CONV, ERTM_NN_OP_CONV_DGRAD, ERTM_NN_OP_CONV_WGRAD, ERTM_NN_OP_UP, ERTM_NN_OP_UP_DGRAD,
+       ERTM_NN_OP_UP_WGRAD, ERTM_NN_OP_POOL, ERTM_NN_OP_POOL_BWD, ERTM_NN_OP_ZERO, ERTM_NN_OP_PACK };
+typedef struct ertm_nn_op {
+    int kind, flag, p[3];
+    long long n;
+    ertm_nn_act a, b, m;
+} ertm_nn_op;
+int ertm_nn_run(const ertm_nn_op *ops, int nops, void *const *ptr, int nptr, int *done, int *err,
+                void *stream);
+
 #ifdef __cplusplus
 }
 #endif

@@ -5,6 +5,7 @@ Tolerances: a BF16 output is within half a unit in the last place of the FP32 re
 2^-9 relative per element (2^-8 with room for a sum that rounds the other way), so 2^-8 in
 relative L2; FP32 weight gradients sum at most 5,000 products of exact BF16 factors here,
 each addition within 2^-24: 1e-4.  (PyTorch's TF32 convolutions are exact on BF16 factors.)"""
+import ctypes as C
 import importlib
 
 import pytest
@@ -123,3 +124,41 @@ def test_pool_vector_equals_scalar(env, n, h, w, c):
         for d, g in zip(dx, (dy, off)):
             ops.pool_bwd(xa, g, nn.act(d, n, h, w, c, 8), relu_mask=mask)
         assert torch.equal(*dx)
+
+
+# one packed pass from a dense FP32 input against the general path (views, other types)
+@pytest.mark.parametrize("n,h,w", [(1, 8, 8), (2, 16, 24)])
+def test_op_lists(env, n, h, w):
+    torch, nn, ops, dev = env
+    net = nn.UNet(dev, seed=2)
+    x = torch.randn(n, h, w, 3, device=dev)
+    want = net.forward(x).clone()
+    wide = torch.randn(n, h, w, 5, device=dev)
+    wide[..., 1:4] = x
+    for other in (wide[..., 1:4], x.double(), x.cpu()):
+        assert torch.equal(net.forward(other), want)
+    B, G = net._buffers(n, h, w)
+    o, P = net.ops, net.params                 # the first layers one by one
+    ea, eb = torch.zeros_like(B["e0a"]), torch.zeros_like(B["cat0"])
+    o.conv(nn.act(B["in0"], n, h, w), P["e0a"].wb, P["e0a"].b, nn.act(ea, n, h, w))
+    o.conv(nn.act(ea, n, h, w), P["e0b"].wb, P["e0b"].b, nn.act(eb, n, h, w, 16, 16))
+    assert torch.equal(ea, B["e0a"]) and torch.equal(eb[..., 16:], B["cat0"][..., 16:])
+    g = torch.randn(n, h, w, nn.OUT_P, device=dev).bfloat16()
+    for p in P.values():
+        p.g.fill_(3.0)                         # zeroed by the pass
+        p.bg.fill_(3.0)
+    net.backward(g)
+    dw, db = torch.zeros_like(P["out"].g), torch.zeros_like(P["out"].bg)
+    o.conv_wgrad(nn.act(B["d0b"], n, h, w), nn.act(g, n, h, w), dw)
+    o.bias_grad(nn.act(g, n, h, w), db)
+    assert _rel(P["out"].g, dw) <= 1e-5 and _rel(P["out"].bg, db) <= 1e-5
+    # refused: an unknown operation, a pointer outside the table
+    L = nn.lib()
+    ptr, done = (C.c_void_p * 1)(x.data_ptr()), C.c_int(9)
+    op = type(net._buffers(n, h, w).fwd.ops[0])()
+    for kind, p0 in ((99, 0), (nn.ZERO, 1), (nn.ZERO, -1)):
+        op.kind, op.n = kind, 4
+        op.p[0] = p0
+        rc = L.ertm_nn_run(C.byref(op), 1, ptr, 1, C.byref(done), None, o.st)
+        assert rc == -1 and done.value == 0
+    assert int(o.err.item()) == 0
