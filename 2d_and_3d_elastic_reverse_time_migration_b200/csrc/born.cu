@@ -41,9 +41,9 @@
 // fill its wait, so a grid in L2 costs little more than the launch and a large group
 // streams.  Before, each warp marched down 8-32 rows with one round trip per row.
 // Measured on B200, ms per call before -> now: Born forward, 10 shots of 880 x 480, three
-// mechanisms, 100 steps 34.4 -> 22.5 (4.96 TB/s of the 264 B per shot-cell and step that
+// mechanisms, 100 steps 34.4 -> 20.9 (5.34 TB/s of the 264 B per shot-cell and step that
 // the pair of kernels cannot do without); adjoint, 8 shots of 592 x 336, elastic, 240
-// steps 37.5 -> 21.2.
+// steps 37.5 -> 21.2, before its last segment's rebuild went.
 //
 // Tiles start at allocated columns 64 b (cell 64 b - BXH): every row access is whole
 // 128-byte lines.  Lanes on the zero halo columns load and compute and store nothing.
@@ -303,7 +303,7 @@ __global__ void __launch_bounds__(256, 2) k_born_velocity(const __grid_constant_
             const int t = f ? a.t_v + 2 : a.t_v0 + 2;      // sigma_xx, zz, xz
             tma4(d, &maps.x, gx, S.kt + R, sh, t, &bar);
             tma4(d + O_ZZ, &maps.z, S.ax, S.kt, sh, t + 1, &bar);
-            tma4(d + O_XZ, &maps.xz, gx, S.kt, sh, t + 2, &bar);
+            tma4(d + O_XZ, &maps.vxz, gx, S.kt, sh, t + 2, &bar);
         }
     }
     const int px = (int)a.px;
@@ -530,7 +530,7 @@ __global__ void __launch_bounds__(256, 2) k_adj_str(const __grid_constant__ Born
         mbar_expect_tx(&bar, 4u * (T::X + T::Z + T::XZ));
         tma4(sm, &maps.x, gx, S.kt + R, sh, a.t_s, &bar);
         tma4(sm + O_ZZ, &maps.z, S.ax, S.kt, sh, a.t_s + 1, &bar);
-        tma4(sm + O_XZ, &maps.xz, gx, S.kt, sh, a.t_s + 2, &bar);
+        tma4(sm + O_XZ, &maps.vxz, gx, S.kt, sh, a.t_s + 2, &bar);
     }
     const int px = (int)a.px;
     float* ax = a.ax + S.zo;
@@ -658,16 +658,16 @@ cudaError_t born_launch_pert(const BornArgs& a, const float* rvp, const float* r
 }
 
 namespace {
-dim3 tile_grid(const BornArgs& a)
+dim3 tile_grid(const BornArgs& a, int nr)
 {
-    return dim3((a.nx + BXH + TX2 - 1) / TX2, (a.nz + 4 * a.nr - 1) / (4 * a.nr), a.nshot);
+    return dim3((a.nx + BXH + TX2 - 1) / TX2, (a.nz + 4 * nr - 1) / (4 * nr), a.nshot);
 }
 template <typename... P, typename... A>
-cudaError_t launch_tile(void (*K)(P...), unsigned long long* opted, const BornArgs& a, size_t smem, cudaStream_t s,
-                        const A&... args)
+cudaError_t launch_tile(void (*K)(P...), unsigned long long* opted, const BornArgs& a, int nr, size_t smem,
+                        cudaStream_t s, const A&... args)
 {
     const cudaError_t e = smem > 48 * 1024 ? smem_opt_in(K, smem, opted) : cudaSuccess;
-    return e != cudaSuccess ? e : launch_pdl(K, tile_grid(a), 256, smem, s, args...);
+    return e != cudaSuccess ? e : launch_pdl(K, tile_grid(a, nr), 256, smem, s, args...);
 }
 
 template <int R, int NR>
@@ -683,68 +683,87 @@ template <int R, int NM, int NR, bool BORN>
 cudaError_t stress_r(const BornMaps& m, const BornArgs& a, int it, cudaStream_t s)
 {
     static unsigned long long opted = 0;
-    return launch_tile(k_born_stress<R, BORN, NM, NR>, &opted, a, xz_bytes<R, NR>(BORN ? 4 : 2), s, m, a, it);
+    return launch_tile(k_born_stress<R, BORN, NM, NR>, &opted, a, a.nr, xz_bytes<R, NR>(BORN ? 4 : 2), s, m, a, it);
 }
 template <int R, int NR, bool BORN, bool KEEP>
 cudaError_t velocity_r(const BornMaps& m, const BornArgs& a, int it, cudaStream_t s)
 {
     static unsigned long long opted = 0;
-    return launch_tile(k_born_velocity<R, BORN, KEEP, NR>, &opted, a, sig_bytes<R, NR>(BORN ? 2 : 1), s, m, a, it);
+    return launch_tile(k_born_velocity<R, BORN, KEEP, NR>, &opted, a, a.nrv, sig_bytes<R, NR>(BORN ? 2 : 1), s, m, a,
+                       it);
 }
-template <int R, int NM, int NR>
+template <int R, int NM, bool BORN>
+cudaError_t stress_nr(const BornMaps& m, const BornArgs& a, int it, cudaStream_t s)
+{
+    if constexpr (NM == 0)
+        if (a.nr == 4) return stress_r<R, NM, 4, BORN>(m, a, it, s);
+    return a.nr == 1 ? stress_r<R, NM, 1, BORN>(m, a, it, s) : stress_r<R, NM, 2, BORN>(m, a, it, s);
+}
+template <int R, bool BORN, bool KEEP>
+cudaError_t velocity_nr(const BornMaps& m, const BornArgs& a, int it, cudaStream_t s)
+{
+    return a.nrv == 1   ? velocity_r<R, 1, BORN, KEEP>(m, a, it, s)
+           : a.nrv == 2 ? velocity_r<R, 2, BORN, KEEP>(m, a, it, s)
+                        : velocity_r<R, 4, BORN, KEEP>(m, a, it, s);
+}
+template <int R, int NM>
 cudaError_t step_r(const BornMaps& m, const BornArgs& a, int it, bool born, bool keep, cudaStream_t s)
 {
-    cudaError_t e = born ? stress_r<R, NM, NR, true>(m, a, it, s) : stress_r<R, NM, NR, false>(m, a, it, s);
+    cudaError_t e = born ? stress_nr<R, NM, true>(m, a, it, s) : stress_nr<R, NM, false>(m, a, it, s);
     if (e != cudaSuccess) return e;
-    if (born) return velocity_r<R, NR, true, false>(m, a, it, s);
-    return keep ? velocity_r<R, NR, false, true>(m, a, it, s) : velocity_r<R, NR, false, false>(m, a, it, s);
+    if (born) return velocity_nr<R, true, false>(m, a, it, s);
+    return keep ? velocity_nr<R, false, true>(m, a, it, s) : velocity_nr<R, false, false>(m, a, it, s);
 }
 template <int R, int NM, int NR>
+cudaError_t vm_r(const BornMaps& m, const BornArgs& a, cudaStream_t s)
+{
+    static unsigned long long opted = 0;
+    return launch_tile(k_adj_vm<R, NM, NR>, &opted, a, a.nr, xz_bytes<R, NR>(5), s, m, a);
+}
+template <int R, int NR>
+cudaError_t str_r(const BornMaps& m, const BornArgs& a, int it, cudaStream_t s)
+{
+    static unsigned long long opted = 0;
+    return launch_tile(k_adj_str<R, NR>, &opted, a, a.nrv, sig_bytes<R, NR>(1), s, m, a, it - 1);
+}
+template <int R, int NM>
 cudaError_t adj_r(const BornMaps& m, const BornArgs& a, int it, cudaStream_t s)
 {
-    static unsigned long long opted = 0, opted2 = 0;
-    const cudaError_t e = launch_tile(k_adj_vm<R, NM, NR>, &opted, a, xz_bytes<R, NR>(5), s, m, a);
+    cudaError_t e;
+    if constexpr (NM == 0) {
+        e = a.nr == 4 ? vm_r<R, NM, 4>(m, a, s) : a.nr == 2 ? vm_r<R, NM, 2>(m, a, s) : vm_r<R, NM, 1>(m, a, s);
+    } else {
+        e = a.nr == 2 ? vm_r<R, NM, 2>(m, a, s) : vm_r<R, NM, 1>(m, a, s);
+    }
     if (e != cudaSuccess) return e;
-    return launch_tile(k_adj_str<R, NR>, &opted2, a, sig_bytes<R, NR>(1), s, m, a, it - 1);
-}
-template <int R, int NM>
-cudaError_t step_nr(const BornMaps& m, const BornArgs& a, int it, bool born, bool keep, cudaStream_t s)
-{
-    if constexpr (NM == 0)
-        if (a.nr == 4) return step_r<R, NM, 4>(m, a, it, born, keep, s);
-    return a.nr == 1 ? step_r<R, NM, 1>(m, a, it, born, keep, s) : step_r<R, NM, 2>(m, a, it, born, keep, s);
-}
-template <int R, int NM>
-cudaError_t adj_nr(const BornMaps& m, const BornArgs& a, int it, cudaStream_t s)
-{
-    if constexpr (NM == 0)
-        if (a.nr == 4) return adj_r<R, NM, 4>(m, a, it, s);
-    return a.nr == 1 ? adj_r<R, NM, 1>(m, a, it, s) : adj_r<R, NM, 2>(m, a, it, s);
+    return a.nrv == 4 ? str_r<R, 4>(m, a, it, s) : a.nrv == 2 ? str_r<R, 2>(m, a, it, s) : str_r<R, 1>(m, a, it, s);
 }
 template <int R>
 cudaError_t step_nm(const BornMaps& m, const BornArgs& a, int it, bool born, bool keep, cudaStream_t s)
 {
     switch (a.nm) {
-    case 0: return step_nr<R, 0>(m, a, it, born, keep, s);
-    case 1: return step_nr<R, 1>(m, a, it, born, keep, s);
-    case 2: return step_nr<R, 2>(m, a, it, born, keep, s);
-    default: return step_nr<R, 3>(m, a, it, born, keep, s);
+    case 0: return step_r<R, 0>(m, a, it, born, keep, s);
+    case 1: return step_r<R, 1>(m, a, it, born, keep, s);
+    case 2: return step_r<R, 2>(m, a, it, born, keep, s);
+    default: return step_r<R, 3>(m, a, it, born, keep, s);
     }
 }
 template <int R>
 cudaError_t adj_nm(const BornMaps& m, const BornArgs& a, int it, cudaStream_t s)
 {
     switch (a.nm) {
-    case 0: return adj_nr<R, 0>(m, a, it, s);
-    case 1: return adj_nr<R, 1>(m, a, it, s);
-    case 2: return adj_nr<R, 2>(m, a, it, s);
-    default: return adj_nr<R, 3>(m, a, it, s);
+    case 0: return adj_r<R, 0>(m, a, it, s);
+    case 1: return adj_r<R, 1>(m, a, it, s);
+    case 2: return adj_r<R, 2>(m, a, it, s);
+    default: return adj_r<R, 3>(m, a, it, s);
     }
 }
 }  // namespace
 
-// Rows per thread: as many (1, 2, or 4 without memory variables, which take up to 24
-// registers a row) as still give every SM a CTA.
+// Rows per thread of a kernel with nm mechanisms: as many (1, 2, or 4 without memory
+// variables, which take up to 24 registers a row) as still give every SM a CTA.  The
+// velocity and stress^T kernels have none in any medium (10 shots of 880 x 480, three
+// mechanisms: forward 22.4 -> 20.9 ms, adjoint 89 -> 84 ms with 4 rows there instead of 2).
 int born_rows(int nx, int nz, int nshot, int nm)
 {
     const long long cols = (nx + BXH + TX2 - 1) / TX2;

@@ -44,7 +44,7 @@ struct BornArgs {
     long long ss;
     const int* shot_tab;
     long long tstride;
-    int nr;                                // rows per thread of the step kernels (born_rows), as the maps' boxes
+    int nr, nrv;                           // rows per thread (born_rows): stress and velocity^T; velocity and stress^T
     // TMA types (BornMaps): v0x, v0z, sigma0 xx, zz, xz in a row from t_v0, the scattered
     // ones from t_v; ax, az from t_adj; Sxx, Szz, Sxz from t_s; the history slot's v0x,
     // v0z from t_hist
@@ -56,7 +56,8 @@ struct BornArgs {
 // 64 columns x 4 nr rows with halos in both directions (xz), in x only, in z only; the
 // history volumes and the shared B g1, both with xz boxes.
 struct BornMaps {
-    CUtensorMap xz, x, z, hist, bg1;
+    CUtensorMap xz, hist, bg1;   // boxes of the stress and velocity^T kernels (nr rows per thread)
+    CUtensorMap x, z, vxz;       // of the velocity and stress^T kernels (nrv)
 };
 
 int born_rows(int nx, int nz, int nshot, int nm);

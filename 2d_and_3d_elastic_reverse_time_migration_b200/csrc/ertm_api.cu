@@ -1708,17 +1708,19 @@ int born_group_maps(ertm_ctx* c, BornArgs& a, BornMaps& m, int G, int hist_slots
 {
     const auto& B = c->born;
     a.nr = born_rows(a.nx, a.nz, G, a.nm);
+    a.nrv = born_rows(a.nx, a.nz, G, 0);   // no memory variables in those
     a.t_v0 = PV_BG;
     a.t_v = PV_SC;
     a.t_adj = PV_ADJ;
     a.t_s = PV_S;
     a.t_hist = 0;
-    const int xw = TX2 + 2 * xb_of(a.R), tz = 4 * a.nr, zh = tz + 2 * a.R;
+    const int xw = TX2 + 2 * xb_of(a.R), zh = 4 * a.nr + 2 * a.R, tzv = 4 * a.nrv, zhv = tzv + 2 * a.R;
     std::memset(&m, 0, sizeof m);
     int rc;
     if ((rc = born_map(c, &m.xz, B.block, G, PV_N, xw, zh))) return rc;
-    if ((rc = born_map(c, &m.x, B.block, G, PV_N, xw, tz))) return rc;
-    if ((rc = born_map(c, &m.z, B.block, G, PV_N, TX2, zh))) return rc;
+    if ((rc = born_map(c, &m.x, B.block, G, PV_N, xw, tzv))) return rc;
+    if ((rc = born_map(c, &m.z, B.block, G, PV_N, TX2, zhv))) return rc;
+    if ((rc = born_map(c, &m.vxz, B.block, G, PV_N, xw, zhv))) return rc;
     if (!hist_slots) return ERTM_OK;
     if ((rc = born_map(c, &m.hist, B.hist, G, 4 * hist_slots, xw, zh))) return rc;
     return born_map(c, &m.bg1, B.sv[SV_BG1], 1, 1, xw, zh);
