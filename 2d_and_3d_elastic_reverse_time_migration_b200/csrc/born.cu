@@ -43,7 +43,7 @@
 // Measured on B200, ms per call before -> now: Born forward, 10 shots of 880 x 480, three
 // mechanisms, 100 steps 34.4 -> 20.9 (5.34 TB/s of the 264 B per shot-cell and step that
 // the pair of kernels cannot do without); adjoint, 8 shots of 592 x 336, elastic, 240
-// steps 37.5 -> 21.2, before its last segment's rebuild went.
+// steps 37.5 -> 21.2, and 16.7 with two segments less to rebuild.
 //
 // Tiles start at allocated columns 64 b (cell 64 b - BXH): every row access is whole
 // 128-byte lines.  Lanes on the zero halo columns load and compute and store nothing.

@@ -51,6 +51,9 @@ struct ertm_ctx {
     int device = 0;
     cudaStream_t own_stream = nullptr;
     cudaStream_t stream = nullptr;
+    // second stream of the Born adjoint and the events that order it with `stream` (first use)
+    cudaStream_t side = nullptr;
+    cudaEvent_t side_ev[2] = {nullptr, nullptr};
     float coef[8] = {0};
 
     float* f_base[NFIELD] = {nullptr};
@@ -121,7 +124,7 @@ struct ertm_ctx {
         int G = 0;
         float* ckpt = nullptr;            // checkpoints: nck x 14 types x G shots
         long long ckpt_floats = 0;
-        float* hist = nullptr;            // history: K x 4 types x G shots
+        float* hist = nullptr;            // history: K (or 2 K) x 4 types x G shots
         long long hist_floats = 0;
         int* tab = nullptr;               // shot table, G x 8 ints (device)
         int tab_cap = 0;
@@ -898,6 +901,9 @@ int ertm_destroy(ertm_ctx* c)
     cudaFree(c->born.hist);
     cudaFree(c->born.tab);
     cudaFree(c->born.wav);
+    if (c->side) cudaStreamDestroy(c->side);
+    for (cudaEvent_t e : c->side_ev)
+        if (e) cudaEventDestroy(e);
     if (c->own_stream) cudaStreamDestroy(c->own_stream);
     delete c;
     return ERTM_OK;
@@ -1744,6 +1750,14 @@ int born_stage_in(ertm_ctx* c, const float* const* src, int count, const float**
     return ERTM_OK;
 }
 
+int born_side_stream(ertm_ctx* c)
+{
+    if (!c->side) CK(c, cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking));
+    for (cudaEvent_t& e : c->side_ev)
+        if (!e) CK(c, cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    return ERTM_OK;
+}
+
 // Shots per launch: at most `want`, bounded so that the group's volumes (and, for the
 // adjoint, its checkpoints and history) take at most about 60 % of the free memory.
 int born_group_size(ertm_ctx* c, int want, long long floats_per_shot)
@@ -1836,9 +1850,19 @@ int ertm_born_adjoint_shots(ertm_ctx* c, const ertm_shot* shots, int nshots, con
     const long long nd = 3LL * nt * shots[0].nrx;
     const bool dev_res = is_device_ptr(residual);
     const long long per_shot = B.n * ((long long)PV_N + 14LL * (nck - 1) + 4LL * K) + (dev_res ? 0 : nd);
-    const int G = born_group_size(c, nshots, per_shot);
+    // With room for two segments' histories of all shots, the last two segments are recorded as
+    // they are made, and an earlier one is rebuilt on a second stream while the one after it is
+    // reversed: neither chain of short kernels fills the GPU (240 steps in segments of 80: 6 shots
+    // of 168 x 104 4.08 -> 3.34 ms, of 300 x 200 6.63 -> 5.37, 10 of 880 x 480 53.9 -> 47.4).  Kernels
+    // shorter than their launches lose by the second stream (one shot of 168 x 104, one segment
+    // recorded at once: 3.29 ms without, 3.64 with it), so at least 100,000 cells.
+    const bool two = nck > 1 && born_group_size(c, nshots, per_shot + 4LL * K * B.n) >= nshots;
+    const bool side = two && nck > 2 && (long long)nshots * c->g.nx * c->g.nz >= 100000;
+    const int G = two ? nshots : born_group_size(c, nshots, per_shot);
+    if (side && (rc = born_side_stream(c))) return rc;
+    const int slots = two ? 2 * K : K;
     if ((rc = born_group_volumes(c, G))) return rc;
-    const long long ck_need = 14LL * (nck - 1) * G * B.n, hist_need = 4LL * K * G * B.n;
+    const long long ck_need = 14LL * (nck - 1) * G * B.n, hist_need = 4LL * slots * G * B.n;
     if (B.ckpt_floats < ck_need) {
         cudaFree(B.ckpt);
         B.ckpt = nullptr;
@@ -1867,7 +1891,7 @@ int ertm_born_adjoint_shots(ertm_ctx* c, const ertm_shot* shots, int nshots, con
         born_group_args(c, a, g);
         if ((rc = born_group_shots(c, a, shots + s0, g))) return rc;
         BornMaps maps;
-        if ((rc = born_group_maps(c, a, maps, g, K))) return rc;
+        if ((rc = born_group_maps(c, a, maps, g, slots))) return rc;
         a.tstride = nd;
         if (dev_res) a.traces = const_cast<float*>(residual) + (size_t)s0 * nd;
         else {
@@ -1883,54 +1907,69 @@ int ertm_born_adjoint_shots(ertm_ctx* c, const ertm_shot* shots, int nshots, con
             return cudaMemcpyAsync(B.ckpt + seg * ck_seg, B.pv[PV_BG], sizeof(float) * ck_seg,
                                    cudaMemcpyDeviceToDevice, c->stream);
         };
-        auto load = [&](int seg) {
+        auto load = [&](int seg, cudaStream_t st) {
             return cudaMemcpyAsync(B.pv[PV_BG], B.ckpt + seg * ck_seg, sizeof(float) * ck_seg,
-                                   cudaMemcpyDeviceToDevice, c->stream);
+                                   cudaMemcpyDeviceToDevice, st);
         };
-        // The segments end at nt, nt - K, ...: the last one is a full one, and its steps, which
+        // The segments end at nt, nt - K, ...: the last ones are full ones, and their steps, which
         // the reverse sweep needs first, record their history as they are made.  Only the
-        // earlier ones are made twice, once for the checkpoints and once for the history
-        // (592 x 336, 8 shots, 240 steps in segments of 100: 18.9 ms, 21.3 with every segment made
-        // twice).
+        // segments before `made` are made twice, once for the checkpoints and once for the history
+        // (592 x 336, 8 shots, 240 steps in segments of 100: 21.3 ms with every segment made twice,
+        // 18.9 with the last one recorded at once, 16.7 with the last two).
+        const int made = nck - (two ? 2 : 1);
         auto seg_begin = [&](int seg) { return std::max(0, nt - (nck - seg) * K); };
         auto seg_end = [&](int seg) { return nt - (nck - 1 - seg) * K; };
-        auto record = [&](int seg) {
-            const int t0 = seg_begin(seg);
-            for (int it = t0; it < seg_end(seg); it++) {
-                float* h = B.hist + (size_t)(it - t0) * 4 * g * B.n;
-                a.kv0x = h;
-                a.kv0z = h + g * B.n;
-                a.ka0x = h + 2 * g * B.n;
-                a.ka0z = h + 3 * g * B.n;
-                const cudaError_t e = born_launch_step(maps, a, it, false, true, c->stream);
-                if (e != cudaSuccess) return e;
-            }
-            return cudaSuccess;
+        auto slot = [&](int seg, int it) { return (two && (nck - 1 - seg) % 2 ? K : 0) + it - seg_begin(seg); };
+        auto record = [&](int seg, int it, cudaStream_t st) {
+            float* h = B.hist + (size_t)slot(seg, it) * 4 * g * B.n;
+            a.kv0x = h;
+            a.kv0z = h + g * B.n;
+            a.ka0x = h + 2 * g * B.n;
+            a.ka0z = h + 3 * g * B.n;
+            return born_launch_step(maps, a, it, false, true, st);
         };
-        for (int sg = 0; sg < nck - 1; sg++) {
+        for (int sg = 0; sg < made; sg++) {
             CK(c, save(sg));
             for (int it = seg_begin(sg); it < seg_end(sg); it++)
                 CK(c, born_launch_step(maps, a, it, false, false, c->stream));
         }
-        CK(c, record(nck - 1));
+        for (int sg = made; sg < nck; sg++)
+            for (int it = seg_begin(sg); it < seg_end(sg); it++) CK(c, record(sg, it, c->stream));
         // 2. reverse sweep, one checkpoint segment at a time
         if ((rc = born_zero_types(c, PV_ADJ, PV_N - PV_ADJ, g))) return rc;   // adjoint, gradients, scratch
         CK(c, born_launch_inject(a, nt - 1, c->stream));
         for (int sg = nck - 1; sg >= 0; sg--) {
             const int t0 = seg_begin(sg), t1 = seg_end(sg);
-            if (sg < nck - 1) {
-                CK(c, load(sg));
-                CK(c, record(sg));
+            if (!side && sg < made) {
+                CK(c, load(sg, c->stream));
+                for (int it = t0; it < t1; it++) CK(c, record(sg, it, c->stream));
             }
-            for (int it = t1 - 1; it >= t0; it--) {
-                const float* h = B.hist + (size_t)(it - t0) * 4 * g * B.n;
-                a.ha0x = h + 2 * g * B.n;
-                a.ha0z = h + 3 * g * B.n;
-                a.t_hist = 4 * (it - t0);
-                CK(c, born_launch_adjoint_step(maps, a, it, c->stream));
+            // the earlier segment's steps, launched in turn with this one's; its half of the
+            // history was read by the segment reversed before this one
+            const bool next = side && sg > 0 && sg - 1 < made;
+            const int p0 = next ? seg_begin(sg - 1) : 0, p1 = next ? seg_end(sg - 1) : 0;
+            if (next) {
+                CK(c, cudaEventRecord(c->side_ev[0], c->stream));
+                CK(c, cudaStreamWaitEvent(c->side, c->side_ev[0], 0));
+                CK(c, load(sg - 1, c->side));
+            }
+            for (int q = 0; q < std::max(t1 - t0, p1 - p0); q++) {
+                if (q < p1 - p0) CK(c, record(sg - 1, p0 + q, c->side));
+                if (q < t1 - t0) {
+                    const int it = t1 - 1 - q;
+                    const float* h = B.hist + (size_t)slot(sg, it) * 4 * g * B.n;
+                    a.ha0x = h + 2 * g * B.n;
+                    a.ha0z = h + 3 * g * B.n;
+                    a.t_hist = 4 * slot(sg, it);
+                    CK(c, born_launch_adjoint_step(maps, a, it, c->stream));
+                }
+            }
+            if (next) {
+                CK(c, cudaEventRecord(c->side_ev[1], c->side));
+                CK(c, cudaStreamWaitEvent(c->stream, c->side_ev[1], 0));
             }
         }
-        c->launches += 2LL * (2 * nt - K) + 2LL * nt + 1;
+        c->launches += 2LL * (nt + (made > 0 ? seg_end(made - 1) : 0)) + 2LL * nt + 1;
         // 3. gradients w.r.t. the relative perturbations, summed over the group's shots
         CK(c, born_launch_final(a, tgt[0], tgt[1], tgt[2], s0 > 0, c->stream));
         c->launches++;

@@ -93,7 +93,8 @@ typedef struct {
     float pml_vmax;          /* CPML velocity; 0 -> max Vp of the model */
     float sponge_coef;       /* reference coe_attenuation (sponge kinds) */
     int   device;            /* CUDA device ordinal */
-    int   checkpoint_every;  /* Born adjoint: background checkpoint interval; 0 -> 200 */
+    int   checkpoint_every;  /* Born adjoint: background checkpoint interval; 0 -> 200.  The
+                              * history of two intervals is held where memory allows, of one else */
     int   autotune;          /* 1: time the z-chunk candidates of the step kernels once per
                                 grid shape (cached for the process); 0: fixed rule */
     int   visco_nmech;       /* Born operators: GSLS relaxation mechanisms, 0 (elastic) .. 3 */
