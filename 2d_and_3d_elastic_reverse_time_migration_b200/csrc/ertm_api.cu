@@ -602,13 +602,38 @@ int autotune_kchunk(ertm_ctx* c, int which, int* out)
     return ERTM_OK;
 }
 
+int zero_arrays(ertm_ctx* c, const ZeroList& z, cudaStream_t st)
+{
+    CK(c, launch_zero(z, st));
+    c->launches++;
+    return ERTM_OK;
+}
+
 int reset_state(ertm_ctx* c)
 {
-    for (int q = 0; q < NFIELD; q++)
-        if (c->f_base[q]) CK(c, cudaMemsetAsync(c->f_base[q], 0, sizeof(float) * c->g.total, c->stream));
-    for (int p = 0; p < NPSI; p++)
-        if (c->psi[p]) CK(c, cudaMemsetAsync(c->psi[p], 0, sizeof(float) * c->psi_n[p], c->stream));
-    return ERTM_OK;
+    ZeroList z;
+    for (int q = 0; q < NFIELD; q++) z.add(c->f_base[q], c->g.total);
+    for (int p = 0; p < NPSI; p++) z.add(c->psi[p], c->psi_n[p]);
+    return zero_arrays(c, z, c->stream);
+}
+
+int zero_excitation(ertm_ctx* c, cudaStream_t st)
+{
+    ZeroList z;
+    z.add(c->ex_amp2_base, c->g.total);
+    z.add(c->ex_time_base, c->g.total);
+    for (int q = 0; q < 3; q++) z.add(c->ex_v_base[q], c->g.total);
+    z.add(c->ex_tp_base, c->g.total);
+    if (c->angles) z.add(c->ang_base[0], c->g.total);
+    return zero_arrays(c, z, st);
+}
+
+int zero_images(ertm_ctx* c, cudaStream_t st)
+{
+    ZeroList z;
+    for (int q = 0; q < 3; q++) z.add(c->img_base[q], c->g.total);
+    if (c->angles) z.add(c->ang_base[1], c->g.total);
+    return zero_arrays(c, z, st);
 }
 
 int upload_wavelet(ertm_ctx* c, const ertm_shot* s)
@@ -637,19 +662,20 @@ struct Range {
 // for the step index *c->it_d + add.  nsteps steps run in direction `dir`, as a CUDA
 // graph of kGraphSteps steps replayed back to back (the base index lives in device
 // memory and moves once per replay, so one graph serves every chunk and no step
-// carries a counter launch); the first step and the remainder are launched directly.
+// carries a counter launch); the first steps and the remainder are launched directly.
 // A short graph: building one costs about 6 us per launch in it (measured 400 us for 32
 // steps of a 2D pass, against 0.6 us that a replayed step saves over a direct launch),
-// while a replay of 8 steps already hides its own launch.  Long passes amortise 32.
+// while a replay of 8 steps already hides its own launch.  Long passes amortise 32.  Two
+// graphs' worth of steps go first, so that the GPU has work while the host builds the graph
+// (a pass of 680 x 380 costs 133 us besides its steps; 196 with one step first and its state
+// zeroed array by array).
 template <typename F>
 int time_loop(ertm_ctx* c, int nsteps, int dir, F&& one_step)
 {
     const int kGraphSteps = nsteps >= 1500 ? 32 : 8;
+    const int lead = nsteps >= 4 * kGraphSteps ? 2 * kGraphSteps : 1;
     int done = 0;
-    if (nsteps > 0) {
-        CK(c, one_step(0));
-        done = 1;
-    }
+    for (; done < std::min(nsteps, lead); done++) CK(c, one_step(dir * done));
     int base = 0;                    // steps that the device's index has moved
     if (nsteps - done >= 2 * kGraphSteps) {
         CK(c, launch_advance(c->it_d, dir * done, c->stream));
@@ -1062,12 +1088,7 @@ int ertm_forward_together_using_smoothed_model(ertm_ctx* c, const ertm_shot* s)
     if (rc) return rc;
     if ((rc = ensure_excitation(c))) return rc;
     const Geom& g = c->g;
-    CK(c, cudaMemsetAsync(c->ex_amp2_base, 0, sizeof(float) * g.total, c->stream));
-    CK(c, cudaMemsetAsync(c->ex_time_base, 0, sizeof(int) * g.total, c->stream));
-    for (int q = 0; q < 3; q++)
-        if (c->ex_v_base[q]) CK(c, cudaMemsetAsync(c->ex_v_base[q], 0, sizeof(float) * g.total, c->stream));
-    CK(c, cudaMemsetAsync(c->ex_tp_base, 0, sizeof(float) * g.total, c->stream));
-    if (c->angles) CK(c, cudaMemsetAsync(c->ang_base[0], 0, sizeof(float) * g.total, c->stream));
+    if ((rc = zero_excitation(c, c->stream))) return rc;
     int nsrc = c->cfg.src_steps > 0 ? c->cfg.src_steps : 2 * c->cfg.nt / 3;
     c->have_excitation = false;
     c->have_src_angle = false;
@@ -1089,9 +1110,8 @@ int ertm_backward_together_using_smoothed_model(ertm_ctx* c, const ertm_shot* s,
     if (!data_in && nrec_of(s) > 0) return fail(c, ERTM_EINVAL, "data_in is NULL");
     if ((rc = ensure_images(c))) return rc;
     const Geom& g = c->g;
-    for (int q = 0; q < 3; q++) CK(c, cudaMemsetAsync(c->img_base[q], 0, sizeof(float) * g.total, c->stream));
+    if ((rc = zero_images(c, c->stream))) return rc;
     c->have_rcv_angle = false;
-    if (c->angles) CK(c, cudaMemsetAsync(c->ang_base[1], 0, sizeof(float) * g.total, c->stream));
     const long long nrec = nrec_of(s);
     const size_t nd = 3 * (size_t)c->cfg.nt * nrec;
     float* traces = nullptr;
@@ -1260,11 +1280,7 @@ int ertm_rtm_multi(ertm_ctx* const* ctx, int n, const ertm_shot* shots, const fl
         ertm_ctx* c = ctx[q];
         const Geom& g = c->g;
         if ((rc = ensure_excitation(c))) return rc;
-        CK(c0, cudaMemsetAsync(c->ex_amp2_base, 0, sizeof(float) * g.total, st));
-        CK(c0, cudaMemsetAsync(c->ex_time_base, 0, sizeof(int) * g.total, st));
-        for (int k = 0; k < 3; k++)
-            if (c->ex_v_base[k]) CK(c0, cudaMemsetAsync(c->ex_v_base[k], 0, sizeof(float) * g.total, st));
-        CK(c0, cudaMemsetAsync(c->ex_tp_base, 0, sizeof(float) * g.total, st));
+        if ((rc = zero_excitation(c, st))) return rc;
         c->have_excitation = false;
         const float vmax = c->cfg.pml_vmax > 0 ? c->cfg.pml_vmax : c->vpmax[1];
         if ((rc = upload_profiles(c, vmax))) return rc;
@@ -1287,7 +1303,7 @@ int ertm_rtm_multi(ertm_ctx* const* ctx, int n, const ertm_shot* shots, const fl
         ertm_ctx* c = ctx[q];
         const Geom& g = c->g;
         if ((rc = ensure_images(c))) return rc;
-        for (int k = 0; k < 3; k++) CK(c0, cudaMemsetAsync(c->img_base[k], 0, sizeof(float) * g.total, st));
+        if ((rc = zero_images(c, st))) return rc;
         const long long nrec = nrec_of(&shots[q]);
         const size_t nd = 3 * (size_t)c->cfg.nt * nrec;
         float* traces = nullptr;

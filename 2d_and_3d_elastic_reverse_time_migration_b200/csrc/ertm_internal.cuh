@@ -228,6 +228,20 @@ cudaError_t launch_inject(const KArgs& a, int it, cudaStream_t s);
 cudaError_t launch_advance(int* it_ptr, int delta, cudaStream_t s);
 cudaError_t launch_set_int(int* p, int v, cudaStream_t s);
 cudaError_t launch_sqrt_gather(const Geom& g, const float* amp2, float* out, cudaStream_t s);
+// arrays of 32-bit words zeroed by one launch
+constexpr int ZERO_MAX = 64;
+struct ZeroList {
+    float* p[ZERO_MAX];
+    long long n[ZERO_MAX];
+    int count = 0;
+    void add(void* q, long long words)   // NULL: nothing
+    {
+        if (!q || words < 1) return;
+        p[count] = (float*)q;
+        n[count++] = words;
+    }
+};
+cudaError_t launch_zero(const ZeroList& z, cudaStream_t s);
 cudaError_t launch_axpy(long long n, const float* x, float* y, cudaStream_t s);   // y += x
 // 2D propagation angle at the cells whose excitation step it is; window (2 hw + 1)^2:
 // hw = 2 in the source pass, 4 in the receiver pass

@@ -462,26 +462,6 @@ __global__ void k_f32_to_bf16(const float* a, bf16* b, long long n)
         b[q] = __float2bfloat16(a[q]);
 }
 
-// Zeroes the arrays of `z`, one per blockIdx.y: the 36 gradient arrays of a network (4 KB to
-// 590 KB) in one launch of about 4 us instead of 36 fills.
-constexpr int ZMAX = 64;
-struct ZeroList {
-    float* p[ZMAX];
-    long long n[ZMAX];
-};
-__global__ void k_zero(const __grid_constant__ ZeroList z)
-{
-    float* p = z.p[blockIdx.y];
-    const long long n = z.n[blockIdx.y], t = blockIdx.x * (long long)blockDim.x + threadIdx.x,
-                    nt = (long long)gridDim.x * blockDim.x;
-    long long head = 0;
-    if (((uintptr_t)p & 15) == 0) {
-        head = n & ~3LL;
-        for (long long q = t; q < n / 4; q += nt) reinterpret_cast<float4*>(p)[q] = make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-    for (long long q = head + t; q < n; q += nt) p[q] = 0.f;
-}
-
 // c FP32 values per pixel -> 8 BF16 channels, zero in the padding: one 16-byte store per pixel
 __global__ void __launch_bounds__(256) k_pack8(const float* __restrict__ x, uint4* __restrict__ y, int c, long long n)
 {
@@ -623,18 +603,13 @@ int ertm_nn_run(const ertm_nn_op* ops, int nops, void* const* ptr, int nptr, int
         case ERTM_NN_OP_POOL: rc = ertm_nn_pool2(&o.a, p[0], stream); break;
         case ERTM_NN_OP_POOL_BWD: rc = ertm_nn_pool2_bwd(&o.a, p[0], &o.b, o.flag, stream); break;
         case ERTM_NN_OP_ZERO: {
-            ZeroList z;
-            long long most = 0;
-            for (used = 0; i + used < nops && used < ZMAX && ops[i + used].kind == ERTM_NN_OP_ZERO; used++) {
+            ertm::ZeroList z;
+            for (used = 0; i + used < nops && used < ertm::ZERO_MAX && ops[i + used].kind == ERTM_NN_OP_ZERO; used++) {
                 const ertm_nn_op& f = ops[i + used];
                 if (f.n < 1 || f.p[0] < 0 || f.p[0] >= nptr || !ptr[f.p[0]]) return ERTM_EINVAL;
-                z.p[used] = (float*)ptr[f.p[0]];
-                z.n[used] = f.n;
-                most = std::max(most, f.n);
+                z.add(ptr[f.p[0]], f.n);
             }
-            const dim3 grid((unsigned)std::min((most / 4 + 255) / 256 + 1, 148LL), used);
-            k_zero<<<grid, 256, 0, (cudaStream_t)stream>>>(z);
-            rc = rc_of(cudaGetLastError());
+            rc = rc_of(ertm::launch_zero(z, (cudaStream_t)stream));
             break;
         }
         case ERTM_NN_OP_PACK: {

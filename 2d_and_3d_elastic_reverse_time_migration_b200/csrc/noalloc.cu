@@ -267,11 +267,12 @@ int run_noalloc(const ertm_config* cfg, const float* vp, const float* vs, const 
     float* wav = cv.take<float>(s->nw > 0 ? s->nw : 1);
 
     // clear what must start at zero: halos and state of every volume, memory variables
-    for (int q = 0; q < nf; q++) NCK(cudaMemsetAsync(fbase[fl[q]], 0, 4 * g.total, st));
-    for (int q = 0; q < 3; q++) NCK(cudaMemsetAsync(mbase[q], 0, 4 * g.total, st));
-    for (int p = 0; p < NPSI; p++)
-        if (psi[p]) NCK(cudaMemsetAsync(psi[p], 0, 4 * psi_n[p], st));
-    NCK(cudaMemsetAsync(counters, 0, 16 * sizeof(int), st));
+    ZeroList z;
+    for (int q = 0; q < nf; q++) z.add(fbase[fl[q]], g.total);
+    for (int q = 0; q < 3; q++) z.add(mbase[q], g.total);
+    for (int p = 0; p < NPSI; p++) z.add(psi[p], psi_n[p]);
+    z.add(counters, 16);
+    NCK(launch_zero(z, st));
     if (s->nw > 0) NCK(cudaMemcpyAsync(wav, s->wavelet, 4 * (size_t)s->nw, cudaMemcpyDeviceToDevice, st));
 
     // model products rho vp^2, rho vs^2, 1/rho into the padded layout
