@@ -41,9 +41,10 @@
 // fill its wait, so a grid in L2 costs little more than the launch and a large group
 // streams.  Before, each warp marched down 8-32 rows with one round trip per row.
 // Measured on B200, ms per call before -> now: Born forward, 10 shots of 880 x 480, three
-// mechanisms, 100 steps 34.4 -> 20.9 (5.34 TB/s of the 264 B per shot-cell and step that
+// mechanisms, 100 steps 34.4 -> 20.8 (5.36 TB/s of the 264 B per shot-cell and step that
 // the pair of kernels cannot do without); adjoint, 8 shots of 592 x 336, elastic, 240
-// steps 37.5 -> 21.2, and 16.7 with two segments less to rebuild.
+// steps 37.5 -> 21.2, and 16.6 with two segments less to rebuild; two CG iterations on 6
+// shots of 168 x 104 54.8 -> 11.7 (12.7 before the own values were loaded ahead of the wait).
 //
 // Tiles start at allocated columns 64 b (cell 64 b - BXH): every row access is whole
 // 128-byte lines.  Lanes on the zero halo columns load and compute and store nothing.
@@ -174,6 +175,7 @@ __global__ void __launch_bounds__(256, 2) k_born_stress(const __grid_constant__ 
     __shared__ uint64_t bar;
     const Place<R, NR> S(a);
     tile2_begin(&bar);
+    tile2_go(true);
     if (threadIdx.x == 0) {
         const int gx = S.ax - T::XB, sh = blockIdx.z;
         mbar_expect_tx(&bar, 4u * (BORN ? 4 : 2) * T::XZ);
@@ -196,12 +198,12 @@ __global__ void __launch_bounds__(256, 2) k_born_stress(const __grid_constant__ 
         const int c = S.c + r * px;
 #pragma unroll
         for (int q = 0; q < 3; q++) {
-            o[q][r] = s0[q][c];
-            if (BORN) so[q][r] = sc[q][c];
+            o[q][r] = __ldcg(&s0[q][c]);
+            if (BORN) so[q][r] = __ldcg(&sc[q][c]);
 #pragma unroll
             for (int l = 0; l < NM; l++) {
-                r0v[q][l][r] = a.r0[q * 3 + l][S.zo + c];
-                if (BORN) rv[q][l][r] = a.r[q * 3 + l][S.zo + c];
+                r0v[q][l][r] = __ldcg(&a.r0[q * 3 + l][S.zo + c]);
+                if (BORN) rv[q][l][r] = __ldcg(&a.r[q * 3 + l][S.zo + c]);
             }
         }
         g1[r] = __ldg(a.g1 + c);
@@ -216,6 +218,7 @@ __global__ void __launch_bounds__(256, 2) k_born_stress(const __grid_constant__ 
     const bool src_step = it >= 0 && it < a.nw;
     const bool src_col = src_step && S.i == shot_par(a, 0);
     const int srcz = shot_par(a, 1);
+    tile2_go(false);
     if (!tile2_wait(&bar, kWaitPolls, a.err, false)) return;
     if (!S.act || S.r0 >= a.nz) return;
     const float* v0x = sm + S.xz();
@@ -294,6 +297,7 @@ __global__ void __launch_bounds__(256, 2) k_born_velocity(const __grid_constant_
     __shared__ uint64_t bar;
     const Place<R, NR> S(a);
     tile2_begin(&bar);
+    tile2_go(true);
     if (threadIdx.x == 0) {
         const int gx = S.ax - T::XB, sh = blockIdx.z;
         mbar_expect_tx(&bar, 4u * (BORN ? 2 : 1) * (T::X + T::Z + T::XZ));
@@ -316,18 +320,19 @@ __global__ void __launch_bounds__(256, 2) k_born_velocity(const __grid_constant_
     for (int r = 0; r < NR; r++) {
         if (!S.act || S.r0 + r >= a.nz) continue;
         const int c = S.c + r * px;
-        ov0x[r] = v0x[c];
-        ov0z[r] = v0z[c];
+        ov0x[r] = __ldcg(&v0x[c]);
+        ov0z[r] = __ldcg(&v0z[c]);
         b[r] = __ldg(a.B + c);
         g1[r] = __ldg(a.g1 + c);
         g2[r] = __ldg(a.g2 + c);
         if (BORN) {
-            ovx[r] = vx[c];
-            ovz[r] = vz[c];
+            ovx[r] = __ldcg(&vx[c]);
+            ovz[r] = __ldcg(&vz[c]);
             rr[r] = __ldg(a.rr + c);
         }
     }
     const int rz = BORN && a.traces ? shot_par(a, 5) : -1;
+    tile2_go(false);
     if (!tile2_wait(&bar, kWaitPolls, a.err, false)) return;
     if (!S.act || S.r0 >= a.nz) return;
     // sigma_xz: backward z difference; sigma_zz: forward
@@ -414,6 +419,7 @@ __global__ void __launch_bounds__(256, 2) k_adj_vm(const __grid_constant__ BornM
     __shared__ uint64_t bar;
     const Place<R, NR> S(a);
     tile2_begin(&bar);
+    tile2_go(true);
     if (threadIdx.x == 0) {
         const int gx = S.ax - T::XB, sh = blockIdx.z;
         mbar_expect_tx(&bar, 4u * 5 * T::XZ);
@@ -436,19 +442,25 @@ __global__ void __launch_bounds__(256, 2) k_adj_vm(const __grid_constant__ BornM
         const long long cz = S.zo + c;
 #pragma unroll
         for (int q = 0; q < 3; q++) {
-            hv[q][r] = h[q][c];
+            hv[q][r] = __ldcg(&h[q][c]);
 #pragma unroll
-            for (int l = 0; l < NM; l++) lv[q][l][r] = a.lr[q * 3 + l][cz];
+            for (int l = 0; l < NM; l++) lv[q][l][r] = __ldcg(&a.lr[q * 3 + l][cz]);
         }
-        gM[r] = a.gM[cz];
-        gU[r] = a.gU[cz];
-        gR[r] = a.gR[cz];
-        h0x[r] = a.ha0x[cz];
-        h0z[r] = a.ha0z[cz];
+        gM[r] = __ldcg(&a.gM[cz]);
+        gU[r] = __ldcg(&a.gU[cz]);
+        gR[r] = __ldcg(&a.gR[cz]);
         g1[r] = __ldg(a.g1 + c);
         g2[r] = __ldg(a.g2 + c);
         pi[r] = __ldg(a.M + c);
         mu[r] = __ldg(a.U + c);
+    }
+    tile2_go(false);
+    // the history may be the last launch's
+#pragma unroll
+    for (int r = 0; r < NR; r++) {
+        if (!S.act || S.r0 + r >= a.nz) continue;
+        h0x[r] = a.ha0x[S.zo + S.c + r * px];
+        h0z[r] = a.ha0z[S.zo + S.c + r * px];
     }
     const bool landed = tile2_wait(&bar, kWaitPolls, a.err, false);
     float* fx = sm + S.xz();
@@ -525,6 +537,7 @@ __global__ void __launch_bounds__(256, 2) k_adj_str(const __grid_constant__ Born
     __shared__ uint64_t bar;
     const Place<R, NR> S(a);
     tile2_begin(&bar);
+    tile2_go(true);
     if (threadIdx.x == 0) {
         const int gx = S.ax - T::XB, sh = blockIdx.z;
         mbar_expect_tx(&bar, 4u * (T::X + T::Z + T::XZ));
@@ -540,11 +553,12 @@ __global__ void __launch_bounds__(256, 2) k_adj_str(const __grid_constant__ Born
     for (int r = 0; r < NR; r++) {
         if (!S.act || S.r0 + r >= a.nz) continue;
         const int c = S.c + r * px;
-        ox[r] = ax[c];
-        oz[r] = az[c];
+        ox[r] = __ldcg(&ax[c]);
+        oz[r] = __ldcg(&az[c]);
         g12[r] = __ldg(a.g2 + c) * __ldg(a.g1 + c);
     }
     const int rz = it_next >= 0 ? shot_par(a, 5) : -1;
+    tile2_go(false);
     if (!tile2_wait(&bar, kWaitPolls, a.err, false)) return;
     if (!S.act || S.r0 >= a.nz) return;
     const float* sxx = sm + S.x();

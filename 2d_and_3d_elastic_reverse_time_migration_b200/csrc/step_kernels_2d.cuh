@@ -13,10 +13,11 @@
 // waits (griddepcontrol.wait) before it touches memory.
 //
 // Measured on B200 against the z-marching kernels that 2D grids shared with 3D (one
-// 32-cell row per CTA and TMA round trip) and their separate step-counter launch:
-// us per step, modelling 168 x 104 21.4 -> 5.5, RTM 680 x 380 25.6 -> 8.4, modelling
-// 1471 x 803 (R = 6) 47 -> 22; RTM 4096 x 2048 438 -> 180, where the step streams from
-// HBM (8.4 M cells x 108 B in 154 us without the P/S split: 5.9 TB/s).
+// 32-cell row per CTA and TMA round trip) and their separate step-counter launch, ms per
+// call: modelling 168 x 104, 240 steps 4.98 -> 1.11; RTM 680 x 380, 400 steps 10.07 -> 3.38;
+// modelling 1471 x 803 (R = 6), 90 steps 4.24 -> 2.03.  RTM 4096 x 2048 438 -> 180 us per
+// step, where the step streams from HBM (8.4 M cells x 108 B in 154 us without the P/S
+// split: 5.9 TB/s).
 //
 // The arithmetic per cell is that of the 3D kernels without the y terms.
 #pragma once
@@ -35,8 +36,14 @@ struct Tile2 {
     static constexpr int XZ = XW * ZH, X = XW * TZ, Z = TX2 * ZH;
 };
 
-// Shared by both kernels: barrier set-up before, and memory access after, the wait for
-// the previous launch.
+// Shared by the tile kernels.  Launches alternate between two kernels, each of which writes
+// what it alone loads cell by cell and the other stages: a thread's own values were last
+// written two launches ago.  That launch had completed when the previous one passed its
+// wait, and only then does that one let this one start.  So the staging warp waits and
+// issues the copies first, while the others load their own values, past L1, before they
+// wait.  Of it: us per step, modelling 168 x 104 4.36 -> 3.93, 680 x 380 8.20 -> 6.74;
+// modelling 1471 x 803 2.10 -> 2.03 ms.  (Every warp loading before the wait: 3.81, 6.74, but
+// 2.19 ms: in launches of several waves the copies are issued late.)
 __device__ __forceinline__ void tile2_begin(uint64_t* bar)
 {
     if (threadIdx.x == 0) {
@@ -44,6 +51,11 @@ __device__ __forceinline__ void tile2_begin(uint64_t* bar)
         mbar_fence_init();
     }
     __syncthreads();
+}
+// `first`: the staging warp (0), which waits before anything else; the others, after their loads
+__device__ __forceinline__ void tile2_go(bool first)
+{
+    if ((threadIdx.x < 32) != first) return;
     pdl_wait();
     pdl_launch();
 }
@@ -84,6 +96,7 @@ __global__ void __launch_bounds__(256, 2) k_stress2d(const __grid_constant__ Str
     const int sz = (int)a.sz;
     const bool skip = tile2_skip<T::TZ>(a);
     tile2_begin(&bar);
+    tile2_go(true);
     if (threadIdx.x == 0 && !skip) {
         const int gx = (int)blockIdx.x * TX2 + XH - T::XB;
         mbar_expect_tx(&bar, 4u * 2 * T::XZ);
@@ -105,7 +118,7 @@ __global__ void __launch_bounds__(256, 2) k_stress2d(const __grid_constant__ Str
         axf = __ldg(a.pa[0][0] + i); bxf = __ldg(a.pb[0][0] + i);
         axh = __ldg(a.pa[0][1] + i); bxh = __ldg(a.pb[0][1] + i);
     }
-    // the thread's own cells, loaded while the tiles are on their way
+    // the thread's own cells
     float o[3][NR], otp[NR], vM[NR], vU[NR], px[2][NR], pz[2][NR];
 #pragma unroll
     for (int r = 0; r < NR; r++) {
@@ -113,20 +126,21 @@ __global__ void __launch_bounds__(256, 2) k_stress2d(const __grid_constant__ Str
         if (!act || k >= a.nz) continue;
         const int c = k * sz + i;
 #pragma unroll
-        for (int q = 0; q < 3; q++) o[q][r] = sig[q][c];
-        if (PS) otp[r] = tp[c];
+        for (int q = 0; q < 3; q++) o[q][r] = __ldcg(&sig[q][c]);
+        if (PS) otp[r] = __ldcg(&tp[c]);
         vM[r] = __ldg(a.M + c);
         vU[r] = __ldg(a.MU + c);
         if (CPML && inx) {
-            px[0][r] = a.psi[P_EXX][k * WX + slx];
-            px[1][r] = a.psi[P_DXVZ][k * WX + slx];
+            px[0][r] = __ldcg(&a.psi[P_EXX][k * WX + slx]);
+            px[1][r] = __ldcg(&a.psi[P_DXVZ][k * WX + slx]);
         }
         if (CPML && (k < a.w[4] || k >= a.nz - a.w[5])) {
             const int z = (k < a.w[4] ? k : k - a.nz + a.w[4] + a.w[5]) * a.nx + i;
-            pz[0][r] = a.psi[P_EZZ][z];
-            pz[1][r] = a.psi[P_DZVX][z];
+            pz[0][r] = __ldcg(&a.psi[P_EZZ][z]);
+            pz[1][r] = __ldcg(&a.psi[P_DZVX][z]);
         }
     }
+    tile2_go(false);
     if (!tile2_wait(&bar, consumer_polls(a), a.err, skip)) return;
     if (!act || r0 >= a.nz) return;
     // tile cell (row kt + q, column i) sits at [(q + R) * XW + tx + XB]
@@ -209,6 +223,7 @@ __global__ void __launch_bounds__(256, 2) k_velocity2d(const __grid_constant__ V
     const int sz = (int)a.sz;
     const bool skip = tile2_skip<T::TZ>(a);
     tile2_begin(&bar);
+    tile2_go(true);
     if (threadIdx.x == 0 && !skip) {
         const int gx = (int)blockIdx.x * TX2 + XH;
         mbar_expect_tx(&bar, 4u * (T::X + T::XZ + T::Z + (PS ? T::XZ : 0)));
@@ -239,25 +254,26 @@ __global__ void __launch_bounds__(256, 2) k_velocity2d(const __grid_constant__ V
         const int k = r0 + r;
         if (!act || k >= a.nz) continue;
         const int c = k * sz + i;
-        ovx[r] = vx[c];
-        ovz[r] = vz[c];
+        ovx[r] = __ldcg(&vx[c]);
+        ovz[r] = __ldcg(&vz[c]);
         vb[r] = __ldg(a.B + c);
         if (PS) {
-            opx[r] = vxp[c];
-            opz[r] = vzp[c];
+            opx[r] = __ldcg(&vxp[c]);
+            opz[r] = __ldcg(&vzp[c]);
         }
-        if (EPI == EPI_EXCITE) oex[r] = a.ex_amp2[c];
-        if (EPI == EPI_IMAGE) oex[r] = __int_as_float(a.ex_time[c]);
+        if (EPI == EPI_EXCITE) oex[r] = __ldcg(&a.ex_amp2[c]);
+        if (EPI == EPI_IMAGE) oex[r] = __int_as_float(__ldcg(&a.ex_time[c]));
         if (CPML && inx) {
-            px[0][r] = a.psi[P_DXTXX][k * WX + slx];
-            px[1][r] = a.psi[P_DXTXZ][k * WX + slx];
+            px[0][r] = __ldcg(&a.psi[P_DXTXX][k * WX + slx]);
+            px[1][r] = __ldcg(&a.psi[P_DXTXZ][k * WX + slx]);
         }
         if (CPML && (k < a.w[4] || k >= a.nz - a.w[5])) {
             const int z = (k < a.w[4] ? k : k - a.nz + a.w[4] + a.w[5]) * a.nx + i;
-            pz[0][r] = a.psi[P_DZTXZ][z];
-            pz[1][r] = a.psi[P_DZTZZ][z];
+            pz[0][r] = __ldcg(&a.psi[P_DZTXZ][z]);
+            pz[1][r] = __ldcg(&a.psi[P_DZTZZ][z]);
         }
     }
+    tile2_go(false);
     if (!tile2_wait(&bar, consumer_polls(a), a.err, skip)) return;
     if (!act || r0 >= a.nz) return;
     const float* Txx = sm + tr * NR * XW + tx + T::XB;
