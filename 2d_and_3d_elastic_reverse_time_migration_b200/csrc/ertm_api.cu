@@ -668,16 +668,26 @@ struct Range {
 // while a replay of 8 steps already hides its own launch.  Long passes amortise 32.  Two
 // graphs' worth of steps go first, so that the GPU has work while the host builds the graph
 // (a pass of 680 x 380 costs 133 us besides its steps; 196 with one step first and its state
-// zeroed array by array).
+// zeroed array by array).  2D grids of 100,000 to 600,000 cells are launched directly up to 200
+// steps: their steps (4-15 us) outlast the launches but too few of them outlast the graph's
+// construction (680 x 380, 120 steps 0.90 ms, 1.08 with a graph; 240 steps 1.75 and, with four
+// graphs' worth of steps first, 1.77; 800 steps 5.75 and 5.62).  On smaller grids the host is
+// the slower side (168 x 104, 800 steps 4.3 ms, 3.4 with a graph), on larger ones two graphs'
+// worth of steps hide the construction (1471 x 803, 120 steps 2.73 and 2.68).
 template <typename F>
 int time_loop(ertm_ctx* c, int nsteps, int dir, F&& one_step)
 {
     const int kGraphSteps = nsteps >= 1500 ? 32 : 8;
-    const int lead = nsteps >= 4 * kGraphSteps ? 2 * kGraphSteps : 1;
+    const long long cells = (long long)c->g.nx * c->g.nz;
+    const bool medium2d = c->g.two_d && cells > 100000 && cells < 600000;
+    const bool use_graph = !medium2d || nsteps >= 200;
+    const int lead = medium2d && nsteps >= 8 * kGraphSteps ? 4 * kGraphSteps
+                     : nsteps >= 4 * kGraphSteps           ? 2 * kGraphSteps
+                                                           : 1;
     int done = 0;
     for (; done < std::min(nsteps, lead); done++) CK(c, one_step(dir * done));
     int base = 0;                    // steps that the device's index has moved
-    if (nsteps - done >= 2 * kGraphSteps) {
+    if (use_graph && nsteps - done >= 2 * kGraphSteps) {
         CK(c, launch_advance(c->it_d, dir * done, c->stream));
         base = done;
         c->launches++;

@@ -16,11 +16,11 @@ static long long rup(long long v, long long m) { return (v + m - 1) / m * m; }
 
 // Rows per thread of the 2D tile kernels: as many (1, 2 or 4) as still give every SM a
 // CTA (64 columns x 4 rows of threads).  More rows per thread share more of the z window
-// and re-read fewer halo rows, fewer rows give small grids more CTAs.  Measured on B200,
-// us per step (R = 4, C-PML, modelling) with 1 / 2 / 4 rows: 168 x 104 4.3 / 4.8 / 6.1,
-// 680 x 380 10.5 / 9.6 / 8.0, 4096 x 2048 201 / 166 / 154.  With R = 6 the four-row
-// kernels' registers leave one CTA less per SM, which costs a grid that streams from
-// HBM more than the window saves: 4096 x 2048 205 / 155 / 165 (1471 x 803: 30 / 23 / 22).
+// and re-read fewer halo rows, fewer rows give small grids more CTAs.  Measured on B200, ms
+// for 200 steps (R = 4, C-PML, modelling) with 1 / 2 / 4 rows: 168 x 104 1.07 / 1.13 / 1.35,
+// 680 x 380 2.16 / 2.01 / 1.60, 1471 x 803 6.18 / 4.89 / 4.40.  With R = 6 the four-row
+// kernels' registers leave one CTA less per SM, which costs a grid that streams from HBM
+// more than the window saves (4096 x 2048, us per step: 205 / 155 / 165).
 static int rows2d(int nx, int nz, int R)
 {
     const long long cols = (nx + TX2 - 1) / TX2;
