@@ -153,10 +153,11 @@ void sponge_profile(int n, int w0, int w1, int kind, float coe, int i0, int m, f
 // from there to 40-48 (480 x 480 x 380, RTM: 235.0, 234.8, 234.6 ms for 32, 40, 48; five
 // windows of different sizes in one launch: 120.5, 120.7, 121.5) and grows above (236.1, 245.2
 // and 123.5, 128.7 for 64, 96) and below (237.5 and 121.3 for 24).  A smaller launch needs its
-// last wave full: the chunk of 8 to 48 planes with the least waves x (planes + start-up),
+// last wave full: the chunk of 4 to 48 planes with the least waves x (planes + start-up),
 // start-up being the fill of the z queues and of the ring, about 8 planes' time (151 x 133 x
 // 117, modelling, 80 steps: 9.45 ms in chunks of 30 planes, 340 CTAs on 296 places, and 8.19
-// in chunks of 39, 255 CTAs).
+// in chunks of 39, 255 CTAs; 64 x 64 x 64, RTM, 75 steps: 2.07 ms in chunks of 8, 128 CTAs, and
+// 1.78 in chunks of 4).
 int choose_kchunk(long long tiles, int nz)
 {
     constexpr long long places = CTAS3 * 148;
@@ -164,7 +165,7 @@ int choose_kchunk(long long tiles, int nz)
     int best = (nz + n32 - 1) / n32;
     if (tiles * n32 >= 8 * places) return best;
     double best_cost = 1e300;
-    for (int n = (nz + 47) / 48; n <= (nz + 7) / 8; n++) {
+    for (int n = (nz + 47) / 48; n <= (nz + 3) / 4; n++) {
         const int kc = (nz + n - 1) / n, chunks = (nz + kc - 1) / kc;
         const long long waves = (tiles * chunks + places - 1) / places;
         const double cost = (double)waves * (kc + 8);
