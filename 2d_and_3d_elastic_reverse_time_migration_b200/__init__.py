@@ -381,6 +381,11 @@ class Context:
         n = self.ncell
         args = [vp, vs, rho]
         args = [a if _is_torch(a) else np.ascontiguousarray(a, np.float32) for a in args]
+        for a in args:                           # the context copies them on its own stream
+            if _is_torch(a) and a.is_cuda:
+                import torch
+                torch.cuda.current_stream(a.device).synchronize()
+                break
         self._ck(self._L.ertm_set_model(self._h, which, *[_ptr(a, n) for a in args]))
 
     @_logged
