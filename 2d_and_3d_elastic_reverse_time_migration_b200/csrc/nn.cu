@@ -94,15 +94,13 @@ __device__ __forceinline__ void stage(uint8_t* dst, const L& ld, int r0, int k0)
 }
 
 template <int BN, class LA, class LB, class EP>
-__global__ void __launch_bounds__(NT) k_gemm(LA la, LB lb, EP ep, int M, int N, int K, int kt_per, int* err)
+__global__ void __launch_bounds__(NT) k_gemm(LA la, LB lb, EP ep, int M, int N, int K, int* err)
 {
     extern __shared__ __align__(128) uint8_t smraw[];
     Smem<BN>& S = *reinterpret_cast<Smem<BN>*>(smraw);
     constexpr int TCOLS = BN < 32 ? 32 : BN;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
-    const int KT = (K + BK - 1) / BK;
-    const int kt0 = blockIdx.z * kt_per, kt1 = min(KT, kt0 + kt_per);
 
     constexpr int NS = Smem<BN>::NS;
     if (threadIdx.x == 0) {
@@ -121,14 +119,14 @@ __global__ void __launch_bounds__(NT) k_gemm(LA la, LB lb, EP ep, int M, int N, 
     const uint32_t tmem = S.tmem;
     constexpr uint32_t IDESC = idesc_bf16(BN);
     bool ok = true;
-    const int nu = kt1 - kt0;
+    const int nu = (K + BK - 1) / BK;
     // every thread copies its chunks of K tile u into slot u % NS with cp.async, one
     // commit group per tile (empty groups keep the count uniform)
     auto issue = [&](int u) {
         if (u < nu) {
             const int sl = u % NS;
-            stage<BM>(S.a[sl], la, m0, (kt0 + u) * BK);
-            stage<BN>(S.b[sl], lb, n0, (kt0 + u) * BK);
+            stage<BM>(S.a[sl], la, m0, u * BK);
+            stage<BN>(S.b[sl], lb, n0, u * BK);
         }
         cp_commit();
     };
@@ -179,31 +177,25 @@ __global__ void __launch_bounds__(NT) k_gemm(LA la, LB lb, EP ep, int M, int N, 
 }
 
 template <int BN, class LA, class LB, class EP>
-cudaError_t gemm_bn(const LA& la, const LB& lb, const EP& ep, int M, int N, int K, int splitk, int* err,
-                    cudaStream_t st)
+cudaError_t gemm_bn(const LA& la, const LB& lb, const EP& ep, int M, int N, int K, int* err, cudaStream_t st)
 {
-    const int KT = (K + BK - 1) / BK;
-    splitk = splitk < 1 ? 1 : (splitk > KT ? KT : splitk);
-    const int kt_per = (KT + splitk - 1) / splitk;
-    const int gz = (KT + kt_per - 1) / kt_per;
     const size_t smem = sizeof(Smem<BN>);
     static unsigned long long opted = 0;   // devices with the opt-in made
     cudaError_t attr = ertm::smem_opt_in(k_gemm<BN, LA, LB, EP>, smem, &opted);
     if (attr != cudaSuccess) return attr;
-    dim3 grid((M + BM - 1) / BM, (N + BN - 1) / BN, gz);
-    k_gemm<BN, LA, LB, EP><<<grid, NT, smem, st>>>(la, lb, ep, M, N, K, kt_per, err);
+    dim3 grid((M + BM - 1) / BM, (N + BN - 1) / BN);
+    k_gemm<BN, LA, LB, EP><<<grid, NT, smem, st>>>(la, lb, ep, M, N, K, err);
     return cudaGetLastError();
 }
 
 // N tile: 16 <= BN <= 128, multiple of 16 (tcgen05 M = 128 needs N % 16 == 0)
 template <class LA, class LB, class EP>
-cudaError_t gemm(const LA& la, const LB& lb, const EP& ep, int M, int N, int K, int splitk, int* err,
-                 cudaStream_t st)
+cudaError_t gemm(const LA& la, const LB& lb, const EP& ep, int M, int N, int K, int* err, cudaStream_t st)
 {
-    if (N <= 16) return gemm_bn<16>(la, lb, ep, M, N, K, splitk, err, st);
-    if (N <= 32) return gemm_bn<32>(la, lb, ep, M, N, K, splitk, err, st);
-    if (N <= 64) return gemm_bn<64>(la, lb, ep, M, N, K, splitk, err, st);
-    return gemm_bn<128>(la, lb, ep, M, N, K, splitk, err, st);
+    if (N <= 16) return gemm_bn<16>(la, lb, ep, M, N, K, err, st);
+    if (N <= 32) return gemm_bn<32>(la, lb, ep, M, N, K, err, st);
+    if (N <= 64) return gemm_bn<64>(la, lb, ep, M, N, K, err, st);
+    return gemm_bn<128>(la, lb, ep, M, N, K, err, st);
 }
 
 // ---------------------------------------------------------------------------
@@ -488,7 +480,7 @@ int ertm_nn_gemm(const void* a, const void* b, float* d, int M, int N, int K, in
     LoadRows la{reinterpret_cast<const bf16*>(a), M, K, K};
     LoadRows lb{reinterpret_cast<const bf16*>(b), N, K, K};
     EpiF32 ep{d, N, N, M};
-    return rc_of(gemm(la, lb, ep, M, N, K, 1, err, (cudaStream_t)stream));
+    return rc_of(gemm(la, lb, ep, M, N, K, err, (cudaStream_t)stream));
 }
 
 int ertm_nn_pool2(const ertm_nn_act* x, void* y, void* stream)
