@@ -1901,6 +1901,9 @@ int ertm_born_adjoint_shots(ertm_ctx* c, const ertm_shot* shots, int nshots, con
         B.hist = nullptr;
         B.hist_floats = 0;
         CK(c, cudaMalloc(&B.hist, sizeof(float) * hist_need));
+        // the recording steps write cells only, the adjoint reads v0 with its halo, which is zero;
+        // a volume's halo is at the same places in every group and segment
+        CK(c, cudaMemsetAsync(B.hist, 0, sizeof(float) * hist_need, c->stream));
         B.hist_floats = hist_need;
     }
     if (!dev_res && (rc = ensure_traces(c, (size_t)nd * G))) return rc;
