@@ -161,7 +161,7 @@ inline cudaError_t smem_opt_in(KPTR K, size_t smem, unsigned long long* done)
 
 // A step kernel launched as a programmatic dependent of the launch before it in the
 // stream: its CTAs may become resident while that one drains, and it waits for it
-// (pdl_wait) before touching memory.  The edge survives stream capture.
+// (pdl_wait) before it reads what that one writes.  The edge survives stream capture.
 template <typename... P>
 inline cudaError_t launch_pdl(void (*K)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, const P&... args)
 {

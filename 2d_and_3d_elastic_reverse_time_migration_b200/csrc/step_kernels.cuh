@@ -70,8 +70,9 @@ __device__ __forceinline__ void damping(const KArgs& a, bool cpml, int i, int j,
     }
 }
 
-// step index of this launch (a plain load: a dependent launch may start before the
-// counter's last change, see step_kernels_2d.cuh)
+// step index of this launch; a kernel that is launched as a programmatic dependent reads it
+// after its wait, since the launch before may have changed it.  (A volatile load: the value
+// may not come from a read-only cache.)
 __device__ __forceinline__ int step_index(const KArgs& a)
 {
     return *(volatile const int*)a.it_ptr + a.it_add;

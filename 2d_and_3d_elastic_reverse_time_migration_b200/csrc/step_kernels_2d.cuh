@@ -9,8 +9,9 @@
 // single mbarrier, and meanwhile every thread loads the values of its own cells
 // straight into registers.  The z stencils of a thread's rows share one column window
 // read from shared memory.  Consecutive launches overlap through programmatic
-// dependent launch: a kernel sets up its barrier while the previous one drains and
-// waits (griddepcontrol.wait) before it touches memory.
+// dependent launch: while the previous one drains, a kernel sets up its barrier and loads
+// what was written two launches ago; what is newer it reads after griddepcontrol.wait
+// (see tile2_begin).
 //
 // Measured on B200 against the z-marching kernels that 2D grids shared with 3D (one
 // 32-cell row per CTA and TMA round trip) and their separate step-counter launch, ms per
@@ -39,7 +40,10 @@ struct Tile2 {
 // Shared by the tile kernels.  Launches alternate between two kernels, each of which writes
 // what it alone loads cell by cell and the other stages: a thread's own values were last
 // written two launches ago.  That launch had completed when the previous one passed its
-// wait, and only then does that one let this one start.  So the staging warp waits and
+// wait, and only then does that one let this one start.  Nothing else that changes in a pass
+// is read ahead of the wait, the step index least of all: the launch before the first step
+// writes it (what the host copies or clears for a pass lies a whole launch further back, or
+// is no kernel, and overlaps with nothing).  So the staging warp waits and
 // issues the copies first, while the others load their own values, past L1, before they
 // wait.  Of it: us per step, modelling 168 x 104 4.36 -> 3.93, 680 x 380 8.20 -> 6.74;
 // modelling 1471 x 803 2.10 -> 2.03 ms.  (Every warp loading before the wait: 3.81, 6.74, but
@@ -104,10 +108,6 @@ __global__ void __launch_bounds__(256, 2) k_stress2d(const __grid_constant__ Str
         tma3(sm + XZP, &maps.v[1], gx, 0, kt, &bar);
     }
     const bool act = i < a.nx;
-    const int it = step_index(a);
-    const bool src_on = (it >= 0) && (it < a.nw);
-    const bool src_here = src_on && (i == a.ssx);
-    const float wsrc = src_on ? __ldg(a.wavelet + it) : 0.f;
     float* sig[3] = {a.f[F_TXX], a.f[F_TZZ], a.f[F_TXZ]};
     float* tp = a.f[F_TP];
     const int WX = a.w[0] + a.w[1];
@@ -141,6 +141,14 @@ __global__ void __launch_bounds__(256, 2) k_stress2d(const __grid_constant__ Str
         }
     }
     tile2_go(false);
+    // source sample of this step, in the threads of its cell's column
+    float wsrc = 0.f;
+    bool src_here = i == a.ssx && r0 <= a.ssz && a.ssz < r0 + NR;
+    if (src_here) {
+        const int it = step_index(a);
+        src_here = it >= 0 && it < a.nw;
+        if (src_here) wsrc = __ldg(a.wavelet + it);
+    }
     if (!tile2_wait(&bar, consumer_polls(a), a.err, skip)) return;
     if (!act || r0 >= a.nz) return;
     // tile cell (row kt + q, column i) sits at [(q + R) * XW + tx + XB]
@@ -233,7 +241,6 @@ __global__ void __launch_bounds__(256, 2) k_velocity2d(const __grid_constant__ V
         if (PS) tma3(sm + O_TP, &maps.tp, gx - T::XB, 0, kt, &bar);
     }
     const bool act = i < a.nx;
-    const int it = step_index(a);
     const int rec = ((REC || EPI == EPI_IMAGE) && act) ? receiver_index(a, i, 0) : -1;
     const long long nrec = (long long)a.nrx * a.nry;
     float* vx = a.f[F_VX];
@@ -274,6 +281,7 @@ __global__ void __launch_bounds__(256, 2) k_velocity2d(const __grid_constant__ V
         }
     }
     tile2_go(false);
+    const int it = EPI != EPI_NONE || REC ? step_index(a) : 0;
     if (!tile2_wait(&bar, consumer_polls(a), a.err, skip)) return;
     if (!act || r0 >= a.nz) return;
     const float* Txx = sm + tr * NR * XW + tx + T::XB;
