@@ -258,6 +258,17 @@ def _is_torch(a) -> bool:
     return type(a).__module__.startswith("torch")
 
 
+def _after_torch(*arrays):
+    """Waits for the work that torch's current stream still has queued on the CUDA tensors
+    among `arrays`: a context reads its inputs and writes its outputs on a stream of its own,
+    which waits for no other."""
+    devices = {a.device for a in arrays if _is_torch(a) and a.is_cuda}
+    if devices:
+        import torch
+        for d in devices:
+            torch.cuda.current_stream(d).synchronize()
+
+
 def _ptr(a, n: int | None = None, writable: bool = False):
     """Raw pointer of a float32/int32 numpy array or torch tensor (contiguous)."""
     if a is None:
@@ -381,11 +392,7 @@ class Context:
         n = self.ncell
         args = [vp, vs, rho]
         args = [a if _is_torch(a) else np.ascontiguousarray(a, np.float32) for a in args]
-        for a in args:                           # the context copies them on its own stream
-            if _is_torch(a) and a.is_cuda:
-                import torch
-                torch.cuda.current_stream(a.device).synchronize()
-                break
+        _after_torch(*args)
         self._ck(self._L.ertm_set_model(self._h, which, *[_ptr(a, n) for a in args]))
 
     @_logged
@@ -394,6 +401,7 @@ class Context:
         if out is None:
             out = np.zeros((3, self.cfg.nt, shot.nrec), np.float32)
         s = shot.struct()
+        _after_torch(out, shot.wavelet)
         self._ck(self._L.ertm_forward_together_using_real_model(self._h, C.byref(s),
                                                                 _ptr(out, n, True)))
         return out
@@ -401,6 +409,7 @@ class Context:
     @_logged
     def forward_together_using_smoothed_model(self, shot: Shot):
         s = shot.struct()
+        _after_torch(shot.wavelet)
         self._ck(self._L.ertm_forward_together_using_smoothed_model(self._h, C.byref(s)))
 
     @_logged
@@ -409,6 +418,7 @@ class Context:
         pp, ps, tp = self._vol(pp), self._vol(ps), self._vol(tp)
         d = data if _is_torch(data) else np.ascontiguousarray(data, np.float32)
         s = shot.struct()
+        _after_torch(d, pp, ps, tp, shot.wavelet)
         self._ck(self._L.ertm_backward_together_using_smoothed_model(
             self._h, C.byref(s), _ptr(d, 3 * self.cfg.nt * shot.nrec), _ptr(pp, n, True),
             _ptr(ps, n, True), _ptr(tp, n, True)))
@@ -420,6 +430,7 @@ class Context:
         pp, ps, tp = self._vol(pp), self._vol(ps), self._vol(tp)
         d = data if _is_torch(data) else np.ascontiguousarray(data, np.float32)
         s = shot.struct()
+        _after_torch(d, pp, ps, tp, shot.wavelet)
         self._ck(self._L.ertm_rtm_shot(self._h, C.byref(s), _ptr(d, 3 * self.cfg.nt * shot.nrec),
                                        _ptr(pp, n, True), _ptr(ps, n, True), _ptr(tp, n, True)))
         return pp, ps, tp
@@ -437,6 +448,7 @@ class Context:
             d = d if _is_torch(d) else np.ascontiguousarray(d, np.float32)
             keep.append(d)
             ptrs[q] = _ptr(d, 3 * self.cfg.nt * sh.nrec)
+        _after_torch(*data, pp, ps, tp, *[sh.wavelet for sh in shots])
         self._ck(self._L.ertm_rtm_batch(self._h, arr, len(shots), ptrs, _ptr(pp, n, True),
                                         _ptr(ps, n, True), _ptr(tp, n, True)))
         del keep
@@ -445,6 +457,7 @@ class Context:
     def get_wavefield(self, name_or_id, out=None):
         fid = FIELDS.index(name_or_id) if isinstance(name_or_id, str) else int(name_or_id)
         out = self._vol(out)
+        _after_torch(out)
         self._ck(self._L.ertm_get_wavefield(self._h, fid, _ptr(out, self.ncell, True)))
         return out
 
@@ -478,11 +491,13 @@ class Context:
 
     def propagate(self, which: int, shot: Shot, nsteps: int):
         s = shot.struct()
+        _after_torch(shot.wavelet)
         self._ck(self._L.ertm_propagate(self._h, which, C.byref(s), nsteps))
 
     def time_kernels(self, shot: Shot, nsteps: int):
         ms = (C.c_float * 2)()
         s = shot.struct()
+        _after_torch(shot.wavelet)
         self._ck(self._L.ertm_time_kernels(self._h, C.byref(s), nsteps, ms))
         return float(ms[0]), float(ms[1])
 
@@ -494,6 +509,7 @@ class Context:
             out = np.zeros((3, self.cfg.nt, shot.nrec), np.float32)
         args = [a if _is_torch(a) else np.ascontiguousarray(a, np.float32) for a in (r_vp, r_vs, r_rho)]
         s = shot.struct()
+        _after_torch(*args, out, shot.wavelet)
         self._ck(self._L.ertm_born_forward(self._h, C.byref(s), *[_ptr(a, n) for a in args],
                                            _ptr(out, 3 * self.cfg.nt * shot.nrec, True)))
         return out
@@ -505,6 +521,7 @@ class Context:
         outs = [self._vol(o) for o in (g_vp, g_vs, g_rho)]
         r = residual if _is_torch(residual) else np.ascontiguousarray(residual, np.float32)
         s = shot.struct()
+        _after_torch(r, *outs, shot.wavelet)
         self._ck(self._L.ertm_born_adjoint(self._h, C.byref(s), _ptr(r, 3 * self.cfg.nt * shot.nrec),
                                            *[_ptr(o, n, True) for o in outs]))
         return tuple(outs)
@@ -528,6 +545,7 @@ class Context:
             out = np.zeros((ns, 3, self.cfg.nt, nrec), np.float32)
         args = [a if _is_torch(a) else np.ascontiguousarray(a, np.float32) for a in (r_vp, r_vs, r_rho)]
         arr, keep = self._shot_array(shots)
+        _after_torch(*args, out, *[sh.wavelet for sh in shots])
         self._ck(self._L.ertm_born_forward_shots(self._h, arr, ns, *[_ptr(a, n) for a in args],
                                                  _ptr(out, ns * 3 * self.cfg.nt * nrec, True)))
         del keep
@@ -541,6 +559,7 @@ class Context:
         outs = [self._vol(o) for o in (g_vp, g_vs, g_rho)]
         r = residual if _is_torch(residual) else np.ascontiguousarray(residual, np.float32)
         arr, keep = self._shot_array(shots)
+        _after_torch(r, *outs, *[sh.wavelet for sh in shots])
         self._ck(self._L.ertm_born_adjoint_shots(self._h, arr, ns,
                                                  _ptr(r, ns * 3 * self.cfg.nt * shots[0].nrec),
                                                  *[_ptr(o, n, True) for o in outs]))
@@ -570,8 +589,11 @@ def forward_together_using_real_model_noalloc(cfg: Config, vp, vs, rho, shot: Sh
     For callers that may not allocate device memory when they call in: every
     array (vp, vs, rho, shot.wavelet, out of shape (3, nt, nrec)) must already be
     a CUDA tensor; the library's wavefields live in a fixed 64 MiB device array.
-    Calls share that array, so calls that overlap on the GPU race."""
+    Calls share that array, so calls that overlap on the GPU race.  With a stream of the
+    caller's the call is ordered on it; without one it waits for torch's current stream."""
     L = lib()
+    if stream_ptr is None:
+        _after_torch(vp, vs, rho, shot.wavelet, out)
     n = cfg.nx * cfg.ny * cfg.nz
     cs, ss = cfg.struct(), shot.struct()
     buf = C.create_string_buffer(512)
@@ -621,6 +643,7 @@ def rtm_multi(contexts: list, shots: list, data: list, outs: list | None = None)
     for q, (c, o) in enumerate(zip(contexts, outs)):
         for k in range(3):
             op[k][q] = _ptr(o[k], c.ncell, True)
+    _after_torch(*data, *[v for o in outs for v in o], *[sh.wavelet for sh in shots])
     rc = L.ertm_rtm_multi(hs, n, arr, dp, op[0], op[1], op[2])
     del keep
     if rc != 0:
@@ -649,6 +672,7 @@ def rtm_windows(base: Config, vp, vs, rho, windows: list, shots: list, data: lis
         parr[q] = _ptr(d, 3 * w.nt * sh.nrec)
     cs = base.struct()
     buf = C.create_string_buffer(1024)
+    _after_torch(*model, *data, *outs, *[sh.wavelet for sh in shots])
     rc = L.ertm_rtm_windows(C.byref(cs), *[_ptr(a, n) for a in model], len(shots), warr, sarr, parr,
                             lanes, *[_ptr(o, n, True) for o in outs], buf, len(buf))
     del keep

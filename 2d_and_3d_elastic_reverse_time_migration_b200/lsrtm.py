@@ -124,8 +124,6 @@ def born_all(ctx, shots, m):
         if _is_torch(m[0]):
             import torch
             out = torch.zeros((len(shots), 3, ctx.cfg.nt, shots[0].nrec), device=m[0].device)
-            # the library works on its own stream: the inputs must be complete first
-            torch.cuda.current_stream(m[0].device).synchronize()
             return ctx.born_forward_shots(shots, *m, out=out)
         return ctx.born_forward_shots(shots, *m)
     return _stack([ctx.born_forward(s, *m) for s in shots])
@@ -141,7 +139,6 @@ def adjoint_all(ctx, shots, res):
         if _is_torch(res):
             import torch
             g = [torch.zeros(ctx.cfg.shape, device=res.device) for _ in range(3)]
-            torch.cuda.current_stream(res.device).synchronize()
             return ctx.born_adjoint_shots(shots, res, *g)
         return ctx.born_adjoint_shots(shots, res)
     g = None
