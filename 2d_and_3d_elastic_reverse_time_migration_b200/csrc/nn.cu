@@ -588,10 +588,14 @@ int ertm_nn_run(const ertm_nn_op* ops, int nops, void* const* ptr, int nptr, int
             rc = ertm_nn_conv3x3(&o.a, p[0], (const float*)p[1], &o.b, o.flag, (float*)p[2], err, stream);
             break;
         case ERTM_NN_OP_CONV_DGRAD: rc = ertm_nn_conv3x3_dgrad(&o.a, p[0], &o.b, mask, err, stream); break;
-        case ERTM_NN_OP_CONV_WGRAD: rc = ertm::nn_conv3x3_wgrad(&o.a, &o.b, (float*)p[0], (float*)p[1], err, stream); break;
+        case ERTM_NN_OP_CONV_WGRAD:
+            rc = ertm::nn_conv3x3_wgrad(&o.a, &o.b, (float*)p[0], (float*)p[1], ertm::kSplitsOfPlan, err, stream);
+            break;
         case ERTM_NN_OP_UP: rc = ertm_nn_up2(&o.a, p[0], (const float*)p[1], &o.b, o.flag, err, stream); break;
         case ERTM_NN_OP_UP_DGRAD: rc = ertm_nn_up2_dgrad(&o.a, p[0], &o.b, mask, err, stream); break;
-        case ERTM_NN_OP_UP_WGRAD: rc = ertm::nn_up2_wgrad(&o.a, &o.b, (float*)p[0], (float*)p[1], err, stream); break;
+        case ERTM_NN_OP_UP_WGRAD:
+            rc = ertm::nn_up2_wgrad(&o.a, &o.b, (float*)p[0], (float*)p[1], ertm::kSplitsOfPlan, err, stream);
+            break;
         case ERTM_NN_OP_POOL: rc = ertm_nn_pool2(&o.a, p[0], stream); break;
         case ERTM_NN_OP_POOL_BWD: rc = ertm_nn_pool2_bwd(&o.a, p[0], &o.b, o.flag, stream); break;
         case ERTM_NN_OP_ZERO: {

@@ -135,6 +135,8 @@ __device__ __forceinline__ void unpack8(const uint4& u, float* f)
 namespace ertm {
 // ertm_nn_conv3x3_wgrad and ertm_nn_up2_wgrad with the bias gradient of the same dy, db += its
 // sum over the pixels, in the same kernel (db NULL: none).
-int nn_conv3x3_wgrad(const ertm_nn_act* x, const ertm_nn_act* dy, float* dw, float* db, int* err, void* stream);
-int nn_up2_wgrad(const ertm_nn_act* x, const ertm_nn_act* dy, float* du, float* db, int* err, void* stream);
+constexpr int kSplitsOfPlan = 1 << 30;   // splitk: as many as the plan takes
+int nn_conv3x3_wgrad(const ertm_nn_act* x, const ertm_nn_act* dy, float* dw, float* db, int splitk, int* err,
+                     void* stream);
+int nn_up2_wgrad(const ertm_nn_act* x, const ertm_nn_act* dy, float* du, float* db, int splitk, int* err, void* stream);
 }  // namespace ertm

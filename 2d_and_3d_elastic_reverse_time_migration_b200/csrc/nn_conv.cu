@@ -1046,8 +1046,9 @@ cudaError_t conv_launch(const Act* x, int nmap, int step, const bf16* w, int K, 
 
 // Tiles of a weight gradient.  3x3: rr rows of dy against rr + 2 of x; more rows re-read
 // less of x and waste fewer row pairs but need TMEM (mb * n columns per kx, 512 in all)
-// and shared memory for two stages or more.
-bool wgrad_plan(WgP& best, size_t& smem, dim3& grid, int nb, int h, int w, int ci, int co, bool up)
+// and shared memory for two stages or more.  At most `most` CTAs add to an element of dw;
+// with one the sum is repeatable.
+bool wgrad_plan(WgP& best, size_t& smem, dim3& grid, int nb, int h, int w, int ci, int co, bool up, int most)
 {
     WgP p{};
     p.nb = nb;
@@ -1130,7 +1131,7 @@ bool wgrad_plan(WgP& best, size_t& smem, dim3& grid, int nb, int h, int w, int c
                         const int others = p.kgroups * p.cparts * div_up(oblk, p.OB);
                         const int px = up ? rr * tw : tw;        // accumulator chain per unit
                         const int least = div_up((long long)p.units * px, 4096);
-                        const int splits = std::min(p.units, std::max(std::max(1, SMS / others), least));
+                        const int splits = std::min({p.units, most, std::max(std::max(1, SMS / others), least)});
                         const int waves = div_up((long long)splits * others, SMS);
                         const double mma = (double)p.ksteps * p.nkx * p.mb * mma_cost(p.n);
                         const double sums = up ? (double)p.mb * 128 * p.n : 9.0 * p.CB * p.cx * p.OB * p.cy * p.nkx / 3 * rr;
@@ -1151,18 +1152,19 @@ bool wgrad_plan(WgP& best, size_t& smem, dim3& grid, int nb, int h, int w, int c
     return best_cost < 1e299;
 }
 
-cudaError_t wgrad_launch(const Act& x, const Act& dy, float* dw, float* db, bool up, int* err, cudaStream_t st)
+cudaError_t wgrad_launch(const Act& x, const Act& dy, float* dw, float* db, bool up, int most, int* err, cudaStream_t st)
 {
     struct Plan {
         WgP p;
         size_t smem;
         dim3 grid;
     };
-    static thread_local PlanCache<Plan, 6> cache;
-    const int key[6] = {x.nb, x.h, x.w, x.c, dy.c, up};
+    most = std::max(1, most);
+    static thread_local PlanCache<Plan, 7> cache;
+    const int key[7] = {x.nb, x.h, x.w, x.c, dy.c, up, most};
     bool hit;
     auto& slot = cache.at(key, hit);
-    if (!hit) slot.ok = wgrad_plan(slot.plan.p, slot.plan.smem, slot.plan.grid, x.nb, x.h, x.w, x.c, dy.c, up);
+    if (!hit) slot.ok = wgrad_plan(slot.plan.p, slot.plan.smem, slot.plan.grid, x.nb, x.h, x.w, x.c, dy.c, up, most);
     if (!slot.ok) return cudaErrorInvalidValue;
     const WgP& p = slot.plan.p;
     const size_t smem = slot.plan.smem;
@@ -1190,23 +1192,24 @@ cudaError_t wgrad_launch(const Act& x, const Act& dy, float* dw, float* db, bool
 }  // namespace
 
 namespace ertm {
-int nn_conv3x3_wgrad(const ertm_nn_act* x, const ertm_nn_act* dy, float* dw, float* db, int* err, void* stream)
+int nn_conv3x3_wgrad(const ertm_nn_act* x, const ertm_nn_act* dy, float* dw, float* db, int splitk, int* err,
+                     void* stream)
 {
     if (!act_ok(x) || !act_ok(dy) || !dw || (db && !same_grid(x, dy))) return ERTM_EINVAL;
     Act da = act_of(dy);            // dy's pixels are taken in x's grid, in order
     da.nb = x->n;
     da.h = x->h;
     da.w = x->w;
-    return rc_of(wgrad_launch(act_of(x), da, dw, db, false, err, (cudaStream_t)stream));
+    return rc_of(wgrad_launch(act_of(x), da, dw, db, false, splitk, err, (cudaStream_t)stream));
 }
 
-int nn_up2_wgrad(const ertm_nn_act* x, const ertm_nn_act* dy, float* du, float* db, int* err, void* stream)
+int nn_up2_wgrad(const ertm_nn_act* x, const ertm_nn_act* dy, float* du, float* db, int splitk, int* err, void* stream)
 {
     if (!act_ok(x) || !act_ok(dy) || !du || dy->h != 2 * x->h || dy->w != 2 * x->w || (db && dy->n != x->n))
         return ERTM_EINVAL;
     Act da = act_of(dy);
     da.nb = x->n;
-    return rc_of(wgrad_launch(act_of(x), da, du, db, true, err, (cudaStream_t)stream));
+    return rc_of(wgrad_launch(act_of(x), da, du, db, true, splitk, err, (cudaStream_t)stream));
 }
 }  // namespace ertm
 
@@ -1246,8 +1249,7 @@ int ertm_nn_conv3x3_dgrad(const ertm_nn_act* dy, const void* wflip, const ertm_n
 
 int ertm_nn_conv3x3_wgrad(const ertm_nn_act* x, const ertm_nn_act* dy, float* dw, int splitk, int* err, void* stream)
 {
-    (void)splitk;   // a hint: the plan splits the pixels by itself
-    return ertm::nn_conv3x3_wgrad(x, dy, dw, nullptr, err, stream);
+    return ertm::nn_conv3x3_wgrad(x, dy, dw, nullptr, splitk, err, stream);
 }
 
 int ertm_nn_up2(const ertm_nn_act* x, const void* u, const float* bias, const ertm_nn_act* y, int relu, int* err,
@@ -1277,8 +1279,7 @@ int ertm_nn_up2_dgrad(const ertm_nn_act* dy, const void* ut, const ertm_nn_act* 
 
 int ertm_nn_up2_wgrad(const ertm_nn_act* x, const ertm_nn_act* dy, float* du, int splitk, int* err, void* stream)
 {
-    (void)splitk;
-    return ertm::nn_up2_wgrad(x, dy, du, nullptr, err, stream);
+    return ertm::nn_up2_wgrad(x, dy, du, nullptr, splitk, err, stream);
 }
 
 }  // extern "C"

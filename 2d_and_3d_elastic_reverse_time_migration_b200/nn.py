@@ -25,6 +25,7 @@ from . import ErtmError, _NnAct, _NnOp, lib
 
 IN_C, OUT_C = 3, 3
 IN_P, OUT_P = 8, 16
+SPLITS = 1 << 30     # split-K of a weight gradient: as many partial sums as the kernel takes
 LEVELS = (16, 32, 64, 128)
 
 
@@ -75,9 +76,8 @@ class Ops:
                                          self.st), "conv3x3_dgrad")
 
     def conv_wgrad(self, x, dy, dw, splitk=0):
-        P = x.n * x.h * x.w
-        sk = splitk or max(1, min(148 * 2, P // 4096))
-        _ck(self.L.ertm_nn_conv3x3_wgrad(C.byref(x), C.byref(dy), _p(dw), sk, _p(self.err), self.st),
+        """splitk: at most that many partial sums per element (1: repeatable); 0: the kernel's choice."""
+        _ck(self.L.ertm_nn_conv3x3_wgrad(C.byref(x), C.byref(dy), _p(dw), splitk or SPLITS, _p(self.err), self.st),
             "conv3x3_wgrad")
 
     def up(self, x, u, bias, y, relu=True):
@@ -90,9 +90,7 @@ class Ops:
                                      self.st), "up2_dgrad")
 
     def up_wgrad(self, x, dy, du, splitk=0):
-        P = x.n * x.h * x.w
-        sk = splitk or max(1, min(148 * 2, P // 4096))
-        _ck(self.L.ertm_nn_up2_wgrad(C.byref(x), C.byref(dy), _p(du), sk, _p(self.err), self.st),
+        _ck(self.L.ertm_nn_up2_wgrad(C.byref(x), C.byref(dy), _p(du), splitk or SPLITS, _p(self.err), self.st),
             "up2_wgrad")
 
     def pool(self, x, y):

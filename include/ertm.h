@@ -430,7 +430,10 @@ int ertm_nn_conv3x3(const ertm_nn_act *x, const void *w, const float *bias, cons
  * wflip from ertm_nn_flip3 */
 int ertm_nn_conv3x3_dgrad(const ertm_nn_act *dy, const void *wflip, const ertm_nn_act *dx,
                           const ertm_nn_act *mask, int *err, void *stream);
-/* weight gradient of a 3x3 convolution, accumulated: dw[dy.c][9][x.c] += ... (split-K) */
+/* weight gradient of a 3x3 convolution, accumulated: dw[dy.c][9][x.c] += ...  An element is
+ * the sum of at most splitk partial sums over the pixels (values below 1 count as 1), added
+ * atomically: with 1 the result is repeatable, with a large value the kernel splits as far as
+ * that makes it faster. */
 int ertm_nn_conv3x3_wgrad(const ertm_nn_act *x, const ertm_nn_act *dy, float *dw, int splitk,
                           int *err, void *stream);
 /* 2x2 stride-2 transposed convolution: y[2i+a][2j+b][o] = relu?(sum_c x[i][j][c] u[(2a+b)*y.c+o][c]
@@ -440,7 +443,7 @@ int ertm_nn_up2(const ertm_nn_act *x, const void *u, const float *bias, const er
 /* input gradient of ertm_nn_up2 (ut = u transposed, [x.c][4 y.c]), optional ReLU mask */
 int ertm_nn_up2_dgrad(const ertm_nn_act *dy, const void *ut, const ertm_nn_act *dx,
                       const ertm_nn_act *mask, int *err, void *stream);
-/* weight gradient of ertm_nn_up2, accumulated: du[4 dy.c][x.c] += ... */
+/* weight gradient of ertm_nn_up2, accumulated: du[4 dy.c][x.c] += ...; splitk as above */
 int ertm_nn_up2_wgrad(const ertm_nn_act *x, const ertm_nn_act *dy, float *du, int splitk, int *err,
                       void *stream);
 /* 2x2 max pooling into a dense BF16 output [n][h/2][w/2][x.c] */

@@ -162,3 +162,28 @@ def test_op_lists(env, n, h, w):
         rc = L.ertm_nn_run(C.byref(op), 1, ptr, 1, C.byref(done), None, o.st)
         assert rc == -1 and done.value == 0
     assert int(o.err.item()) == 0
+
+
+# splitk bounds the partial sums of an element; one sum is repeatable, with any number of pixels
+@pytest.mark.parametrize("n,h,w,ci,co", [(2, 7, 61, 24, 40), (3, 40, 130, 32, 48), (2, 64, 128, 16, 16),
+                                         (1, 33, 70, 128, 64)])
+def test_one_sum_per_weight_is_repeatable(env, n, h, w, ci, co):
+    torch, nn, ops, dev = env
+    x = torch.randn(n, h, w, ci, device=dev).relu().bfloat16()
+    dy, dyu = (torch.randn(n, s * h, s * w, co, device=dev).bfloat16() for s in (1, 2))
+
+    def grads(k):
+        dw, du = torch.zeros(co, 9 * ci, device=dev), torch.zeros(4 * co, ci, device=dev)
+        ops.conv_wgrad(nn.act(x, n, h, w), nn.act(dy, n, h, w), dw, splitk=k)
+        ops.up_wgrad(nn.act(x, n, h, w), nn.act(dyu, n, 2 * h, 2 * w), du, splitk=k)
+        return dw, du
+
+    first, many = grads(1), grads(0)
+    for _ in range(20):
+        assert all(torch.equal(a, b) for a, b in zip(grads(1), first))
+    for k in (2, 5):                           # as the other splits, to the FP32 rounding of the sums
+        for a, b in zip(grads(k), many):
+            assert _rel(a, b) <= 1e-4
+    for a, b in zip(first, many):
+        assert _rel(a, b) <= 1e-4
+    assert int(ops.err.item()) == 0
