@@ -276,6 +276,7 @@ constexpr int EPW = 16;                // epilogue warps: four per quarter of th
 constexpr int CTHREADS = 32 * (EPW + 2);
 constexpr int MAXSLOT = 16;
 constexpr int SMEM_MAX = 220 * 1024;   // dynamic shared memory a CTA may take
+constexpr int ZEROS = 128 * 16;        // one 16-byte chunk of each of an MMA's 128 rows
 
 // Tile plan of a convolution launch
 struct ConvP {
@@ -290,6 +291,7 @@ struct ConvP {
     int slots, nbuf, bn, tcols;
     uint32_t pitch;               // bytes of a staged pixel
     uint32_t plane, abytes, aslot, slot;   // bytes: a chunk plane, a box, a slot's input part, a slot
+    uint32_t zeros;               // pair8: offset of a slot's ZEROS bytes of zeros
     uint32_t wtap;                // chunk planes: bytes of the weights of one block and tap
     uint32_t woff, wbytes;        // resident weights: shared-memory offset, bytes
     int groups, entries;          // 16-channel groups and MMAs of a tile (streamed: of a block)
@@ -326,6 +328,12 @@ __global__ void __launch_bounds__(CTHREADS, 1) k_conv(const __grid_constant__ Co
         mbar_init(&wfull, 1);
         mbar_init(&done, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (p.pair8) {
+        for (int q = threadIdx.x; q < p.slots * (ZEROS / 16); q += CTHREADS)
+            *reinterpret_cast<uint4*>(sm + (size_t)(q / (ZEROS / 16)) * p.slot + p.zeros + q % (ZEROS / 16) * 16) =
+                make_uint4(0, 0, 0, 0);
+        proxy_fence();
     }
     if (warp == EPW + 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(su32(&tmem_s)),
@@ -404,10 +412,11 @@ __global__ void __launch_bounds__(CTHREADS, 1) k_conv(const __grid_constant__ Co
             } else
                 w = (p.stream ? (p.aslot >> 4) : 0) + (gg * p.taps + t) * (p.wtap >> 4);
             if (p.pair8) {
-                // K = taps 2t, 2t+1 of the one chunk; the ninth has zero weights beside it
+                // K = taps 2t, 2t+1 of the one chunk.  The ninth has zero weights beside it, and
+                // zeros for pixels: a pixel there could be infinite, and its product NaN.
                 const int ta = 2 * t, tb = ta + 1;
                 a = (ta / 3) * p.wp + ta % 3;
-                lbo = tb < 9 ? (tb / 3) * p.wp + tb % 3 - a : (uint32_t)p.wp;
+                lbo = tb < 9 ? (tb / 3) * p.wp + tb % 3 - a : (p.zeros >> 4) - (a + b * p.mstep);
             } else if (p.halo)
                 a += ((t / 3) * p.wp + t % 3) * p16;
             tab[i] = MmaEntry{a + b * p.mstep * p16 | lbo << 16, w | (uint32_t)(b * p.bn) << 16};
@@ -926,7 +935,7 @@ bool conv_plan(ConvP& best, size_t& smem, int& gx, int& gy, int nb, int h, int w
     for (int ro = 1; ro <= 16; ro *= 2) {
         if (ro > 1 && ro / 2 >= h) break;
         p.ro = ro;
-        p.rows = ro + 2 * p.halo + (p.pair8 ? 1 : 0);
+        p.rows = ro + 2 * p.halo;
         p.mstep = rowmode ? p.wp : 128;
         p.nblk = rowmode ? ro : div_up((long long)(ro - 1) * p.wp + p.txw, 128);
         p.ty = div_up(h, ro);
@@ -943,11 +952,12 @@ bool conv_plan(ConvP& best, size_t& smem, int& gx, int& gy, int nb, int h, int w
             p.taps = three ? (p.pair8 ? 5 : 9) : 1;
             p.plane = (uint32_t)(p.rows * p.wp) * p.pitch;
             p.abytes = p.cb ? p.plane : p.nch * p.plane;
-            p.aslot = up_to(p.abytes, 1024);
+            p.zeros = p.pair8 ? up_to(p.abytes, 128) : 0;
+            p.aslot = up_to(p.pair8 ? p.zeros + ZEROS : p.abytes, 1024);
             const int BB = p.B * nmap, lines = p.rows * p.wp * (p.cb ? 1 : p.nch);
             // the last block of positions may read past the last plane: keep that in bounds
             const int last = (p.nblk - 1) * p.mstep + 127 + (three ? 2 * p.wp + 2 : 0);
-            const int over = std::max(0, last + 1 - p.rows * p.wp) * (int)p.pitch + (p.pair8 ? p.wp * 16 : 0);
+            const int over = std::max(0, last + 1 - p.rows * p.wp) * (int)p.pitch;
             for (int parts = 1; parts <= n16 / 16; parts++) {
                 const int bn = up_to(div_up(n16, parts), 16);
                 if (bn > 128 || p.nblk * bn > 512 || (parts > 1 && bn == up_to(div_up(n16, parts - 1), 16))) continue;

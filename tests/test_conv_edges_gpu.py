@@ -187,3 +187,37 @@ def test_one_sum_per_weight_is_repeatable(env, n, h, w, ci, co):
     for a, b in zip(first, many):
         assert _rel(a, b) <= 1e-4
     assert int(ops.err.item()) == 0
+
+
+def _conv64(torch, x, wt, taps):
+    """y (n, h, w, co) of x (n, h, w, ci) and weights (co, taps, ci) in 64 bits on the CPU, one output
+    pixel's own taps only (zero padding)."""
+    F = torch.nn.functional
+    n, h, w, ci = x.shape
+    cols = F.unfold(_nchw(x.double().cpu()), 3, padding=1).view(n, ci, taps, h * w).permute(0, 3, 2, 1)
+    return (cols.reshape(n * h * w, -1) @ wt.double().cpu().view(wt.shape[0], -1).T).view(n, h, w, -1)
+
+
+def _same_kind(torch, got, ref, tol):
+    """NaN and infinities at the same places, the finite rest within tol in relative L2"""
+    got, ref = got.double().cpu(), ref.double().cpu()
+    assert torch.equal(torch.isnan(got), torch.isnan(ref))
+    inf = torch.isinf(ref)
+    assert torch.equal(torch.isinf(got), inf) and torch.equal(got[inf], ref[inf])
+    f = torch.isfinite(ref)
+    assert bool(f.any()) and float((got[f] - ref[f]).norm()) <= tol * float(ref[f].norm())
+
+
+# an infinite or NaN input reaches the outputs that have it under one of their taps, and no
+# other; channel counts of every way to stage them (one chunk, swizzled, chunk planes, streamed)
+@pytest.mark.parametrize("n,h,w,ci,co", [(1, 9, 13, 8, 16), (2, 12, 128, 8, 16), (1, 6, 300, 8, 24), (1, 9, 13, 24, 16),
+                                         (1, 7, 128, 16, 16), (1, 11, 40, 48, 32), (1, 6, 21, 288, 16)])
+def test_conv_keeps_nonfinite_inputs_local(env, n, h, w, ci, co):
+    torch, nn, ops, dev = env
+    x = torch.randn(n, h, w, ci, device=dev).bfloat16()
+    x[0, h - 1, w - 1, 3], x[0, 4, 7, 0], x[0, 0, 0, 5] = float("inf"), float("nan"), float("-inf")
+    wt = (0.5 + torch.rand(co, 9 * ci, device=dev)).bfloat16()
+    y = torch.zeros(n, h, w, co, device=dev)
+    ops.conv(nn.act(x, n, h, w), wt, None, nn.act(y, n, h, w), relu=False, y32=y)
+    _same_kind(torch, y, _conv64(torch, x, wt, 9), 1e-5)
+    assert int(ops.err.item()) == 0
