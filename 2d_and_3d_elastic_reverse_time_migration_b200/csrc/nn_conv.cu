@@ -579,15 +579,78 @@ struct WgP {
 struct WgMaps {
     CUtensorMap a[4], b;
 };
+struct WgSrc {
+    Act x, dy;
+};
+
+// A 3x3 weight's sum over the CTA's tiles, product by product
+__device__ float wgrad_sum(const WgP& p, const WgSrc& a, int c, int o, int tap)
+{
+    const int ky = tap / 3, kx = tap - 3 * ky;
+    float s = 0.f;
+    for (int u = blockIdx.x; u < p.units; u += gridDim.x) {
+        const int xt = u % p.tx, q = u / p.tx, yt = q % p.ty, nb = q / p.ty;
+        const int bottom = min(p.h, (yt + 1) * p.rr), end = min(p.w, (xt + 1) * p.tw);
+        for (int y = yt * p.rr; y < bottom; y++) {
+            const int xy = y + ky - 1;
+            for (int i = xt * p.tw; i < end; i++) {
+                const int xc = i + kx - 1;
+                const float d = __bfloat162float(a.dy.p[((long long)(nb * p.h + y) * p.w + i) * a.dy.cs + a.dy.off + o]);
+                float v = 0.f;
+                if (xy >= 0 && xy < p.h && xc >= 0 && xc < p.w)
+                    v = __bfloat162float(a.x.p[((long long)(nb * p.h + xy) * p.w + xc) * a.x.cs + a.x.off + c]);
+                s += v * d;
+            }
+        }
+    }
+    return s;
+}
+// The weights whose accumulator is NaN, once more and without the tensor core.  dy is staged
+// as zeros past the last column and row, where the first tap of a row or column still meets
+// x's last one: an infinite activation there makes a product NaN that the gradient does
+// not have.  Out of line, and after the sums that are none: calls among them took registers
+// from every launch (loss and gradients of a 16 x 256 x 512 batch 2.31 -> 2.40 ms).
+__device__ __noinline__ void wgrad_repair(const WgP& p, const WgSrc& src, const float* acc, uint32_t tmem, float* dw)
+{
+    const int kx0 = blockIdx.y * p.nkx;
+    const int c0 = (int)(blockIdx.z % p.cparts) * p.CB * p.cx, o0 = (int)(blockIdx.z / p.cparts) * p.OB * p.cy;
+    auto add = [&](int c, int o, int tap) {
+        atomicAdd(dw + ((long long)o * 9 + tap) * p.ci + c, wgrad_sum(p, src, c, o, tap));
+    };
+    if (p.rr > 1) {                      // sums in shared memory, as k_wgrad leaves them
+        const int cw = p.CB * p.cx, na = p.OB * p.cy * 9 * cw;
+        for (int q = threadIdx.x; q < na; q += CTHREADS) {
+            const int c = c0 + q % cw, t = q / cw, tap = t % 9, o = o0 + t / 9;
+            if (c < p.ci && o < p.co && tap % 3 >= kx0 && tap % 3 < kx0 + p.nkx && acc[q] != acc[q]) add(c, o, tap);
+        }
+        return;
+    }
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), quad = warp & 3;
+    if (warp >= EPW) return;
+    for (int t = warp >> 2; t < p.nkx * p.mb; t += EPW / 4) {
+        const int k = t / p.mb, b = t - k * p.mb, row = quad * 32 + (threadIdx.x & 31);
+        const int at = b * (128 / p.cx) + row / p.cx, cbk = at / p.jr, ky = at - cbk * p.jr;
+        const int c = c0 + cbk * p.cx + row % p.cx, tap = ky * 3 + kx0 + k;
+        const bool in = at < p.atoms && ky < 3 && kx0 + k < 3 && c < p.ci;
+        for (int n8 = 0; n8 < p.n; n8 += 8) {
+            float v[8];
+            __syncwarp();
+            tmem_ld8(tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(t * p.n + n8), v);
+#pragma unroll
+            for (int q = 0; q < 8; q++)
+                if (in && o0 + n8 + q < p.co && v[q] != v[q]) add(c, o0 + n8 + q, tap);
+        }
+    }
+}
 
 // Partial sums of a CTA's tiles stay in TMEM (3x3: one accumulator per kx, lanes (x
 // chunk, x row j, channel), columns (dy chunk, dy row r, channel)); at the end the lanes
 // and columns with j - r = ky in 0..2 are the gradient of tap ky, summed over r in shared
 // memory and added to dw once per CTA.  A CTA takes at most 4096 pixels per accumulator
-// chain.  x and dy are read past the last column and row as zeros, so an infinite
-// activation in the last column meets a zero gradient there.
+// chain, unless the caller bounds the splits.
 __global__ void __launch_bounds__(CTHREADS, 1) k_wgrad(const __grid_constant__ WgMaps maps,
-                                                       const __grid_constant__ WgP p, float* __restrict__ dw,
+                                                       const __grid_constant__ WgP p,
+                                                       const __grid_constant__ WgSrc src, float* __restrict__ dw,
                                                        float* __restrict__ db, int* err)
 {
     extern __shared__ __align__(1024) uint8_t sm[];
@@ -762,6 +825,7 @@ __global__ void __launch_bounds__(CTHREADS, 1) k_wgrad(const __grid_constant__ W
             for (int q = threadIdx.x; q < na; q += CTHREADS) acc[q] = 0.f;
             __syncthreads();
         }
+        bool nan = false;                // a 3x3 sum is NaN: not added here
         for (int rs = 0; rs < (direct ? 1 : p.rr); rs++) {
             // in shared memory one dy row r at a time: then j - r = ky names every sum once
             if (epi)
@@ -795,9 +859,17 @@ __global__ void __launch_bounds__(CTHREADS, 1) k_wgrad(const __grid_constant__ W
                         const int tap = ky * 3 + kx, cl = cbk * p.cx + ch, ol = ob * p.cy + nc;
                         if (direct) {
                             if (c0 + cl >= p.ci || o0 + ol >= p.co) continue;
+                            float* d = dw + ((long long)(o0 + ol) * 9 + tap) * p.ci + c0 + cl;
+                            const float sum = ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
+                            if (sum == sum) {        // none of them is NaN
 #pragma unroll
-                            for (int q = 0; q < 8; q++)
-                                atomicAdd(dw + ((long long)(o0 + ol + q) * 9 + tap) * p.ci + c0 + cl, v[q]);
+                                for (int q = 0; q < 8; q++) atomicAdd(d + (long long)q * 9 * p.ci, v[q]);
+                            } else {
+                                nan = true;
+#pragma unroll
+                                for (int q = 0; q < 8; q++)
+                                    if (v[q] == v[q]) atomicAdd(d + (long long)q * 9 * p.ci, v[q]);
+                            }
                         } else {
 #pragma unroll
                             for (int q = 0; q < 8; q++) acc[((ol + q) * 9 + tap) * cw + cl] += v[q];
@@ -817,9 +889,13 @@ __global__ void __launch_bounds__(CTHREADS, 1) k_wgrad(const __grid_constant__ W
         if (!direct)
             for (int q = threadIdx.x; q < na; q += CTHREADS) {
                 const int c = c0 + q % cw, t = q / cw, tap = t % 9, o = o0 + t / 9;
-                if (c < p.ci && o < p.co && tap % 3 >= kx0 && tap % 3 < kx0 + p.nkx)
-                    atomicAdd(dw + ((long long)o * 9 + tap) * p.ci + c, acc[q]);
+                if (c < p.ci && o < p.co && tap % 3 >= kx0 && tap % 3 < kx0 + p.nkx) {
+                    if (acc[q] == acc[q]) atomicAdd(dw + ((long long)o * 9 + tap) * p.ci + c, acc[q]);
+                    else nan = true;
+                }
             }
+        // the same in every thread of the block
+        if (__syncthreads_or(nan)) wgrad_repair(p, src, acc, tmem, dw);
     }
     if (!ok && err) atomicExch(err, NN_WAIT);
     tc_fence_before();
@@ -1196,7 +1272,7 @@ cudaError_t wgrad_launch(const Act& x, const Act& dy, float* dw, float* db, bool
     static unsigned long long opted = 0;
     const cudaError_t e = ertm::smem_opt_in(k_wgrad, SMEM_MAX, &opted);
     if (e != cudaSuccess) return e;
-    return ertm::launch_pdl(k_wgrad, grid, dim3(CTHREADS), smem, st, maps, p, dw, db, err);
+    return ertm::launch_pdl(k_wgrad, grid, dim3(CTHREADS), smem, st, maps, p, WgSrc{x, dy}, dw, db, err);
 }
 
 }  // namespace

@@ -221,3 +221,29 @@ def test_conv_keeps_nonfinite_inputs_local(env, n, h, w, ci, co):
     ops.conv(nn.act(x, n, h, w), wt, None, nn.act(y, n, h, w), relu=False, y32=y)
     _same_kind(torch, y, _conv64(torch, x, wt, 9), 1e-5)
     assert int(ops.err.item()) == 0
+
+
+# the same of the weight gradients, with infinite and NaN activations in the last row and column,
+# where a tile's dy ends in zeros, and infinite gradients beside the padding
+@pytest.mark.parametrize("n,h,w,ci,co", [(1, 1, 1, 8, 8), (1, 9, 13, 8, 16), (2, 12, 128, 16, 16), (1, 7, 40, 64, 32),
+                                         (1, 5, 300, 24, 40), (3, 33, 64, 32, 48), (2, 6, 31, 128, 144)])
+@pytest.mark.parametrize("splitk", [0, 1])
+def test_wgrad_keeps_nonfinite_inputs_local(env, n, h, w, ci, co, splitk):
+    torch, nn, ops, dev = env
+    x = torch.randn(n, h, w, ci, device=dev).bfloat16()
+    dy = (0.5 + torch.rand(n, h, w, co, device=dev)).bfloat16()
+    x[n - 1, h - 1, w - 1, 0], x[0, h // 2, w - 1, 1] = float("inf"), float("-inf")
+    x[0, h - 1, w // 2, 2], x[0, 0, 0, 3] = float("nan"), float("inf")
+    dy[0, 0, w // 2, 4], dy[n - 1, h - 1, w - 1, 5] = float("inf"), float("nan")
+    dw = torch.zeros(co, 9 * ci, device=dev)
+    ops.conv_wgrad(nn.act(x, n, h, w), nn.act(dy, n, h, w), dw, splitk=splitk)
+    cols = torch.nn.functional.unfold(_nchw(x.double().cpu()), 3, padding=1).view(n, ci, 9, h * w)
+    ref = torch.einsum("nctp,npo->otc", cols, dy.double().cpu().view(n, h * w, co))
+    _same_kind(torch, dw.view(co, 9, ci), ref, 1e-4)
+    dyu = (0.5 + torch.rand(n, 2 * h, 2 * w, co, device=dev)).bfloat16()
+    dyu[0, 1, 2 * w - 1, 4], dyu[n - 1, 2 * h - 1, 0, 5] = float("inf"), float("nan")
+    du = torch.zeros(4 * co, ci, device=dev)
+    ops.up_wgrad(nn.act(x, n, h, w), nn.act(dyu, n, 2 * h, 2 * w), du, splitk=splitk)
+    g = dyu.double().cpu().view(n, h, 2, w, 2, co).permute(0, 1, 3, 2, 4, 5).reshape(n * h * w, 4 * co)
+    _same_kind(torch, du, g.T @ x.double().cpu().view(n * h * w, ci), 1e-4)
+    assert int(ops.err.item()) == 0
