@@ -664,26 +664,35 @@ struct Range {
 // memory and moves once per replay, so one graph serves every chunk and no step
 // carries a counter launch); the first steps and the remainder are launched directly.
 // A short graph: building one costs about 6 us per launch in it (measured 400 us for 32
-// steps of a 2D pass, against 0.6 us that a replayed step saves over a direct launch),
+// steps of a 2D pass, against 0.3-1 us that a replayed step saves over a direct launch),
 // while a replay of 8 steps already hides its own launch.  Long passes amortise 32.  Two
 // graphs' worth of steps go first, so that the GPU has work while the host builds the graph
 // (a pass of 680 x 380 costs 133 us besides its steps; 196 with one step first and its state
-// zeroed array by array).  2D grids of 100,000 to 600,000 cells are launched directly up to 200
-// steps: their steps (4-15 us) outlast the launches but too few of them outlast the graph's
-// construction (680 x 380, 120 steps 0.90 ms, 1.08 with a graph; 240 steps 1.75 and, with four
-// graphs' worth of steps first, 1.77; 800 steps 5.75 and 5.62).  On smaller grids the host is
-// the slower side (168 x 104, 800 steps 4.3 ms, 3.4 with a graph), on larger ones two graphs'
-// worth of steps hide the construction (1471 x 803, 120 steps 2.73 and 2.68).
+// zeroed array by array).
+// On 2D grids below 400,000 cells 16 steps (4-9 us each) do not outlast the construction:
+// four graphs' worth go first, and passes below 200 steps, which the graph would not serve
+// long enough, take none.  Measured, ms per pass, direct / graph after 16 steps / after 32:
+//   cells       60 steps             120 steps            240 steps            800 steps
+//    17,472  0.301 / 0.423 / -    0.565 / 0.654 / 0.659  1.073 / 1.134 / 1.140  3.52 / 3.36 / 3.38
+//    35,000  0.312 / 0.415 / -    0.583 / 0.672 / 0.678  1.116 / 1.156 / 1.163  3.62 / 3.41 / 3.43
+//    60,000  0.342 / 0.423 / -    0.659 / 0.685 / 0.685  1.299 / 1.214 / 1.214  4.06 / 3.67 / 3.68
+//    97,500  0.408 / 0.467 / -    0.788 / 0.797 / 0.775  1.549 / 1.451 / 1.428  5.12 / 4.50 / 4.47
+//   132,000  0.411 / 0.490 / -    0.779 / 0.838 / 0.812  1.523 / 1.544 / 1.522  4.99 / 4.85 / 4.81
+//   258,400  0.464 / 0.528 / -    0.889 / 0.937 / 0.889  1.748 / 1.771 / 1.736  5.75 / 5.62 / 5.58
+//   392,000  0.709 / 0.711 / -    1.369 / 1.349 / 1.353  2.707 / 2.644 / 2.642  8.90 / 8.66 / 8.65
+//   585,600  0.788 / 0.780 / -    1.545 / 1.488 / 1.498  3.001 / 2.905 / 2.909  9.86 / 9.54 / 9.53
+// and RTM likewise (17,472 cells, 120 steps 1.01 / 1.17 / 1.18, 800 steps 6.36 / 6.12 / 6.13; 258,400
+// 1.72 / 1.80 / 1.73 and 11.1 / 10.8 / 10.7; 585,600 2.92 / 2.80 / 2.82 and 18.8 / 17.7 / 17.8).  In
+// steps the sides meet between 120 and 400, on average at 240; in cells at 400,000.
 template <typename F>
 int time_loop(ertm_ctx* c, int nsteps, int dir, F&& one_step)
 {
     const int kGraphSteps = nsteps >= 1500 ? 32 : 8;
-    const long long cells = (long long)c->g.nx * c->g.nz;
-    const bool medium2d = c->g.two_d && cells > 100000 && cells < 600000;
-    const bool use_graph = !medium2d || nsteps >= 200;
-    const int lead = medium2d && nsteps >= 8 * kGraphSteps ? 4 * kGraphSteps
-                     : nsteps >= 4 * kGraphSteps           ? 2 * kGraphSteps
-                                                           : 1;
+    const bool short_steps = c->g.two_d && (long long)c->g.nx * c->g.nz < 400000;
+    const bool use_graph = !short_steps || nsteps >= 200;
+    const int lead = short_steps && nsteps >= 8 * kGraphSteps ? 4 * kGraphSteps
+                     : nsteps >= 4 * kGraphSteps              ? 2 * kGraphSteps
+                                                              : 1;
     int done = 0;
     for (; done < std::min(nsteps, lead); done++) CK(c, one_step(dir * done));
     int base = 0;                    // steps that the device's index has moved

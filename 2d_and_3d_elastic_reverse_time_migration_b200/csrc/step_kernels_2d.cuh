@@ -281,7 +281,7 @@ __global__ void __launch_bounds__(256, 2) k_velocity2d(const __grid_constant__ V
         }
     }
     tile2_go(false);
-    const int it = EPI != EPI_NONE || REC ? step_index(a) : 0;
+    const int it = EPI != EPI_NONE || rec >= 0 ? step_index(a) : 0;
     if (!tile2_wait(&bar, consumer_polls(a), a.err, skip)) return;
     if (!act || r0 >= a.nz) return;
     const float* Txx = sm + tr * NR * XW + tx + T::XB;

@@ -94,3 +94,24 @@ def test_born_segments_do_not_change_the_gradient(ertm, orc, nshots):
         for run in g[every]:
             for a, b in zip(run, g[150][0]):
                 assert np.any(b) and np.array_equal(a, b), every
+
+
+# passes on either side of the lines between direct launches and graphs, and with one, two and
+# four graphs' worth of steps ahead, record the same samples bit for bit
+@pytest.mark.parametrize("nz,nx,steps", [(60, 90, (20, 63, 64, 199, 200, 201, 260)), (632, 632, (20, 40)),
+                                         (633, 633, (16, 20, 40, 70))])
+def test_time_loop_forms_agree(ertm, orc, nz, nx, steps):
+    shape, pml = (nz, 1, nx), (9, 8, 0, 0, 8, 9)
+    m = model(shape, seed=6)
+    src, rec = geometry(shape, pml)
+    got = {}
+    for nt in steps:
+        cfg = ertm.Config(nx=nx, ny=1, nz=nz, dx=DX, dy=DX, dz=DX, dt_ms=DT_MS, nt=nt, pml=pml)
+        with ertm.Context(cfg) as ctx:
+            ctx.set_model(ertm.TRUE_MODEL, *m)
+            got[nt] = ctx.forward_together_using_real_model(
+                ertm.Shot(*src, wavelet=orc.ricker(25.0, DT_MS / 1000.0), **rec))
+    longest = got[max(steps)]
+    assert np.any(longest)
+    for nt, d in got.items():
+        assert np.array_equal(d, longest[:, :nt]), nt
