@@ -676,12 +676,11 @@ dim3 tile_grid(const BornArgs& a, int nr)
 {
     return dim3((a.nx + BXH + TX2 - 1) / TX2, (a.nz + 4 * nr - 1) / (4 * nr), a.nshot);
 }
-template <typename... P, typename... A>
-cudaError_t launch_tile(void (*K)(P...), unsigned long long* opted, const BornArgs& a, int nr, size_t smem,
-                        cudaStream_t s, const A&... args)
+template <size_t SMEM, typename... P, typename... A>
+cudaError_t launch_tile(void (*K)(P...), const BornArgs& a, int nr, cudaStream_t s, const A&... args)
 {
-    const cudaError_t e = smem > 48 * 1024 ? smem_opt_in(K, smem, opted) : cudaSuccess;
-    return e != cudaSuccess ? e : launch_pdl(K, tile_grid(a, nr), 256, smem, s, args...);
+    static_assert(SMEM <= 48 * 1024, "shared memory without opt-in");
+    return launch_pdl(K, tile_grid(a, nr), 256, SMEM, s, args...);
 }
 
 template <int R, int NR>
@@ -696,15 +695,12 @@ constexpr size_t sig_bytes(int n)
 template <int R, int NM, int NR, bool BORN>
 cudaError_t stress_r(const BornMaps& m, const BornArgs& a, int it, cudaStream_t s)
 {
-    static unsigned long long opted = 0;
-    return launch_tile(k_born_stress<R, BORN, NM, NR>, &opted, a, a.nr, xz_bytes<R, NR>(BORN ? 4 : 2), s, m, a, it);
+    return launch_tile<xz_bytes<R, NR>(BORN ? 4 : 2)>(k_born_stress<R, BORN, NM, NR>, a, a.nr, s, m, a, it);
 }
 template <int R, int NR, bool BORN, bool KEEP>
 cudaError_t velocity_r(const BornMaps& m, const BornArgs& a, int it, cudaStream_t s)
 {
-    static unsigned long long opted = 0;
-    return launch_tile(k_born_velocity<R, BORN, KEEP, NR>, &opted, a, a.nrv, sig_bytes<R, NR>(BORN ? 2 : 1), s, m, a,
-                       it);
+    return launch_tile<sig_bytes<R, NR>(BORN ? 2 : 1)>(k_born_velocity<R, BORN, KEEP, NR>, a, a.nrv, s, m, a, it);
 }
 template <int R, int NM, bool BORN>
 cudaError_t stress_nr(const BornMaps& m, const BornArgs& a, int it, cudaStream_t s)
@@ -731,14 +727,12 @@ cudaError_t step_r(const BornMaps& m, const BornArgs& a, int it, bool born, bool
 template <int R, int NM, int NR>
 cudaError_t vm_r(const BornMaps& m, const BornArgs& a, cudaStream_t s)
 {
-    static unsigned long long opted = 0;
-    return launch_tile(k_adj_vm<R, NM, NR>, &opted, a, a.nr, xz_bytes<R, NR>(5), s, m, a);
+    return launch_tile<xz_bytes<R, NR>(5)>(k_adj_vm<R, NM, NR>, a, a.nr, s, m, a);
 }
 template <int R, int NR>
 cudaError_t str_r(const BornMaps& m, const BornArgs& a, int it, cudaStream_t s)
 {
-    static unsigned long long opted = 0;
-    return launch_tile(k_adj_str<R, NR>, &opted, a, a.nrv, sig_bytes<R, NR>(1), s, m, a, it - 1);
+    return launch_tile<sig_bytes<R, NR>(1)>(k_adj_str<R, NR>, a, a.nrv, s, m, a, it - 1);
 }
 template <int R, int NM>
 cudaError_t adj_r(const BornMaps& m, const BornArgs& a, int it, cudaStream_t s)

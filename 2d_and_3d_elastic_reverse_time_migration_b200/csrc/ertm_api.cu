@@ -1106,7 +1106,6 @@ int ertm_forward_together_using_smoothed_model(ertm_ctx* c, const ertm_shot* s)
     int rc = validate_shot(c, s, true);
     if (rc) return rc;
     if ((rc = ensure_excitation(c))) return rc;
-    const Geom& g = c->g;
     if ((rc = zero_excitation(c, c->stream))) return rc;
     int nsrc = c->cfg.src_steps > 0 ? c->cfg.src_steps : 2 * c->cfg.nt / 3;
     c->have_excitation = false;
@@ -1297,7 +1296,6 @@ int ertm_rtm_multi(ertm_ctx* const* ctx, int n, const ertm_shot* shots, const fl
     int nsrc_max = 0;
     for (int q = 0; q < n; q++) {
         ertm_ctx* c = ctx[q];
-        const Geom& g = c->g;
         if ((rc = ensure_excitation(c))) return rc;
         if ((rc = zero_excitation(c, st))) return rc;
         c->have_excitation = false;
@@ -1320,7 +1318,6 @@ int ertm_rtm_multi(ertm_ctx* const* ctx, int n, const ertm_shot* shots, const fl
     int nt_max = 0;
     for (int q = 0; q < n; q++) {
         ertm_ctx* c = ctx[q];
-        const Geom& g = c->g;
         if ((rc = ensure_images(c))) return rc;
         if ((rc = zero_images(c, st))) return rc;
         const long long nrec = nrec_of(&shots[q]);

@@ -45,14 +45,6 @@
 
 namespace ertm {
 
-__device__ __forceinline__ float cpml_upd(float* __restrict__ psi, long long p, float a, float b,
-                                          float d)
-{
-    float v = fmaf(b, psi[p], a * d);
-    psi[p] = v;
-    return d + v;
-}
-
 template <bool Y>
 __device__ __forceinline__ void damping(const KArgs& a, bool cpml, int i, int j, int k, float& g1,
                                         float& g2)
