@@ -108,6 +108,11 @@ struct ertm_ctx {
     // 3D step-kernel variant (ertm_set_step_variant): 0 one cell per thread, 1 cell pairs
     int pairs = 0;
 
+    // graphs of time loops, oldest first; the replays of the first `graphs_done` have finished.
+    // A finished one is destroyed when the next has been launched, while the GPU works on that.
+    std::vector<cudaGraphExec_t> graphs;
+    size_t graphs_done = 0;
+
     std::string err;
     long long launches = 0;
 
@@ -509,6 +514,7 @@ int check_device_error(ertm_ctx* c)
     int e = 0;
     CK(c, cudaMemcpyAsync(&e, c->err_d, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
     CK(c, cudaStreamSynchronize(c->stream));
+    c->graphs_done = c->graphs.size();
     if (e) {
         CK(c, cudaMemsetAsync(c->err_d, 0, sizeof(int), c->stream));
         return fail(c, ERTM_EDEVICE, "a step kernel's bounded wait for its staged planes expired (code %d)", e);
@@ -714,12 +720,17 @@ int time_loop(ertm_ctx* c, int nsteps, int dir, F&& one_step)
             done += kGraphSteps;
             c->launches++;
         }
-        if (exec) cudaGraphExecDestroy(exec);
+        if (exec) c->graphs.push_back(exec);
         if (graph) cudaGraphDestroy(graph);
         if (e != cudaSuccess) return fail(c, ERTM_ECUDA, "graph time loop: %s", cudaGetErrorString(e));
     }
     if (base) base = done;           // the replays moved the index along
     for (; done < nsteps; done++) CK(c, one_step(dir * (done - base)));
+    if (base) {
+        for (size_t q = 0; q < c->graphs_done; q++) cudaGraphExecDestroy(c->graphs[q]);
+        c->graphs.erase(c->graphs.begin(), c->graphs.begin() + c->graphs_done);
+        c->graphs_done = 0;
+    }
     return ERTM_OK;
 }
 
@@ -914,6 +925,7 @@ int ertm_destroy(ertm_ctx* c)
     if (!c) return ERTM_OK;
     cudaSetDevice(c->device);
     if (c->stream) cudaStreamSynchronize(c->stream);
+    for (cudaGraphExec_t e : c->graphs) cudaGraphExecDestroy(e);
     for (int q = 0; q < NFIELD; q++) cudaFree(c->f_base[q]);
     for (int w = 0; w < 2; w++)
         for (int q = 0; q < 5; q++) cudaFree(c->m_base[w][q]);
