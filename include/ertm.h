@@ -29,7 +29,9 @@
  *  - Pointer arguments may be host (pageable or pinned) or device memory of the
  *    context's GPU; the library detects which.
  *  - Calls are ordered on the context's stream and return when their results
- *    are complete.  One context per host thread; a context is not re-entrant.
+ *    are complete.  What other streams still have queued on a device pointer must
+ *    be done, or ordered on that stream, before the call.  One context per host
+ *    thread; a context is not re-entrant.
  *  - Traces are [3][nt][nrec] (vx, vy, vz; vy is zero in 2D), receiver r =
  *    iry*nrx + irx.
  */
